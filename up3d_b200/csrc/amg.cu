@@ -479,23 +479,150 @@ __global__ void k_gather_vals(int64_t m, const int32_t* __restrict__ perm, const
     GRID_STRIDE(k, m) dst[k] = src[perm[k]];
 }
 
-// C = A B on C's precomputed pattern, one row per thread, products added in
-// (A entry, B entry) order
-__global__ void k_spgemm_num(int64_t n, const int32_t* __restrict__ Ap, const int32_t* __restrict__ Ai,
-                             const double* __restrict__ Ax, const int32_t* __restrict__ Bp,
-                             const int32_t* __restrict__ Bi, const double* __restrict__ Bx,
-                             const int32_t* __restrict__ Cp, const int32_t* __restrict__ Ci,
-                             double* __restrict__ Cx) {
-    GRID_STRIDE(r, n) {
-        const int32_t cb = Cp[r], cl = Cp[r + 1] - cb;
-        for (int32_t q = 0; q < cl; ++q) Cx[cb + q] = 0.0;
-        for (int32_t k = Ap[r]; k < Ap[r + 1]; ++k) {
-            const double a = Ax[k];
-            const int32_t j = Ai[k];
-            for (int32_t q = Bp[j]; q < Bp[j + 1]; ++q) {
-                const int32_t pos = cb + dev_lower_bound(Ci + cb, cl, Bi[q]);
-                Cx[pos] = __dadd_rn(Cx[pos], __dmul_rn(a, Bx[q]));
+// C = A B on C's precomputed pattern, products added to each C entry in
+// (A entry, B entry) order, each rounded (the same bits for every kernel
+// below).  One thread per row left a coarse row's hundreds of products (a
+// Galerkin row of the 625 k-row Picard matrix: 89 R entries x 8.5 A P
+// entries) as one chain of dependent loads and global read-modify-writes:
+// 1.26 ms per product on average, 7.5 of the 11.4 ms of a refresh; with the
+// kernels below the six products take 0.9 ms (Picard step 25.5 -> 18.9 ms).
+
+// Short C rows (at most 16 entries: A P of a P1 level, 15 x 3.6 products
+// into 8.5 entries): eight lanes per row, each lane owning the columns at
+// positions sub and sub + 8 of the row and adding the products that land
+// there; the row's A entries are loaded eight at a time, one per lane, and
+// the B rows read as broadcasts.  No search, no shared memory.
+constexpr int SPGEMM_OWNED = 16;
+__global__ void __launch_bounds__(128)
+    k_spgemm_owned(int64_t n, const int32_t* __restrict__ Ap, const int32_t* __restrict__ Ai,
+                   const double* __restrict__ Ax, const int32_t* __restrict__ Bp, const int32_t* __restrict__ Bi,
+                   const double* __restrict__ Bx, const int32_t* __restrict__ Cp, const int32_t* __restrict__ Ci,
+                   double* __restrict__ Cx) {
+    const int sub = threadIdx.x & 7;
+    const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+    const int64_t n_warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    for (int64_t base = warp * 4; base < n; base += n_warps * 4) {   // warp-uniform
+        const int64_t r = base + ((threadIdx.x & 31) >> 3);
+        int32_t cb = 0, cl = 0, s = 0, e = 0;
+        if (r < n) {
+            cb = Cp[r];
+            cl = Cp[r + 1] - cb;
+            s = Ap[r];
+            e = Ap[r + 1];
+        }
+        const int32_t c0 = sub < cl ? Ci[cb + sub] : -1, c1 = sub + 8 < cl ? Ci[cb + sub + 8] : -1;
+        double acc0 = 0.0, acc1 = 0.0;
+        const int len = __reduce_max_sync(0xffffffffu, e - s);
+        for (int k0 = 0; k0 < len; k0 += 8) {
+            double a = 0.0;
+            int32_t b0 = 0, b1 = 0;
+            if (s + k0 + sub < e) {
+                const int32_t j = Ai[s + k0 + sub];
+                a = Ax[s + k0 + sub];
+                b0 = Bp[j];
+                b1 = Bp[j + 1];
             }
+#pragma unroll
+            for (int t = 0; t < 8; ++t) {
+                const double at = __shfl_sync(0xffffffffu, a, t, 8);
+                const int32_t q1 = __shfl_sync(0xffffffffu, b1, t, 8);
+                for (int32_t q = __shfl_sync(0xffffffffu, b0, t, 8); q < q1; ++q) {
+                    const int32_t c = Bi[q];
+                    const double v = __dmul_rn(at, Bx[q]);
+                    if (c == c0) acc0 = __dadd_rn(acc0, v);
+                    if (c == c1) acc1 = __dadd_rn(acc1, v);
+                }
+            }
+        }
+        if (sub < cl) Cx[cb + sub] = acc0;
+        if (sub + 8 < cl) Cx[cb + sub + 8] = acc1;
+    }
+}
+
+// One C row by one warp: G lanes per A entry walk its B row (32 / G entries
+// side by side, SPGEMM_UNROLL rounds of them loaded and located in the C
+// row ahead of the adds), the groups then add in entry order, one after the
+// other.  `cols` / `acc`: the C row's columns and its zeroed sums, in
+// shared memory or (rows longer than the staging) in place.
+constexpr int SPGEMM_UNROLL = 2;
+template <int G>
+__device__ __forceinline__ void spgemm_row(int32_t s, int32_t e, const int32_t* __restrict__ Ai,
+                                           const double* __restrict__ Ax, const int32_t* __restrict__ Bp,
+                                           const int32_t* __restrict__ Bi, const double* __restrict__ Bx,
+                                           const int32_t* cols, int32_t cl, double* acc) {
+    constexpr int NG = 32 / G;
+    const int lane = threadIdx.x & 31, grp = lane / G, sub = lane % G;
+    for (int32_t k0 = s; k0 < e; k0 += 32) {
+        double a = 0.0;
+        int32_t b0 = 0, b1 = 0;
+        if (k0 + lane < e) {
+            const int32_t j = Ai[k0 + lane];
+            a = Ax[k0 + lane];
+            b0 = Bp[j];
+            b1 = Bp[j + 1];
+        }
+        const int cnt = e - k0 < 32 ? e - k0 : 32;
+        for (int t0 = 0; t0 < cnt; t0 += NG * SPGEMM_UNROLL) {
+            double av[SPGEMM_UNROLL], v[SPGEMM_UNROLL];
+            int32_t q0[SPGEMM_UNROLL], q1[SPGEMM_UNROLL], pos[SPGEMM_UNROLL];
+#pragma unroll
+            for (int u = 0; u < SPGEMM_UNROLL; ++u) {
+                const int src = t0 + u * NG + grp;   // past cnt: an empty entry or another lane's, masked below
+                av[u] = __shfl_sync(0xffffffffu, a, src & 31);
+                q0[u] = __shfl_sync(0xffffffffu, b0, src & 31);
+                q1[u] = __shfl_sync(0xffffffffu, b1, src & 31);
+                if (src >= cnt) q1[u] = q0[u];
+                pos[u] = -1;
+                if (q0[u] + sub < q1[u]) {
+                    v[u] = __dmul_rn(av[u], Bx[q0[u] + sub]);
+                    pos[u] = dev_lower_bound(cols, cl, Bi[q0[u] + sub]);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < SPGEMM_UNROLL; ++u)
+                for (int g = 0; g < NG; ++g) {
+                    if (grp == g) {
+                        if (pos[u] >= 0) acc[pos[u]] = __dadd_rn(acc[pos[u]], v[u]);
+                        for (int32_t q = q0[u] + sub + G; q < q1[u]; q += G) {   // B rows longer than G
+                            const int32_t p = dev_lower_bound(cols, cl, Bi[q]);
+                            acc[p] = __dadd_rn(acc[p], __dmul_rn(av[u], Bx[q]));
+                        }
+                    }
+                    __syncwarp();
+                }
+        }
+    }
+}
+
+// One warp per C row, the row's columns and sums staged in shared memory
+// (`cap` entries per warp; longer rows work in place).
+constexpr int SPGEMM_WARPS = 4, SPGEMM_CAP = 1024;
+template <int G>
+__global__ void __launch_bounds__(SPGEMM_WARPS * 32)
+    k_spgemm_warp(int64_t n, int cap, const int32_t* __restrict__ Ap, const int32_t* __restrict__ Ai,
+                  const double* __restrict__ Ax, const int32_t* __restrict__ Bp, const int32_t* __restrict__ Bi,
+                  const double* __restrict__ Bx, const int32_t* __restrict__ Cp, const int32_t* __restrict__ Ci,
+                  double* __restrict__ Cx) {
+    extern __shared__ __align__(16) unsigned char spgemm_sm[];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    double* sacc = reinterpret_cast<double*>(spgemm_sm) + (size_t)w * cap;
+    int32_t* scol = reinterpret_cast<int32_t*>(spgemm_sm + sizeof(double) * SPGEMM_WARPS * cap) + (size_t)w * cap;
+    const int64_t n_warps = (int64_t)gridDim.x * SPGEMM_WARPS;
+    for (int64_t r = (int64_t)blockIdx.x * SPGEMM_WARPS + w; r < n; r += n_warps) {
+        const int32_t cb = Cp[r], cl = Cp[r + 1] - cb;
+        if (cl <= cap) {
+            for (int32_t q = lane; q < cl; q += 32) {
+                scol[q] = Ci[cb + q];
+                sacc[q] = 0.0;
+            }
+            __syncwarp();
+            spgemm_row<G>(Ap[r], Ap[r + 1], Ai, Ax, Bp, Bi, Bx, scol, cl, sacc);
+            for (int32_t q = lane; q < cl; q += 32) Cx[cb + q] = sacc[q];
+            __syncwarp();
+        } else {
+            for (int32_t q = lane; q < cl; q += 32) Cx[cb + q] = 0.0;
+            __syncwarp();
+            spgemm_row<G>(Ap[r], Ap[r + 1], Ai, Ax, Bp, Bi, Bx, Ci + cb, cl, Cx + cb);
         }
     }
 }
@@ -741,6 +868,24 @@ struct DevCSR {
     }
 };
 
+// Values of C = A B (all patterns set up); c_max = longest C row.
+void launch_spgemm(const DevCSR<double>& A, const DevCSR<double>& B, const DevCSR<double>& C, int c_max,
+                   cudaStream_t s) {
+    if (c_max <= SPGEMM_OWNED) {
+        k_spgemm_owned<<<grid_for(C.n, 16, (int64_t)148 * 64), 128, 0, s>>>(C.n, A.p.get(), A.i.get(), A.x.get(), B.p.get(), B.i.get(),
+                                                          B.x.get(), C.p.get(), C.i.get(), C.x.get());
+    } else {
+        const int cap = std::min(c_max, SPGEMM_CAP);
+        const size_t smem = (sizeof(double) + sizeof(int32_t)) * SPGEMM_WARPS * (size_t)cap;
+        const unsigned grid = grid_for(C.n, SPGEMM_WARPS, (int64_t)148 * 64);
+        // lanes per A entry: the mean B row length, rounded up
+        auto kern = B.nnz <= 8 * B.n ? k_spgemm_warp<8> : B.nnz <= 16 * B.n ? k_spgemm_warp<16> : k_spgemm_warp<32>;
+        kern<<<grid, SPGEMM_WARPS * 32, smem, s>>>(C.n, cap, A.p.get(), A.i.get(), A.x.get(), B.p.get(), B.i.get(),
+                                                   B.x.get(), C.p.get(), C.i.get(), C.x.get());
+    }
+    UP3D_CHECK_LAUNCH();
+}
+
 template <class T>
 void upload(DBuf<T>& d, const std::vector<T>& h, cudaStream_t s) {
     d.alloc(std::max<size_t>(h.size(), 1));
@@ -793,6 +938,7 @@ struct SymLevel {
     DBuf<double> t;              // tentative prolongator value of each row
     DevCSR<double> P, R, AP;     // prolongator, restriction (P^T), A P
     DBuf<int32_t> tperm;         // R entry -> P entry
+    int a_max = 0, ap_max = 0;   // longest rows of A and A P
     bool has_skip = false;
 };
 
@@ -897,6 +1043,13 @@ std::vector<int32_t> diag_slots(const HostCSR& A) {
     return d;
 }
 
+int longest_row(const HostCSR& A) {
+    int32_t m = 0;
+#pragma omp parallel for schedule(static) reduction(max : m)
+    for (int64_t r = 0; r < A.n; ++r) m = std::max(m, A.p[r + 1] - A.p[r]);
+    return m;
+}
+
 // Device numeric phase: every level's D^-1, omega, P, R, A P and coarser
 // operator, then the coarsest inverse; fills the cycle's levels.
 void numeric(Amg& a, cudaStream_t s) {
@@ -939,14 +1092,8 @@ void numeric(Amg& a, cudaStream_t s) {
         UP3D_CHECK_LAUNCH();
         k_gather_vals<<<grid_for(F.R.nnz, 256), 256, 0, s>>>(F.R.nnz, F.tperm.get(), F.P.x.get(), F.R.x.get());
         UP3D_CHECK_LAUNCH();
-        k_spgemm_num<<<grid_for(n, 128), 128, 0, s>>>(n, F.A.p.get(), F.A.i.get(), F.A.x.get(), F.P.p.get(),
-                                                      F.P.i.get(), F.P.x.get(), F.AP.p.get(), F.AP.i.get(),
-                                                      F.AP.x.get());
-        UP3D_CHECK_LAUNCH();
-        k_spgemm_num<<<grid_for(F.R.n, 128), 128, 0, s>>>(F.R.n, F.R.p.get(), F.R.i.get(), F.R.x.get(),
-                                                          F.AP.p.get(), F.AP.i.get(), F.AP.x.get(), C.A.p.get(),
-                                                          C.A.i.get(), C.A.x.get());
-        UP3D_CHECK_LAUNCH();
+        launch_spgemm(F.A, F.P, F.AP, F.ap_max, s);
+        launch_spgemm(F.R, F.AP, C.A, C.a_max, s);
     }
     // coarsest dense inverse
     const SymLevel& Cl = *a.sym.back();
@@ -1253,6 +1400,7 @@ void* amg_setup(const up3d_csr& A, const up3d_amg_options& opt, cudaStream_t s) 
             auto* F = new SymLevel();
             a->sym.push_back(F);
             F->A.upload_pattern(Al, s);
+            F->a_max = longest_row(Al);
             upload(F->diag, diag_slots(Al), s);
             F->has_skip = a->sym.size() == 1 && a->has_dir;
             if (F->has_skip) upload(F->skip, cur_skip, s);
@@ -1281,6 +1429,7 @@ void* amg_setup(const up3d_csr& A, const up3d_amg_options& opt, cudaStream_t s) 
             F->P.upload_pattern(P, s);
             F->R.upload_pattern(R, s);
             F->AP.upload_pattern(AP, s);
+            F->ap_max = longest_row(AP);
             UP3D_CUDA(cudaStreamSynchronize(s));  // host vectors above go out of scope
             As.push_back(std::move(Ac));
             cur_skip.assign(As.back().n, 0);
