@@ -401,6 +401,23 @@ void Operator::apply(const float* x, float* y, cudaStream_t s) const {
                         s);
 }
 
+void Operator::residual(const double* b, const double* x, double* r, double* tmp, cudaStream_t s) const {
+    if (!coupled) {
+        launch_residual(A.n, A.indptr, A.indices, A.data, extra.indptr, extra.indices, extra.data, x, b, r,
+                        A.dirichlet, s);
+        return;
+    }
+    apply(x, tmp, s);
+    k_sub<double><<<grid_for(rows(), 256), 256, 0, s>>>(b, tmp, r, rows());
+    UP3D_CHECK_LAUNCH();
+}
+
+void Operator::residual(const float* b, const float* x, float* r, float* tmp, cudaStream_t s) const {
+    apply(x, tmp, s);
+    k_sub<float><<<grid_for(rows(), 256), 256, 0, s>>>(b, tmp, r, rows());
+    UP3D_CHECK_LAUNCH();
+}
+
 }  // namespace up3d
 
 // ------------------------------------------------------------ preconditioners
@@ -580,9 +597,7 @@ int gmres_solve(const Operator& op, const T* b, T* x, double rtol, double atol, 
     auto Hat = [&](int col, int k) -> double& { return H[(size_t)col * (restart + 1) + k]; };
     for (int cycle = 0; cycle < maxiter && !done; ++cycle) {
         if (cycle == 0) {
-            op.apply(x, tmp.get(), s);
-            k_sub<T><<<grid_for(n, 256), 256, 0, s>>>(b, tmp.get(), r.get(), n);
-            UP3D_CHECK_LAUNCH();
+            op.residual(b, x, r.get(), tmp.get(), s);
             rnorm = bl.nrm2(r.get(), n);
             if (rnorm < atol_eff) {
                 done = true;
@@ -670,9 +685,7 @@ int gmres_solve(const Operator& op, const T* b, T* x, double rtol, double atol, 
         for (auto& v : y) v = -v;
         UP3D_CUDA(cudaMemcpyAsync(hdev.get(), y.data(), sizeof(double) * (col + 1), cudaMemcpyHostToDevice, s));
         bl.multiaxpy(V.get(), n, col + 1, hdev.get(), x, n);
-        op.apply(x, tmp.get(), s);
-        k_sub<T><<<grid_for(n, 256), 256, 0, s>>>(b, tmp.get(), r.get(), n);
-        UP3D_CHECK_LAUNCH();
+        op.residual(b, x, r.get(), tmp.get(), s);
         rnorm = bl.nrm2(r.get(), n);
         if (rnorm <= atol_eff || breakdown || !std::isfinite(rnorm)) break;
         if (presid <= ptol) ptol_max = std::max(eps, 0.25 * ptol_max);
@@ -736,9 +749,7 @@ int gmres_ir_solve(const Operator& op, const double* b, double* x, double rtol, 
     int64_t tot_inner = 0, it = 0;
     double rn = 0.0, rn_prev = 0.0, rtrue = 0.0;
     for (;; ++it) {
-        op.apply(x, tmp.get(), s);
-        k_sub<double><<<grid_for(n, 256), 256, 0, s>>>(b, tmp.get(), r.get(), n);
-        UP3D_CHECK_LAUNCH();
+        op.residual(b, x, r.get(), tmp.get(), s);
         rn = tested_norm(r.get());
         rtrue = M ? bl.nrm2(r.get(), n) : rn;
         if (rn <= tol || !std::isfinite(rn) || it >= refine_max || tot_inner >= budget) break;
@@ -751,9 +762,7 @@ int gmres_ir_solve(const Operator& op, const double* b, double* x, double rtol, 
             gmres_solve<double>(op, b, x, rtol, atol, restart, cycles_left, M, &inn, &r64, s);
             tot_inner += inn;
             ++it;
-            op.apply(x, tmp.get(), s);
-            k_sub<double><<<grid_for(n, 256), 256, 0, s>>>(b, tmp.get(), r.get(), n);
-            UP3D_CHECK_LAUNCH();
+            op.residual(b, x, r.get(), tmp.get(), s);
             rn = tested_norm(r.get());
             rtrue = M ? bl.nrm2(r.get(), n) : rn;
             break;

@@ -15,6 +15,11 @@ template <class T>
 void launch_spmv2(int64_t n, const int32_t* indptr, const int32_t* indices, const T* data, const int32_t* xptr,
                   const int32_t* xidx, const T* xdata, const T* x, T* y, const uint8_t* dir, cudaStream_t s);
 
+// r = b - (A x + xA x) with each row's sum rounded once (linear.cu)
+void launch_residual(int64_t n, const int32_t* indptr, const int32_t* indices, const double* data,
+                     const int32_t* xptr, const int32_t* xidx, const double* xdata, const double* x, const double* b,
+                     double* r, const uint8_t* dir, cudaStream_t s);
+
 // The coupled (phi, Gamma) operator of a wake-cut mesh (wake.cu): y =
 // J_ff x + B (K x + g) in full reduced size, t = K x + g when t != NULL.
 int64_t coupled_rows(const up3d_coupled* c);
@@ -62,6 +67,9 @@ struct Operator {
     int64_t rows() const { return coupled ? coupled_rows(coupled) : A.n; }
     void apply(const double* x, double* y, cudaStream_t s) const;
     void apply(const float* x, float* y, cudaStream_t s) const;
+    // r = b - A x, through tmp where the operator has no residual kernel
+    void residual(const double* b, const double* x, double* r, double* tmp, cudaStream_t s) const;
+    void residual(const float* b, const float* x, float* r, float* tmp, cudaStream_t s) const;
 };
 
 void amg_apply(void* amg, const double* r, double* z, cudaStream_t s);

@@ -57,7 +57,69 @@ __global__ void __launch_bounds__(CSR_ROWS_BLOCK)
     }
 }
 
+// r = b - (A x + X x), masked as k_spmv, each row's sum carried as an
+// unevaluated pair (error-free products by fma, Knuth's two-sum): rounded
+// once, whatever the cancellation.  A restart's true residual is formed
+// here: near a singular matrix |x| is so large that a plain sum's rounding
+// (eps |A| |x|) is above the tolerance asked for, and whether a cycle met it
+// hung on the order of the sums.  Four lanes per row; once per restart.
+__device__ __forceinline__ void two_sum(double& hi, double& lo, double v) {
+    const double s = __dadd_rn(hi, v), t = __dsub_rn(s, hi);
+    lo += __dadd_rn(__dsub_rn(hi, __dsub_rn(s, t)), __dsub_rn(v, t));
+    hi = s;
+}
+__global__ void __launch_bounds__(CSR_ROWS_BLOCK)
+    k_residual(int64_t n, const int32_t* __restrict__ indptr, const int32_t* __restrict__ indices,
+               const double* __restrict__ data, const int32_t* __restrict__ xptr, const int32_t* __restrict__ xidx,
+               const double* __restrict__ xdata, const double* __restrict__ x, const double* __restrict__ b,
+               double* __restrict__ r, const uint8_t* __restrict__ dir) {
+    constexpr int TPR = 4, RPW = 32 / TPR;
+    const int sub = threadIdx.x % TPR, group = (threadIdx.x & 31) / TPR;
+    const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+    const int64_t n_warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    for (int64_t base = warp * RPW; base < n; base += n_warps * RPW) {   // warp-uniform
+        const int64_t row = base + group;
+        double hi = 0.0, lo = 0.0;
+        auto add = [&](const int32_t* p, const int32_t* idx, const double* val) {
+            for (int32_t k = p[row] + sub; k < p[row + 1]; k += TPR) {
+                const int32_t c = idx[k];
+                if (dir && dir[c]) continue;
+                const double v = val[k], xc = x[c], m = __dmul_rn(v, xc);
+                two_sum(hi, lo, m);
+                lo += fma(v, xc, -m);
+            }
+        };
+        if (row < n) {
+            add(indptr, indices, data);
+            if (xptr) add(xptr, xidx, xdata);
+        }
+#pragma unroll
+        for (int o = TPR / 2; o > 0; o >>= 1) {
+            const double h2 = __shfl_down_sync(0xffffffffu, hi, o, TPR), l2 = __shfl_down_sync(0xffffffffu, lo, o, TPR);
+            two_sum(hi, lo, h2);
+            lo += l2;
+        }
+        if (sub == 0 && row < n) {
+            if (dir && dir[row]) {
+                r[row] = b[row] - x[row];
+            } else {
+                hi = -hi;
+                lo = -lo;
+                two_sum(hi, lo, b[row]);
+                r[row] = hi + lo;
+            }
+        }
+    }
+}
+
 }  // namespace
+
+void launch_residual(int64_t n, const int32_t* indptr, const int32_t* indices, const double* data,
+                     const int32_t* xptr, const int32_t* xidx, const double* xdata, const double* x, const double* b,
+                     double* r, const uint8_t* dir, cudaStream_t s) {
+    k_residual<<<lanes_grid(n, 4), CSR_ROWS_BLOCK, 0, s>>>(n, indptr, indices, data, xptr, xidx, xdata, x, b, r, dir);
+    UP3D_CHECK_LAUNCH();
+}
 
 // P1 rows hold ~15 entries: one warp per 32 rows when the matrix has rows
 // enough to fill the GPU that way, else 4 lanes per row
