@@ -95,8 +95,8 @@ def _graph(kind, rng):
         from up3d_b200.mesh.kuhn import kuhn_box
         nodes, el = kuhn_box(16, 7, 5)
         return len(nodes), np.vstack([el[:, [i, j]] for i in range(4) for j in range(i)])
-    if kind == "path":          # one-dimensional, odd size: rows of 2 and 3
-        n = 2057
+    if kind.startswith("path"):        # one-dimensional, odd size: rows of 2 and 3
+        n = {"path": 2057, "path512": 1536}[kind]
         return n, np.column_stack([np.arange(n - 1), np.arange(1, n)])
     if kind == "band":          # neighbours up to 14 away: long A P and Galerkin rows
         n = 6000
@@ -108,8 +108,8 @@ def _graph(kind, rng):
     return n, rng.integers(0, n, size=(6 * n, 2))
 
 
-CASES = [("p1", 500, False), ("p1", 30, True), ("path", 10, False), ("path", 600, True), ("band", 40, True),
-         ("band", 500, False), ("grid", 400, False), ("expander", 500, False)]
+CASES = [("p1", 500, False), ("p1", 30, True), ("path", 10, False), ("path", 600, True), ("path", 700, False),
+         ("path512", 512, False), ("band", 40, True), ("band", 500, False), ("grid", 400, False), ("expander", 500, False)]
 
 
 @pytest.mark.parametrize("kind,max_coarse,dirichlet", CASES)

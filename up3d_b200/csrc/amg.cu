@@ -13,7 +13,7 @@
 // Setup, numeric (device, on every setup and refresh): D^-1, rho(D^-1 A) by
 // power iteration, omega = (4/3) / rho, the values of P, A P and R A P in a
 // fixed per-row order, and the dense FP64 inverse of the coarsest operator
-// (Gauss-Jordan with partial pivoting).  A refresh with a new matrix of the
+// (Gauss-Jordan with partial pivoting, coarse_inverse.cuh).  A refresh with a new matrix of the
 // same pattern therefore reproduces a fresh setup bit for bit.
 //
 // Cycle (device): V-cycle with damped-Jacobi pre/post smoothing
@@ -33,6 +33,7 @@
 #include <numeric>
 #include <vector>
 
+#include "coarse_inverse.cuh"
 #include "csr_rows.cuh"
 #include "internal.cuh"
 #include "krylov.cuh"
@@ -956,7 +957,7 @@ struct Amg {
     DBuf<uint8_t> in_dir;
     std::vector<SymLevel*> sym;
     // numeric scratch
-    DBuf<double> pw_xy, pw_scal, omega_dev, dense_a, fcol;
+    DBuf<double> pw_xy, pw_scal, omega_dev, gj_fac, dense_a, fcol;
     DBuf<int> flags;
     std::vector<double> omega;
     DBuf<double> cinv;
@@ -1099,15 +1100,21 @@ void numeric(Amg& a, cudaStream_t s) {
     const SymLevel& Cl = *a.sym.back();
     const int64_t nc = Cl.A.n;
     UP3D_CUDA(cudaMemsetAsync(singular, 0, sizeof(int), s));
-    k_densify<<<grid_for(nc, 128), 128, 0, s>>>(nc, Cl.A.p.get(), Cl.A.i.get(), Cl.A.x.get(), a.dense_a.get(),
-                                                a.cinv.get());
-    UP3D_CHECK_LAUNCH();
-    for (int64_t c = 0; c < nc; ++c) {
-        k_gj_pivot<<<1, 1024, 0, s>>>(a.dense_a.get(), a.cinv.get(), nc, c, a.fcol.get(), singular);
+    if (!launch_gj(nc, Cl.A.p.get(), Cl.A.i.get(), Cl.A.x.get(), a.cinv.get(), a.gj_fac.get(), singular, s)) {
+        // larger than a cluster holds: [A | I] in global memory, two
+        // launches per column
+        a.dense_a.alloc(nc * nc);
+        a.fcol.alloc(nc);
+        k_densify<<<grid_for(nc, 128), 128, 0, s>>>(nc, Cl.A.p.get(), Cl.A.i.get(), Cl.A.x.get(), a.dense_a.get(),
+                                                    a.cinv.get());
         UP3D_CHECK_LAUNCH();
-        k_gj_elim<<<grid_for(2 * nc * nc, 256), 256, 0, s>>>(a.dense_a.get(), a.cinv.get(), nc, c, a.fcol.get(),
-                                                             singular);
-        UP3D_CHECK_LAUNCH();
+        for (int64_t c = 0; c < nc; ++c) {
+            k_gj_pivot<<<1, 1024, 0, s>>>(a.dense_a.get(), a.cinv.get(), nc, c, a.fcol.get(), singular);
+            UP3D_CHECK_LAUNCH();
+            k_gj_elim<<<grid_for(2 * nc * nc, 256), 256, 0, s>>>(a.dense_a.get(), a.cinv.get(), nc, c, a.fcol.get(),
+                                                                 singular);
+            UP3D_CHECK_LAUNCH();
+        }
     }
     int sing = 0;
     a.omega.assign(L > 1 ? L - 1 : 0, 0.0);
@@ -1442,9 +1449,8 @@ void* amg_setup(const up3d_csr& A, const up3d_amg_options& opt, cudaStream_t s) 
         a->pw_scal.alloc(8);
         a->omega_dev.alloc(std::max<size_t>(a->sym.size(), 1));
         a->flags.alloc(2);
-        a->dense_a.alloc(nc * nc);
         a->cinv.alloc(nc * nc);
-        a->fcol.alloc(nc);
+        a->gj_fac.alloc(gj_fac_size(nc));
         k_embed<<<grid_for(a->sym[0]->A.nnz, 256), 256, 0, s>>>(a->sym[0]->A.nnz, a->emb_src.get(), A.data,
                                                                 a->sym[0]->A.x.get());
         UP3D_CHECK_LAUNCH();
