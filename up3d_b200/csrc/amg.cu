@@ -396,81 +396,77 @@ __global__ void k_embed(int64_t nnz, const int32_t* __restrict__ src, const doub
     GRID_STRIDE(k, nnz) out[k] = src[k] >= 0 ? data[src[k]] : 1.0;
 }
 
+// State of the power iteration for rho(D^-1 A): the iterate y (unscaled),
+// z = s y with s = sqrt|D^-1|, and st = (power of two that brings y to unit
+// size, Rayleigh quotient).
 __global__ void k_dinv(int64_t n, const int32_t* __restrict__ diag, const double* __restrict__ Ax,
                        double* __restrict__ dinv, double* __restrict__ s, const double* __restrict__ x0,
-                       double* __restrict__ x) {
+                       double* __restrict__ y, double* __restrict__ z, double* __restrict__ st,
+                       int* __restrict__ done) {
     GRID_STRIDE(r, n) {
         const double d = diag[r] >= 0 ? Ax[diag[r]] : 0.0;
         const double di = d != 0.0 ? __ddiv_rn(1.0, d) : 1.0;
+        const double sr = sqrt(fabs(di));
         dinv[r] = di;
-        s[r] = sqrt(fabs(di));
-        x[r] = x0[r];
+        s[r] = sr;
+        y[r] = x0[r];
+        z[r] = sr * x0[r];
+        if (r == 0) {
+            st[0] = 1.0;
+            st[1] = 0.0;
+            *done = 0;
+        }
     }
 }
 
-// y = skip ? 0 : s * (A (s * x))   (rows of 8 lanes)
-__global__ void __launch_bounds__(256)
-    k_pw_apply(int64_t n, const int32_t* __restrict__ Ap, const int32_t* __restrict__ Ai,
-               const double* __restrict__ Ax, const double* __restrict__ s, const double* __restrict__ x,
-               const uint8_t* __restrict__ skip, double* __restrict__ y, const int* __restrict__ done) {
-    if (*done) return;
-    constexpr int TPR = 8, RPW = 32 / TPR;
-    const int sub = threadIdx.x % TPR, group = (threadIdx.x & 31) / TPR;
+// P = (I - omega D^-1 A) T, contributions in the order (T entry, then A's
+// entries in row order).  Eight lanes per row, lane `sub` owning the P
+// entry at position sub (and sub + 8, ... in further passes): each lane
+// forms the term of one A entry, the row's lanes then see the terms one
+// after the other.  (One thread per row, adding to P in global memory, took
+// 61 us on average over the three levels of the 625 k-row matrix.)
+__global__ void __launch_bounds__(128)
+    k_prolong(int64_t n, const int32_t* __restrict__ Ap, const int32_t* __restrict__ Ai,
+              const double* __restrict__ Ax, const int32_t* __restrict__ amap, const int32_t* __restrict__ self,
+              const double* __restrict__ t, const double* __restrict__ dinv, const double* __restrict__ omega,
+              const int32_t* __restrict__ Pp, double* __restrict__ Px) {
+    const int sub = threadIdx.x & 7;
     const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t n_warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t base = warp * RPW; base < n; base += n_warps * RPW) {
-        const int64_t r = base + group;
-        double acc = 0.0;
-        if (r < n)
-            for (int32_t k = Ap[r] + sub; k < Ap[r + 1]; k += TPR) {
-                const int32_t c = Ai[k];
-                acc += Ax[k] * (s[c] * x[c]);
-            }
+    const double om = *omega;
+    for (int64_t base = warp * 4; base < n; base += n_warps * 4) {   // warp-uniform
+        const int64_t r = base + ((threadIdx.x & 31) >> 3);
+        int32_t pb = 0, pl = 0, s = 0, e = 0, own = -1;
+        double f = 0.0, tr = 0.0;
+        if (r < n) {
+            pb = Pp[r];
+            pl = Pp[r + 1] - pb;
+            s = Ap[r];
+            e = Ap[r + 1];
+            own = self[r];
+            f = __dmul_rn(om, dinv[r]);
+            tr = t[r];
+        }
+        const int len = __reduce_max_sync(0xffffffffu, e - s), most = __reduce_max_sync(0xffffffffu, pl);
+        for (int p0 = 0; p0 < most; p0 += 8) {
+            const int32_t slot = pb + p0 + sub;
+            double acc = slot == own ? tr : 0.0;
+            for (int k0 = 0; k0 < len; k0 += 8) {
+                int32_t q = -1;
+                double v = 0.0;
+                if (s + k0 + sub < e) {
+                    const int32_t k = s + k0 + sub;
+                    q = amap[k];
+                    if (q >= 0) v = __dmul_rn(__dmul_rn(-f, Ax[k]), t[Ai[k]]);
+                }
 #pragma unroll
-        for (int o = TPR / 2; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o, TPR);
-        if (sub == 0 && r < n) y[r] = (skip && skip[r]) ? 0.0 : s[r] * acc;
-    }
-}
-
-// dots = (x.y, y.y, x.x): lambda = x.y / x.x (Rayleigh quotient), stop when
-// y == 0, else normalise (dots[3] = |y|)
-__global__ void k_pw_update(double* __restrict__ dots, double* __restrict__ lam, int* __restrict__ done) {
-    if (*done) return;
-    *lam = dots[2] > 0.0 ? dots[0] / dots[2] : 0.0;
-    if (dots[1] == 0.0) *done = 1;
-    else dots[3] = sqrt(dots[1]);
-}
-
-__global__ void k_pw_norm(int64_t n, const double* __restrict__ y, double* __restrict__ x,
-                          const double* __restrict__ dots, const int* __restrict__ done) {
-    if (*done) return;
-    const double nrm = dots[3];
-    GRID_STRIDE(r, n) x[r] = y[r] / nrm;
-}
-
-// omega = (4/3) / rho with rho = 1.05 lambda (small safety margin on the
-// Rayleigh quotient), 2 when lambda <= 0
-__global__ void k_pw_finish(const double* __restrict__ lam, double* __restrict__ omega) {
-    const double l = *lam;
-    const double rho = l > 0.0 ? 1.05 * l : 2.0;
-    *omega = (4.0 / 3.0) / rho;
-}
-
-// P = (I - omega D^-1 A) T, one row per thread, contributions in the
-// order (T entry, then A's entries in row order)
-__global__ void k_prolong(int64_t n, const int32_t* __restrict__ Ap, const int32_t* __restrict__ Ai,
-                          const double* __restrict__ Ax, const int32_t* __restrict__ amap,
-                          const int32_t* __restrict__ self, const double* __restrict__ t,
-                          const double* __restrict__ dinv, const double* __restrict__ omega,
-                          const int32_t* __restrict__ Pp, double* __restrict__ Px) {
-    GRID_STRIDE(r, n) {
-        for (int32_t q = Pp[r]; q < Pp[r + 1]; ++q) Px[q] = 0.0;
-        if (self[r] >= 0) Px[self[r]] = t[r];
-        const double f = __dmul_rn(*omega, dinv[r]);
-        for (int32_t k = Ap[r]; k < Ap[r + 1]; ++k) {
-            const int32_t q = amap[k];
-            if (q < 0) continue;
-            Px[q] = __dadd_rn(Px[q], __dmul_rn(__dmul_rn(-f, Ax[k]), t[Ai[k]]));
+                for (int j = 0; j < 8; ++j) {
+                    const int32_t qj = __shfl_sync(0xffffffffu, q, j, 8);
+                    const double vj = __shfl_sync(0xffffffffu, v, j, 8);
+                    if (qj == slot) acc = __dadd_rn(acc, vj);
+                }
+            }
+            if (p0 + sub < pl) Px[slot] = acc;
         }
     }
 }
@@ -755,6 +751,81 @@ __device__ __forceinline__ void csr_rows_loop(int64_t n, const int32_t* __restri
     }
 }
 
+// One power-iteration step y' = S A S x, x = st[0] y: writes y' and z' = s y',
+// and the last block to finish turns the blocks' sums of x.y', y'.y', x.x
+// (added in block order) into the Rayleigh quotient st[1] and the next
+// scale; *done stops the steps that follow once y' = 0.  With `omega`, the
+// last step's: omega = (4/3) / rho, rho = 1.05 lambda (a small safety margin
+// on the Rayleigh quotient), 2 when lambda <= 0.  The scale is a power of two
+// so that normalising costs neither rounding nor a pass.  One launch per
+// step; the product, two dots, scalar update and normalisation as five
+// launches took 20 x 45 us on the 625 k-row matrix.
+constexpr int PW_BLOCKS = 148 * 8;
+template <int TPR>
+__global__ void __launch_bounds__(256)
+    k_pw_step(int64_t n, const int32_t* __restrict__ Ap, const int32_t* __restrict__ Ai,
+              const double* __restrict__ Ax, const double* __restrict__ s, const uint8_t* __restrict__ skip,
+              const double* __restrict__ y, const double* __restrict__ z, double* __restrict__ y1,
+              double* __restrict__ z1, double* __restrict__ st, int* __restrict__ done,
+              double* __restrict__ partial, unsigned int* __restrict__ counter, double* __restrict__ omega) {
+    __shared__ double sh[TPR == 0 ? 256 / 32 : 1][TPR == 0 ? CSR_ROWS_CHUNK : 1];
+    __shared__ double sums[3][8];
+    __shared__ bool last;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    auto finish = [&](double lam) {
+        if (omega) *omega = (4.0 / 3.0) / (lam > 0.0 ? 1.05 * lam : 2.0);
+    };
+    if (*done) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) finish(st[1]);
+        return;
+    }
+    const double sc = st[0];
+    double acc[3] = {0.0, 0.0, 0.0};
+    csr_rows_loop<double, TPR>(
+        n, Ap, sh[TPR == 0 ? w : 0], [&](int32_t k) { return Ax[k] * z[Ai[k]]; },
+        [&](int64_t r, double a) {
+            const double v = skip && skip[r] ? 0.0 : s[r] * (sc * a), x = sc * y[r];
+            y1[r] = v;
+            z1[r] = s[r] * v;
+            acc[0] += x * v;
+            acc[1] += v * v;
+            acc[2] += x * x;
+        });
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+        const double v = warp_sum(acc[j]);
+        if (lane == 0) sums[j][w] = v;
+    }
+    __syncthreads();
+    if (threadIdx.x < 3) {
+        double v = 0.0;
+        for (int q = 0; q < 8; ++q) v += sums[threadIdx.x][q];
+        partial[threadIdx.x * PW_BLOCKS + blockIdx.x] = v;
+    }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(counter, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    if (w < 3) {
+        double v = 0.0;
+        for (int b = lane; b < (int)gridDim.x; b += 32) v += __ldcg(partial + w * PW_BLOCKS + b);
+        v = warp_sum(v);
+        if (lane == 0) sums[w][0] = v;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const double xy = sums[0][0], yy = sums[1][0], xx = sums[2][0];
+        const double lam = xx > 0.0 ? xy / xx : 0.0;
+        st[1] = lam;
+        if (yy == 0.0) *done = 1;
+        else st[0] = isfinite(yy) ? ldexp(1.0, -ilogb(sqrt(yy))) : 1.0;
+        finish(lam);
+        *counter = 0u;
+    }
+}
+
 // out = x + w D^-1 (b - A x)   (or, with RESID, out = b - A x).  The finest
 // operator is the embedded one (identity rows, no constrained columns): no
 // mask.
@@ -799,6 +870,17 @@ void launch_sweep(int64_t n, int64_t nnz, const int32_t* Ap, const int32_t* Ai, 
                 k_jacobi_sweep<T, RESID, 32><<<lanes_grid(n, 32), 256, 0, s>>>(n, Ap, Ai, Ax, dinv, b, x, out, w);
         }
     }
+    UP3D_CHECK_LAUNCH();
+}
+
+void launch_pw_step(int64_t n, int64_t nnz, const int32_t* Ap, const int32_t* Ai, const double* Ax, const double* sq,
+                    const uint8_t* skip, const double* y, const double* z, double* y1, double* z1, double* st,
+                    int* done, double* partial, unsigned int* counter, double* omega, cudaStream_t s) {
+    const int tpr = use_warp_rows(n, nnz) ? 0 : lanes_per_row(nnz, n);
+    const unsigned grid = tpr == 0 ? csr_rows_grid(n) : std::min(lanes_grid(n, tpr), (unsigned)PW_BLOCKS);
+    auto kern = tpr == 0 ? k_pw_step<0> : tpr == 4 ? k_pw_step<4> : tpr == 8 ? k_pw_step<8>
+                : tpr == 16 ? k_pw_step<16> : k_pw_step<32>;
+    kern<<<grid, 256, 0, s>>>(n, Ap, Ai, Ax, sq, skip, y, z, y1, z1, st, done, partial, counter, omega);
     UP3D_CHECK_LAUNCH();
 }
 
@@ -957,7 +1039,7 @@ struct Amg {
     DBuf<uint8_t> in_dir;
     std::vector<SymLevel*> sym;
     // numeric scratch
-    DBuf<double> pw_xy, pw_scal, omega_dev, gj_fac, dense_a, fcol;
+    DBuf<double> pw_yz, pw_scal, omega_dev, gj_fac, dense_a, fcol;
     DBuf<int> flags;
     std::vector<double> omega;
     DBuf<double> cinv;
@@ -977,9 +1059,6 @@ struct Amg {
     std::vector<Graph> graphs;
     cudaStream_t capture_stream = nullptr;
     int device = 0;
-    // the numeric phase's vector kernels (kept: set-up and every refresh
-    // would otherwise allocate and free its scratch and pinned readback)
-    std::unique_ptr<Blas> blas;
     void drop_graphs() {
         for (auto& g : graphs) cudaGraphExecDestroy(g.exec);
         graphs.clear();
@@ -1055,41 +1134,35 @@ int longest_row(const HostCSR& A) {
 // operator, then the coarsest inverse; fills the cycle's levels.
 void numeric(Amg& a, cudaStream_t s) {
     const size_t L = a.sym.size();
-    if (!a.blas) a.blas.reset(new Blas(s));
-    Blas& blas = *a.blas;
-    blas.s = s;
-    double* dots = a.pw_scal.get();       // x.y, y.y, x.x, |y|
-    double* lam = a.pw_scal.get() + 4;
+    double* st = a.pw_scal.get();
+    double* partial = a.pw_scal.get() + 2;
+    unsigned int* counter = reinterpret_cast<unsigned int*>(a.flags.get() + 2);
+    UP3D_CUDA(cudaMemsetAsync(counter, 0, sizeof(unsigned int), s));
     int* done = a.flags.get();
     int* singular = a.flags.get() + 1;
     for (size_t l = 0; l + 1 < L; ++l) {
         SymLevel& F = *a.sym[l];
         SymLevel& C = *a.sym[l + 1];
         const int64_t n = F.A.n;
-        double* x = a.pw_xy.get();
-        double* y = a.pw_xy.get() + n;
+        double* y = a.pw_yz.get();
+        double* z = y + n;
+        double* y1 = z + n;
+        double* z1 = y1 + n;
         k_dinv<<<grid_for(n, 256), 256, 0, s>>>(n, F.diag.get(), F.A.x.get(), F.dinv.get(), F.sq.get(),
-                                                F.x0.get(), x);
+                                                F.x0.get(), y, z, st, done);
         UP3D_CHECK_LAUNCH();
-        UP3D_CUDA(cudaMemsetAsync(done, 0, sizeof(int), s));
-        UP3D_CUDA(cudaMemsetAsync(lam, 0, sizeof(double), s));
-        const unsigned g8 = grid_for(8 * n, 256, (int64_t)148 * 64);
-        for (int it = 0; it < 20; ++it) {
-            k_pw_apply<<<g8, 256, 0, s>>>(n, F.A.p.get(), F.A.i.get(), F.A.x.get(), F.sq.get(), x,
-                                          F.has_skip ? F.skip.get() : nullptr, y, done);
-            UP3D_CHECK_LAUNCH();
-            blas.multidot(x, n, 2, y, n, dots);   // (x.y, y.y)
-            blas.multidot(x, 0, 1, x, n, dots + 2);
-            k_pw_update<<<1, 1, 0, s>>>(dots, lam, done);
-            UP3D_CHECK_LAUNCH();
-            k_pw_norm<<<grid_for(n, 256), 256, 0, s>>>(n, y, x, dots, done);
-            UP3D_CHECK_LAUNCH();
+        constexpr int PW_STEPS = 20;
+        for (int it = 0; it < PW_STEPS; ++it) {
+            launch_pw_step(n, F.A.nnz, F.A.p.get(), F.A.i.get(), F.A.x.get(), F.sq.get(),
+                           F.has_skip ? F.skip.get() : nullptr, y, z, y1, z1, st, done, partial, counter,
+                           it + 1 == PW_STEPS ? a.omega_dev.get() + l : nullptr, s);
+            std::swap(y, y1);
+            std::swap(z, z1);
         }
-        k_pw_finish<<<1, 1, 0, s>>>(lam, a.omega_dev.get() + l);
-        UP3D_CHECK_LAUNCH();
-        k_prolong<<<grid_for(n, 128), 128, 0, s>>>(n, F.A.p.get(), F.A.i.get(), F.A.x.get(), F.amap.get(),
-                                                   F.self.get(), F.t.get(), F.dinv.get(), a.omega_dev.get() + l,
-                                                   F.P.p.get(), F.P.x.get());
+        k_prolong<<<grid_for(n, 16, (int64_t)148 * 64), 128, 0, s>>>(n, F.A.p.get(), F.A.i.get(), F.A.x.get(),
+                                                                     F.amap.get(), F.self.get(), F.t.get(),
+                                                                     F.dinv.get(), a.omega_dev.get() + l,
+                                                                     F.P.p.get(), F.P.x.get());
         UP3D_CHECK_LAUNCH();
         k_gather_vals<<<grid_for(F.R.nnz, 256), 256, 0, s>>>(F.R.nnz, F.tperm.get(), F.P.x.get(), F.R.x.get());
         UP3D_CHECK_LAUNCH();
@@ -1445,10 +1518,10 @@ void* amg_setup(const up3d_csr& A, const up3d_amg_options& opt, cudaStream_t s) 
         const int64_t nc = As.back().n;
         UP3D_REQUIRE(nc <= 8192, UP3D_ERR_RUNTIME, "AMG coarsest level too large for the dense solve");
         a->n_coarse = nc;
-        a->pw_xy.alloc(2 * nmax);
-        a->pw_scal.alloc(8);
+        a->pw_yz.alloc(4 * nmax);
+        a->pw_scal.alloc(2 + 3 * PW_BLOCKS);
         a->omega_dev.alloc(std::max<size_t>(a->sym.size(), 1));
-        a->flags.alloc(2);
+        a->flags.alloc(3);
         a->cinv.alloc(nc * nc);
         a->gj_fac.alloc(gj_fac_size(nc));
         k_embed<<<grid_for(a->sym[0]->A.nnz, 256), 256, 0, s>>>(a->sym[0]->A.nnz, a->emb_src.get(), A.data,
