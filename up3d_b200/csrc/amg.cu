@@ -728,16 +728,23 @@ __global__ void k_jacobi_first(const T* __restrict__ dinv, const T* __restrict__
 }
 
 // Row loop shared by the CSR kernels below: TPR = 0 is one warp per 32
-// rows (csr_rows.cuh warp_row_sum), else TPR lanes per row; epi(r, acc)
-// writes row r (called once per row, by one lane).
-template <class T, int TPR, class Prod, class Epi>
-__device__ __forceinline__ void csr_rows_loop(int64_t n, const int32_t* __restrict__ Ap, T* sh, Prod prod, Epi epi) {
-    const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    const int64_t n_warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+// rows (csr_rows.cuh warp_row_sum), else TPR lanes per row; the row's sum of
+// A_rc x_c goes to epi(r, acc), called once per row, by one lane.  BLOCK
+// threads per block.
+template <int TPR>
+constexpr int rows_block = TPR == 0 ? CSR_WARP_BLOCK : CSR_ROWS_BLOCK;
+template <class T, int TPR, int BLOCK, class Epi>
+__device__ __forceinline__ void csr_rows_loop(int64_t n, const int32_t* __restrict__ Ap,
+                                              const int32_t* __restrict__ Ai, const T* __restrict__ Ax,
+                                              const T* __restrict__ x, Epi epi) {
+    const int64_t warp = (blockIdx.x * (int64_t)BLOCK + threadIdx.x) >> 5;
+    const int64_t n_warps = ((int64_t)gridDim.x * BLOCK) >> 5;
+    auto term = [&](int32_t c, T v) { return v * x[c]; };
     if constexpr (TPR == 0) {
+        __shared__ T sh[BLOCK / 32][CSR_ROWS_CHUNK];
         const int lane = threadIdx.x & 31;
         for (int64_t r0 = warp * 32; r0 < n; r0 += n_warps * 32) {   // warp-uniform
-            const T acc = warp_row_sum<T>(Ap, r0, n, sh, prod);
+            const T acc = warp_row_sum<T>(Ap, Ai, Ax, r0, n, sh[threadIdx.x >> 5], term);
             if (r0 + lane < n) epi(r0 + lane, acc);
         }
     } else {
@@ -745,7 +752,7 @@ __device__ __forceinline__ void csr_rows_loop(int64_t n, const int32_t* __restri
         const int sub = threadIdx.x % TPR, group = (threadIdx.x & 31) / TPR;
         for (int64_t base = warp * RPW; base < n; base += n_warps * RPW) {   // warp-uniform
             const int64_t r = base + group;
-            const T acc = lanes_row_sum<T, TPR>(Ap, r, n, prod);
+            const T acc = lanes_row_sum<T, TPR>(Ap, Ai, Ax, r, n, term);
             if (sub == 0 && r < n) epi(r, acc);
         }
     }
@@ -768,7 +775,6 @@ __global__ void __launch_bounds__(256)
               const double* __restrict__ y, const double* __restrict__ z, double* __restrict__ y1,
               double* __restrict__ z1, double* __restrict__ st, int* __restrict__ done,
               double* __restrict__ partial, unsigned int* __restrict__ counter, double* __restrict__ omega) {
-    __shared__ double sh[TPR == 0 ? 256 / 32 : 1][TPR == 0 ? CSR_ROWS_CHUNK : 1];
     __shared__ double sums[3][8];
     __shared__ bool last;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -781,16 +787,14 @@ __global__ void __launch_bounds__(256)
     }
     const double sc = st[0];
     double acc[3] = {0.0, 0.0, 0.0};
-    csr_rows_loop<double, TPR>(
-        n, Ap, sh[TPR == 0 ? w : 0], [&](int32_t k) { return Ax[k] * z[Ai[k]]; },
-        [&](int64_t r, double a) {
-            const double v = skip && skip[r] ? 0.0 : s[r] * (sc * a), x = sc * y[r];
-            y1[r] = v;
-            z1[r] = s[r] * v;
-            acc[0] += x * v;
-            acc[1] += v * v;
-            acc[2] += x * x;
-        });
+    csr_rows_loop<double, TPR, 256>(n, Ap, Ai, Ax, z, [&](int64_t r, double a) {
+        const double v = skip && skip[r] ? 0.0 : s[r] * (sc * a), x = sc * y[r];
+        y1[r] = v;
+        z1[r] = s[r] * v;
+        acc[0] += x * v;
+        acc[1] += v * v;
+        acc[2] += x * x;
+    });
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
         const double v = warp_sum(acc[j]);
@@ -830,35 +834,67 @@ __global__ void __launch_bounds__(256)
 // operator is the embedded one (identity rows, no constrained columns): no
 // mask.
 template <class T, bool RESID, int TPR>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(rows_block<TPR>)
     k_jacobi_sweep(int64_t n, const int32_t* __restrict__ Ap, const int32_t* __restrict__ Ai,
                    const T* __restrict__ Ax, const T* __restrict__ dinv, const T* __restrict__ b,
                    const T* __restrict__ x, T* __restrict__ out, T w) {
-    __shared__ T sh[TPR == 0 ? 256 / 32 : 1][TPR == 0 ? CSR_ROWS_CHUNK : 1];
-    csr_rows_loop<T, TPR>(
-        n, Ap, sh[TPR == 0 ? threadIdx.x >> 5 : 0], [&](int32_t k) { return Ax[k] * x[Ai[k]]; },
-        [&](int64_t r, T acc) {
-            const T res = b[r] - acc;
-            out[r] = RESID ? res : x[r] + w * dinv[r] * res;
-        });
+    csr_rows_loop<T, TPR, rows_block<TPR>>(n, Ap, Ai, Ax, x, [&](int64_t r, T acc) {
+        const T res = b[r] - acc;
+        out[r] = RESID ? res : x[r] + w * dinv[r] * res;
+    });
+}
+
+// The same sweep on the sliced rows, one row per lane.
+template <class T, bool RESID>
+__global__ void __launch_bounds__(SELL_BLOCK)
+    k_jacobi_sell(int64_t n, const int32_t* __restrict__ Sp, const int32_t* __restrict__ Si,
+                  const T* __restrict__ Sx, const T* __restrict__ dinv, const T* __restrict__ b,
+                  const T* __restrict__ x, T* __restrict__ out, T w) {
+    const int64_t r = blockIdx.x * (int64_t)SELL_BLOCK + threadIdx.x;
+    const int lane = threadIdx.x & 31;
+    if (r - lane >= n) return;   // warp-uniform
+    const T acc = sell_row_sum<T>(Sp, Si, Sx, x, r >> 5, lane);
+    if (r >= n) return;
+    const T res = b[r] - acc;
+    out[r] = RESID ? res : x[r] + w * dinv[r] * res;
+}
+
+// Column indices of the sliced rows from the CSR ones (-1 on the padding),
+// and the values at the cycle's precision.
+__global__ void k_sell_index(int64_t n, const int32_t* __restrict__ Ap, const int32_t* __restrict__ Ai,
+                             const int32_t* __restrict__ Sp, int32_t* __restrict__ Si) {
+    GRID_STRIDE(r, (n + 31) / 32 * 32) {   // the last slice's unused lanes are padding too
+        const int64_t q = r >> 5;
+        const int32_t s = Sp[q] + (int32_t)(r & 31), w = (Sp[q + 1] - Sp[q]) >> 5;
+        const int32_t p = r < n ? Ap[r] : 0, len = r < n ? Ap[r + 1] - p : 0;
+        for (int32_t k = 0; k < w; ++k) Si[s + 32 * k] = k < len ? Ai[p + k] : -1;
+    }
+}
+template <class T>
+__global__ void k_sell_values(int64_t n, const int32_t* __restrict__ Ap, const double* __restrict__ Ax,
+                              const int32_t* __restrict__ Sp, T* __restrict__ Sx) {
+    GRID_STRIDE(r, (n + 31) / 32 * 32) {   // the last slice's unused lanes are padding too
+        const int64_t q = r >> 5;
+        const int32_t s = Sp[q] + (int32_t)(r & 31), w = (Sp[q + 1] - Sp[q]) >> 5;
+        const int32_t p = r < n ? Ap[r] : 0, len = r < n ? Ap[r + 1] - p : 0;
+        for (int32_t k = 0; k < w; ++k) Sx[s + 32 * k] = k < len ? (T)Ax[p + k] : T(0);
+    }
 }
 
 // y (+)= A x, rectangular (restriction / prolongation)
 template <class T, bool ADD, int TPR>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(rows_block<TPR>)
     k_spmv_rect(int64_t n, const int32_t* __restrict__ Ap, const int32_t* __restrict__ Ai, const T* __restrict__ Ax,
                 const T* __restrict__ x, T* __restrict__ y) {
-    __shared__ T sh[TPR == 0 ? 256 / 32 : 1][TPR == 0 ? CSR_ROWS_CHUNK : 1];
-    csr_rows_loop<T, TPR>(
-        n, Ap, sh[TPR == 0 ? threadIdx.x >> 5 : 0], [&](int32_t k) { return Ax[k] * x[Ai[k]]; },
-        [&](int64_t r, T acc) { y[r] = ADD ? y[r] + acc : acc; });
+    csr_rows_loop<T, TPR, rows_block<TPR>>(n, Ap, Ai, Ax, x,
+                                           [&](int64_t r, T acc) { y[r] = ADD ? y[r] + acc : acc; });
 }
 
 template <class T, bool RESID>
 void launch_sweep(int64_t n, int64_t nnz, const int32_t* Ap, const int32_t* Ai, const T* Ax, const T* dinv,
                   const T* b, const T* x, T* out, T w, cudaStream_t s) {
     if (use_warp_rows(n, nnz)) {
-        k_jacobi_sweep<T, RESID, 0><<<csr_rows_grid(n), 256, 0, s>>>(n, Ap, Ai, Ax, dinv, b, x, out, w);
+        k_jacobi_sweep<T, RESID, 0><<<csr_rows_grid(n, CSR_WARP_BLOCK), CSR_WARP_BLOCK, 0, s>>>(n, Ap, Ai, Ax, dinv, b, x, out, w);
     } else {
         switch (lanes_per_row(nnz, n)) {
             case 4: k_jacobi_sweep<T, RESID, 4><<<lanes_grid(n, 4), 256, 0, s>>>(n, Ap, Ai, Ax, dinv, b, x, out, w); break;
@@ -877,7 +913,7 @@ void launch_pw_step(int64_t n, int64_t nnz, const int32_t* Ap, const int32_t* Ai
                     const uint8_t* skip, const double* y, const double* z, double* y1, double* z1, double* st,
                     int* done, double* partial, unsigned int* counter, double* omega, cudaStream_t s) {
     const int tpr = use_warp_rows(n, nnz) ? 0 : lanes_per_row(nnz, n);
-    const unsigned grid = tpr == 0 ? csr_rows_grid(n) : std::min(lanes_grid(n, tpr), (unsigned)PW_BLOCKS);
+    const unsigned grid = tpr == 0 ? std::min(csr_rows_grid(n, 256), (unsigned)PW_BLOCKS) : std::min(lanes_grid(n, tpr), (unsigned)PW_BLOCKS);
     auto kern = tpr == 0 ? k_pw_step<0> : tpr == 4 ? k_pw_step<4> : tpr == 8 ? k_pw_step<8>
                 : tpr == 16 ? k_pw_step<16> : k_pw_step<32>;
     kern<<<grid, 256, 0, s>>>(n, Ap, Ai, Ax, sq, skip, y, z, y1, z1, st, done, partial, counter, omega);
@@ -888,7 +924,7 @@ template <class T, bool ADD>
 void launch_rect(int64_t n, int64_t nnz, const int32_t* Ap, const int32_t* Ai, const T* Ax, const T* x, T* y,
                  cudaStream_t s) {
     if (use_warp_rows(n, nnz)) {
-        k_spmv_rect<T, ADD, 0><<<csr_rows_grid(n), 256, 0, s>>>(n, Ap, Ai, Ax, x, y);
+        k_spmv_rect<T, ADD, 0><<<csr_rows_grid(n, CSR_WARP_BLOCK), CSR_WARP_BLOCK, 0, s>>>(n, Ap, Ai, Ax, x, y);
     } else {
         switch (lanes_per_row(nnz, n)) {
             case 4: k_spmv_rect<T, ADD, 4><<<lanes_grid(n, 4), 256, 0, s>>>(n, Ap, Ai, Ax, x, y); break;
@@ -1005,6 +1041,9 @@ template <class T>
 struct Level {
     CsrRef<T> A, P, R;
     Ref<T> dinv;
+    const int32_t* sell_p = nullptr;        // A in slices of 32 rows, when it is kept that way
+    const int32_t* sell_i = nullptr;
+    DBuf<T> sell_x;
     DBuf<T> own_A, own_P, own_R, own_dinv;  // FP32 values (unused for FP64)
     DBuf<T> x, b, r;
     T w_smooth = T(0);
@@ -1023,6 +1062,8 @@ struct SymLevel {
     DBuf<int32_t> tperm;         // R entry -> P entry
     int a_max = 0, ap_max = 0;   // longest rows of A and A P
     bool has_skip = false;
+    DBuf<int32_t> sell_p, sell_i;   // A's slices (sell_n = 0: not kept)
+    int64_t sell_n = 0;
 };
 
 }  // namespace
@@ -1074,6 +1115,21 @@ struct Amg {
 
 namespace {
 
+// One sweep (or residual) of a level's operator: the sliced rows where the
+// level has them, else the CSR rows.
+template <class T, bool RESID>
+void smooth(const Level<T>& lv, const T* x, T* out, cudaStream_t s) {
+    const int64_t n = lv.A.n;
+    if (!lv.sell_p) {
+        launch_sweep<T, RESID>(n, lv.A.nnz, lv.A.p.get(), lv.A.i.get(), lv.A.x.get(), lv.dinv.get(), lv.b.get(), x, out,
+                               lv.w_smooth, s);
+        return;
+    }
+    k_jacobi_sell<T, RESID><<<sell_grid(n), SELL_BLOCK, 0, s>>>(n, lv.sell_p, lv.sell_i, lv.sell_x.get(),
+                                                               lv.dinv.get(), lv.b.get(), x, out, lv.w_smooth);
+    UP3D_CHECK_LAUNCH();
+}
+
 template <class T>
 void vcycle(Amg& a, std::vector<Level<T>*>& L, size_t l, cudaStream_t s) {
     Level<T>& lv = *L[l];
@@ -1089,26 +1145,22 @@ void vcycle(Amg& a, std::vector<Level<T>*>& L, size_t l, cudaStream_t s) {
         return;
     }
     const unsigned g1 = grid_for(n, 256);
-    const int64_t nnz = lv.A.nnz;
     // pre-smoothing from x = 0
     k_jacobi_first<T><<<g1, 256, 0, s>>>(lv.dinv.get(), lv.b.get(), lv.x.get(), lv.w_smooth, n);
     UP3D_CHECK_LAUNCH();
     for (int k = 1; k < a.pre; ++k) {
-        launch_sweep<T, false>(n, nnz, lv.A.p.get(), lv.A.i.get(), lv.A.x.get(), lv.dinv.get(), lv.b.get(),
-                               lv.x.get(), lv.r.get(), lv.w_smooth, s);
+        smooth<T, false>(lv, lv.x.get(), lv.r.get(), s);
         std::swap(lv.x.p, lv.r.p);
     }
     // residual, restriction
-    launch_sweep<T, true>(n, nnz, lv.A.p.get(), lv.A.i.get(), lv.A.x.get(), lv.dinv.get(), lv.b.get(), lv.x.get(),
-                          lv.r.get(), lv.w_smooth, s);
+    smooth<T, true>(lv, lv.x.get(), lv.r.get(), s);
     Level<T>& cv = *L[l + 1];
     launch_rect<T, false>(lv.R.n, lv.R.nnz, lv.R.p.get(), lv.R.i.get(), lv.R.x.get(), lv.r.get(), cv.b.get(), s);
     vcycle<T>(a, L, l + 1, s);
     // prolongation
     launch_rect<T, true>(lv.P.n, lv.P.nnz, lv.P.p.get(), lv.P.i.get(), lv.P.x.get(), cv.x.get(), lv.x.get(), s);
     for (int k = 0; k < a.post; ++k) {
-        launch_sweep<T, false>(n, nnz, lv.A.p.get(), lv.A.i.get(), lv.A.x.get(), lv.dinv.get(), lv.b.get(),
-                               lv.x.get(), lv.r.get(), lv.w_smooth, s);
+        smooth<T, false>(lv, lv.x.get(), lv.r.get(), s);
         std::swap(lv.x.p, lv.r.p);
     }
 }
@@ -1128,6 +1180,27 @@ int longest_row(const HostCSR& A) {
 #pragma omp parallel for schedule(static) reduction(max : m)
     for (int64_t r = 0; r < A.n; ++r) m = std::max(m, A.p[r + 1] - A.p[r]);
     return m;
+}
+
+// Slices of a level operator (symbolic), when the sliced rows pay.
+void make_slices(SymLevel& F, const HostCSR& A, cudaStream_t s) {
+    const int64_t nq = (A.n + 31) / 32;
+    std::vector<int32_t> sp(nq + 1, 0);
+    int64_t run = 0;
+    for (int64_t q = 0; q < nq; ++q) {
+        int32_t w = 0;
+        for (int64_t r = 32 * q; r < std::min(A.n, 32 * q + 32); ++r) w = std::max(w, A.p[r + 1] - A.p[r]);
+        run += 32 * (int64_t)w;
+        if (run > INT32_MAX) return;
+        sp[q + 1] = (int32_t)run;
+    }
+    if (!use_sell(A.n, (int64_t)A.i.size(), run)) return;
+    upload(F.sell_p, sp, s);
+    F.sell_i.alloc(run);
+    F.sell_n = run;
+    k_sell_index<<<grid_for(A.n, 256), 256, 0, s>>>(A.n, F.A.p.get(), F.A.i.get(), F.sell_p.get(), F.sell_i.get());
+    UP3D_CHECK_LAUNCH();
+    UP3D_CUDA(cudaStreamSynchronize(s));
 }
 
 // Device numeric phase: every level's D^-1, omega, P, R, A P and coarser
@@ -1229,7 +1302,13 @@ void fill_levels(Amg& a, std::vector<Level<T>*>& Lv, cudaStream_t s) {
     for (size_t l = 0; l < a.sym.size(); ++l) {
         SymLevel& F = *a.sym[l];
         Level<T>& lv = *Lv[l];
-        if constexpr (!std::is_same<T, double>::value) convert<T>(F.A.x.get(), lv.A.x.get(), F.A.nnz, s);
+        if (lv.sell_p) {
+            k_sell_values<T><<<grid_for(F.A.n, 256), 256, 0, s>>>(F.A.n, F.A.p.get(), F.A.x.get(), lv.sell_p,
+                                                                  lv.sell_x.get());
+            UP3D_CHECK_LAUNCH();
+        } else if constexpr (!std::is_same<T, double>::value) {
+            convert<T>(F.A.x.get(), lv.A.x.get(), F.A.nnz, s);
+        }
         if (l + 1 < a.sym.size()) {
             if constexpr (!std::is_same<T, double>::value) {
                 convert<T>(F.P.x.get(), lv.P.x.get(), F.P.nnz, s);
@@ -1262,8 +1341,16 @@ void make_levels(Amg& a, std::vector<Level<T>*>& Lv, cudaStream_t s) {
         SymLevel& F = *a.sym[l];
         auto* lv = new Level<T>();
         Lv.push_back(lv);
-        view(lv->A, F.A, lv->own_A);
         const int64_t n = F.A.n;
+        if (F.sell_n && l + 1 < a.sym.size()) {
+            lv->A.n = lv->A.m = n;
+            lv->A.nnz = F.A.nnz;
+            lv->sell_p = F.sell_p.get();
+            lv->sell_i = F.sell_i.get();
+            lv->sell_x.alloc(F.sell_n);
+        } else {
+            view(lv->A, F.A, lv->own_A);
+        }
         lv->x.alloc(n);
         lv->b.alloc(n);
         lv->r.alloc(n);
@@ -1481,6 +1568,7 @@ void* amg_setup(const up3d_csr& A, const up3d_amg_options& opt, cudaStream_t s) 
             a->sym.push_back(F);
             F->A.upload_pattern(Al, s);
             F->a_max = longest_row(Al);
+            make_slices(*F, Al, s);
             upload(F->diag, diag_slots(Al), s);
             F->has_skip = a->sym.size() == 1 && a->has_dir;
             if (F->has_skip) upload(F->skip, cur_skip, s);

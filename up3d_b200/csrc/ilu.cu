@@ -145,9 +145,8 @@ __global__ void __launch_bounds__(256)
     const int64_t n_warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     for (int64_t base = warp * RPW; base < n; base += n_warps * RPW) {   // warp-uniform
         const int64_t r = base + group;
-        const double acc = lanes_row_sum<double, TPR>(p, r, n, [&](int32_t e) {
-            const int32_t c = ci[e];
-            return (LOWER ? c < r : c > r) ? lu[e] * y[c] : 0.0;
+        const double acc = lanes_row_sum<double, TPR>(p, ci, lu, r, n, [&](int32_t c, double v) {
+            return (LOWER ? c < r : c > r) ? v * y[c] : 0.0;
         });
         if (sub == 0 && r < n) y_new[r] = LOWER ? b[r] - acc : (b[r] - acc) / lu[diag[r]];
     }

@@ -19,29 +19,23 @@ namespace {
 // mask, constrained rows give y = x and constrained columns are dropped.
 // TPR = 0: one warp per 32 rows; else TPR lanes per row.
 template <class T, int TPR>
-__global__ void __launch_bounds__(CSR_ROWS_BLOCK)
+__global__ void __launch_bounds__(TPR == 0 ? CSR_WARP_BLOCK : CSR_ROWS_BLOCK)
     k_spmv(int64_t n, const int32_t* __restrict__ indptr, const int32_t* __restrict__ indices,
            const T* __restrict__ data, const int32_t* __restrict__ xptr, const int32_t* __restrict__ xidx,
            const T* __restrict__ xdata, const T* __restrict__ x, T* __restrict__ y, const uint8_t* __restrict__ dir) {
-    auto p1 = [&](int32_t k) {
-        const int32_t c = indices[k];
-        const T v = data[k] * x[c];
-        return (dir && dir[c]) ? T(0) : v;
-    };
-    auto p3 = [&](int32_t k) {
-        const int32_t c = xidx[k];
-        const T v = xdata[k] * x[c];
-        return (dir && dir[c]) ? T(0) : v;
+    auto term = [&](int32_t c, T v) {
+        const T p = v * x[c];   // beside the mask's load, not behind it
+        return (dir && dir[c]) ? T(0) : p;
     };
     const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t n_warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     if constexpr (TPR == 0) {
-        __shared__ T sh[CSR_ROWS_BLOCK / 32][CSR_ROWS_CHUNK];
+        __shared__ T sh[CSR_WARP_BLOCK / 32][CSR_ROWS_CHUNK];
         T* my = sh[threadIdx.x >> 5];
         const int lane = threadIdx.x & 31;
         for (int64_t r0 = warp * 32; r0 < n; r0 += n_warps * 32) {   // warp-uniform
-            T acc = warp_row_sum<T>(indptr, r0, n, my, p1);
-            if (xptr) acc += warp_row_sum<T>(xptr, r0, n, my, p3);
+            T acc = warp_row_sum<T>(indptr, indices, data, r0, n, my, term);
+            if (xptr) acc += warp_row_sum<T>(xptr, xidx, xdata, r0, n, my, term);
             const int64_t r = r0 + lane;
             if (r < n) y[r] = (dir && dir[r]) ? x[r] : acc;
         }
@@ -50,8 +44,8 @@ __global__ void __launch_bounds__(CSR_ROWS_BLOCK)
         const int sub = threadIdx.x % TPR, group = (threadIdx.x & 31) / TPR;
         for (int64_t base = warp * RPW; base < n; base += n_warps * RPW) {   // warp-uniform
             const int64_t r = base + group;
-            T acc = lanes_row_sum<T, TPR>(indptr, r, n, p1);
-            if (xptr) acc += lanes_row_sum<T, TPR>(xptr, r, n, p3);
+            T acc = lanes_row_sum<T, TPR>(indptr, indices, data, r, n, term);
+            if (xptr) acc += lanes_row_sum<T, TPR>(xptr, xidx, xdata, r, n, term);
             if (sub == 0 && r < n) y[r] = (dir && dir[r]) ? x[r] : acc;
         }
     }
@@ -127,8 +121,8 @@ template <class T>
 void launch_spmv2(int64_t n, const int32_t* indptr, const int32_t* indices, const T* data, const int32_t* xptr,
                   const int32_t* xidx, const T* xdata, const T* x, T* y, const uint8_t* dir, cudaStream_t s) {
     if (n >= CSR_ROWS_MIN_ROWS)
-        k_spmv<T, 0><<<csr_rows_grid(n), CSR_ROWS_BLOCK, 0, s>>>(n, indptr, indices, data, xptr, xidx, xdata, x, y,
-                                                                 dir);
+        k_spmv<T, 0><<<csr_rows_grid(n, CSR_WARP_BLOCK), CSR_WARP_BLOCK, 0, s>>>(n, indptr, indices, data, xptr, xidx,
+                                                                                 xdata, x, y, dir);
     else
         k_spmv<T, 4><<<lanes_grid(n, 4), CSR_ROWS_BLOCK, 0, s>>>(n, indptr, indices, data, xptr, xidx, xdata, x, y,
                                                                  dir);
