@@ -17,82 +17,180 @@
 
 #include "internal.cuh"
 #include "krylov.cuh"
+#include "reduce.cuh"
 
 namespace up3d {
 
 namespace {
 
-constexpr int RB = 256;      // reduction block
-constexpr int RGRID = 592;   // fixed partial count (4 x 148 SMs): reproducible sums
-
 #define GRID_STRIDE(i, n) \
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < (n); i += (int64_t)gridDim.x * blockDim.x)
 
-// Called by every thread of every block after the block has written its
-// partials: the last block to arrive sums partial[b * K + k] over b for
-// each k into out (lanes stride b, then a warp sum: a fixed order)
-// and re-arms the counter for the next launch on the stream.
-__device__ __forceinline__ void last_block_finish(const double* partial, int nb, int K, double* out,
-                                                  unsigned int* counter) {
-    __shared__ bool last;
-    const unsigned int blocks = gridDim.x * gridDim.y;
-    __threadfence();
+// out = x . y; products and sums in FP64 whatever the vector type.
+template <class T>
+__global__ void __launch_bounds__(DOT_BLOCK)
+    k_dot(const T* __restrict__ x, const T* __restrict__ y, int64_t n, double* __restrict__ partial,
+          double* __restrict__ out, unsigned int* __restrict__ counter) {
+    __shared__ double sh[DOT_BLOCK / 32];
+    double acc = 0.0;
+    GRID_STRIDE(i, n) acc += (double)x[i] * (double)y[i];
+    acc = block_sum(acc, sh);
+    if (threadIdx.x == 0) partial[blockIdx.x] = acc;
+    if (!last_block(counter)) return;
+    acc = sum_partials(partial, (int)gridDim.x, sh);
+    if (threadIdx.x == 0) {
+        *out = acc;
+        *counter = 0u;
+    }
+}
+
+// One sweep over K <= 64 basis vectors V_k (ldv apart, 16-byte aligned) and a
+// vector y:
+//   BASIS_DOTS       out[k] = V_k . y, and out[K] = y . y with `self`
+//   BASIS_AXPY_DOTS  y -= sum_k h[k] V_k, then out[k] = V_k . y of the new y, and
+//                    h[k] += out[k] (the two Gram-Schmidt passes' coefficients)
+//   BASIS_AXPY_NORM  y -= sum_k h[k] V_k, then out[0] = y . y
+// so each pass of a CGS2 Arnoldi step reads the basis once.  A block takes
+// tiles of 32 VEC rows (16-byte loads, VEC rows per lane); warp w of its 8
+// holds the values of the vectors k = w + 8 j, j < KJ, in registers, the
+// update's eight partial sums meet in shared memory, and every lane adds its
+// own dot products across tiles, summed over the warp once at the end.
+// Products and sums in FP64 whatever the vector type; the last block adds
+// the blocks' sums (a fixed order).  Bound by the basis's bytes: 625 k rows
+// and 25-32 FP32 vectors (62-80 MB) 23 us, 49-56 (122-140 MB) 35-38 us a pass.
+// A row per lane with all its values in registers took 30 and 50 us (the
+// dots' 94 shuffles per warp); 8 vectors per block group and a second read of
+// the basis for the dots 39 us (dots) and 42 us (update with dots) at 30.
+enum BasisPass { BASIS_DOTS, BASIS_AXPY_DOTS, BASIS_AXPY_NORM };
+constexpr int BASIS_MAX = 64, BASIS_WARPS = DOT_BLOCK / 32;
+constexpr int BASIS_MAX_BLOCKS = 148 * 6;
+// resident blocks per SM aimed at: the registers that a lane's values (16
+// bytes a vector, of two tiles) take
+template <int KJ>
+constexpr int basis_blocks = KJ == 1 ? 6 : KJ == 2 ? 4 : KJ <= 4 ? 3 : 2;
+template <class T, int KJ, int PASS>
+__global__ void __launch_bounds__(DOT_BLOCK, basis_blocks<KJ>)
+    k_basis(const T* __restrict__ V, int64_t ldv, int K, double* h, T* y, int64_t n, bool self,
+            double* __restrict__ partial, double* __restrict__ out, unsigned int* __restrict__ counter) {
+    constexpr int VEC = 16 / sizeof(T), ROWS = 32 * VEC;
+    struct alignas(16) Vec {
+        T x[VEC];
+    };
+    __shared__ alignas(16) double part[BASIS_WARPS][ROWS];   // the update's partial sums, by row
+    __shared__ alignas(16) double fresh[ROWS];               // the updated y
+    __shared__ double sums[8 * KJ + 1];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    double hw[KJ];
+#pragma unroll
+    for (int j = 0; j < KJ; ++j) hw[j] = PASS != BASIS_DOTS && w + 8 * j < K ? h[w + 8 * j] : 0.0;
+    double acc[KJ], yy = 0.0;
+#pragma unroll
+    for (int j = 0; j < KJ; ++j) acc[j] = 0.0;
+    // the tile's values are loaded while the tile before is worked on
+    Vec nv[KJ], ny = {};
+    T nf = T(0);   // y of the row this thread updates (threads below ROWS)
+    auto load = [&](const T* p, int64_t i) {
+        Vec v;
+        if (i + VEC <= n) {
+            v = *reinterpret_cast<const Vec*>(p + i);
+        } else {
+#pragma unroll
+            for (int q = 0; q < VEC; ++q) v.x[q] = i + q < n ? p[i + q] : T(0);
+        }
+        return v;
+    };
+    auto fetch = [&](int64_t i) {
+#pragma unroll
+        for (int j = 0; j < KJ; ++j)
+            if (j < KJ - 1 || w + 8 * j < K) nv[j] = load(V + (int64_t)(w + 8 * j) * ldv, i);
+        if (PASS == BASIS_DOTS) ny = load(y, i);
+        else if (threadIdx.x < ROWS) nf = i - lane * VEC + threadIdx.x < n ? y[i - lane * VEC + threadIdx.x] : T(0);
+    };
+    nv[KJ - 1] = Vec{};
+    const int64_t stride = (int64_t)gridDim.x * ROWS;
+    int64_t base = (int64_t)blockIdx.x * ROWS;
+    if (base < n) fetch(base + lane * VEC);
+    for (; base < n; base += stride) {
+        Vec vr[KJ];
+        double a[VEC];
+#pragma unroll
+        for (int j = 0; j < KJ; ++j) vr[j] = nv[j];
+#pragma unroll
+        for (int q = 0; q < VEC; ++q) a[q] = (double)ny.x[q];
+        const T old = nf;
+        if (base + stride < n) fetch(base + stride + lane * VEC);
+        if (PASS != BASIS_DOTS) {
+#pragma unroll
+            for (int q = 0; q < VEC; q += 2) {
+                double2 t = make_double2(0.0, 0.0);
+#pragma unroll
+                for (int j = 0; j < KJ; ++j) {
+                    t.x = fma(hw[j], (double)vr[j].x[q], t.x);
+                    t.y = fma(hw[j], (double)vr[j].x[q + 1], t.y);
+                }
+                *reinterpret_cast<double2*>(&part[w][lane * VEC + q]) = t;
+            }
+            __syncthreads();
+            if (threadIdx.x < ROWS) {   // one thread per row
+                double t = 0.0;
+#pragma unroll
+                for (int g = 0; g < BASIS_WARPS; ++g) t += part[g][threadIdx.x];
+                const T r = (T)((double)old - t);
+                if (base + threadIdx.x < n) y[base + threadIdx.x] = r;
+                fresh[threadIdx.x] = (double)r;
+                if (PASS == BASIS_AXPY_NORM) yy = fma((double)r, (double)r, yy);
+            }
+            __syncthreads();
+            if (PASS == BASIS_AXPY_DOTS) {
+#pragma unroll
+                for (int q = 0; q < VEC; q += 2) {
+                    const double2 f = *reinterpret_cast<const double2*>(&fresh[lane * VEC + q]);
+                    a[q] = f.x;
+                    a[q + 1] = f.y;
+                }
+            }
+        }
+        if (PASS != BASIS_AXPY_NORM) {
+#pragma unroll
+            for (int j = 0; j < KJ; ++j)
+#pragma unroll
+                for (int q = 0; q < VEC; ++q) acc[j] = fma((double)vr[j].x[q], a[q], acc[j]);
+        }
+        if (PASS == BASIS_DOTS && w == 0) {
+#pragma unroll
+            for (int q = 0; q < VEC; ++q) yy = fma(a[q], a[q], yy);
+        }
+    }
+    if (PASS != BASIS_AXPY_NORM) {
+#pragma unroll
+        for (int j = 0; j < KJ; ++j) {
+            const double v = warp_sum(acc[j]);
+            if (lane == 0) sums[w + 8 * j] = v;
+        }
+    }
+    if (PASS != BASIS_AXPY_DOTS) {
+        __shared__ double sh[BASIS_WARPS];
+        yy = block_sum(yy, sh);
+        if (threadIdx.x == 0) sums[8 * KJ] = yy;
+    }
     __syncthreads();
-    if (threadIdx.x == 0) last = atomicAdd(counter, 1u) == blocks - 1u;
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int k = w; k < K; k += nw) {
-        double acc = 0.0;
-        for (int b = lane; b < nb; b += 32) acc += __ldcg(partial + (int64_t)b * K + k);
-        acc = warp_sum(acc);
-        if (lane == 0) out[k] = acc;
+    const int P = PASS == BASIS_AXPY_NORM ? 1 : K + (PASS == BASIS_DOTS && self);
+    const int nb = (int)gridDim.x;
+    if ((int)threadIdx.x < P)
+        partial[(int64_t)threadIdx.x * nb + blockIdx.x] =
+            sums[PASS == BASIS_AXPY_NORM || (int)threadIdx.x == K ? 8 * KJ : threadIdx.x];
+    if (!last_block(counter)) return;
+    for (int k = w; k < P; k += BASIS_WARPS) {
+        double t = 0.0;
+        for (int b = lane; b < nb; b += 32) t += __ldcg(partial + (int64_t)k * nb + b);
+        t = warp_sum(t);
+        if (lane == 0) {
+            out[k] = t;
+            if (PASS == BASIS_AXPY_DOTS) h[k] += t;   // every block has read h
+        }
     }
     if (threadIdx.x == 0) *counter = 0u;
 }
-
-// partial[b*K + k] = sum over block column b's slice of x_k . y (K vectors
-// of V), MD_KT dot products per block: blockIdx.y picks the group of MD_KT
-// vectors, so the groups run side by side instead of one after another in
-// each block (y, read once per group, stays in L2).  Products and sums in
-// FP64 whatever the vector type.
-constexpr int MD_KT = 8;
-template <class T>
-__global__ void __launch_bounds__(RB)
-    k_multidot(const T* __restrict__ V, int64_t ldv, int Kv, int K, const T* __restrict__ y, int64_t n,
-               double* __restrict__ partial, double* __restrict__ out, unsigned int* __restrict__ counter) {
-    __shared__ double sh[MD_KT][RB / 32];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int k0 = blockIdx.y * MD_KT;
-    const int kt = min(MD_KT, K - k0);
-    double acc[MD_KT];
-#pragma unroll
-    for (int j = 0; j < MD_KT; ++j) acc[j] = 0.0;
-    GRID_STRIDE(i, n) {
-        const double yi = (double)y[i];
-#pragma unroll
-        for (int j = 0; j < MD_KT; ++j)
-            if (j < kt) {
-                const T* v = (k0 + j < Kv) ? V + (int64_t)(k0 + j) * ldv : y;
-                acc[j] += (double)v[i] * yi;
-            }
-    }
-#pragma unroll
-    for (int j = 0; j < MD_KT; ++j) {
-        const double v = warp_sum(acc[j]);
-        if (lane == 0) sh[j][w] = v;
-    }
-    __syncthreads();
-    if (threadIdx.x < kt) {
-        double t = 0.0;
-#pragma unroll
-        for (int q = 0; q < RB / 32; ++q) t += sh[threadIdx.x][q];
-        partial[(int64_t)blockIdx.x * K + k0 + threadIdx.x] = t;
-    }
-    last_block_finish(partial, (int)gridDim.x, K, out, counter);
-}
-
 
 // y -= sum_k h[k] V_k  (h on the device, staged in shared memory 64 at a
 // time; k ascending for every element)
@@ -116,76 +214,6 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-// The second and third passes of a CGS2 Arnoldi step, each one sweep over
-// the basis: y -= sum_k h[k] V_k (K <= 64 vectors) tile by tile (one row
-// per thread, 256-row tiles), then over the same tile, whose V values the
-// update has just brought into cache, the partial dots V_k . y (DOTS) or
-// y . y (NORM) of the new y: partial[b * P + k] with P = K (DOTS) or 1,
-// one block's tiles in ascending order (reproducible sums).
-constexpr int CG_TILE = 256;
-template <class T, bool DOTS>
-__global__ void __launch_bounds__(CG_TILE)
-    k_axpy_dots(const T* __restrict__ V, int64_t ldv, int K, const double* __restrict__ h, T* __restrict__ y,
-                int64_t n, double* __restrict__ partial, double* __restrict__ out, unsigned int* __restrict__ counter) {
-    __shared__ double hs[64];
-    __shared__ double ys[CG_TILE];
-    __shared__ double acc_blk[64];
-    __shared__ double wsum[CG_TILE / 32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (threadIdx.x < K) hs[threadIdx.x] = h[threadIdx.x];
-    if (threadIdx.x < 64) acc_blk[threadIdx.x] = 0.0;
-    __syncthreads();
-    for (int64_t tile = blockIdx.x; tile * CG_TILE < n; tile += gridDim.x) {
-        const int64_t i0 = tile * CG_TILE;
-        const int64_t i = i0 + threadIdx.x;
-        double yi = 0.0;
-        if (i < n) {
-            double a = (double)y[i];
-            const T* v = V + i;
-#pragma unroll 8
-            for (int k = 0; k < K; ++k) a -= hs[k] * (double)v[(int64_t)k * ldv];
-            const T r = (T)a;
-            y[i] = r;
-            yi = (double)r;
-        }
-        if (DOTS) {
-            ys[threadIdx.x] = yi;
-            __syncthreads();
-            const int rows = n - i0 < CG_TILE ? (int)(n - i0) : CG_TILE;
-            for (int k = warp; k < K; k += CG_TILE / 32) {
-                const T* v = V + (int64_t)k * ldv + i0;
-                double d = 0.0;
-#pragma unroll
-                for (int m = 0; m < CG_TILE / 32; ++m) {
-                    const int r = lane + 32 * m;
-                    if (r < rows) d += (double)v[r] * ys[r];
-                }
-                d = warp_sum(d);
-                if (lane == 0) acc_blk[k] += d;
-            }
-            __syncthreads();
-        } else {
-            const double d = warp_sum(yi * yi);
-            if (lane == 0) wsum[warp] = d;
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                double t = 0.0;
-#pragma unroll
-                for (int q = 0; q < CG_TILE / 32; ++q) t += wsum[q];
-                acc_blk[0] += t;
-            }
-            __syncthreads();
-        }
-    }
-    const int P = DOTS ? K : 1;
-    if (threadIdx.x < P) partial[(int64_t)blockIdx.x * P + threadIdx.x] = acc_blk[threadIdx.x];
-    last_block_finish(partial, (int)gridDim.x, P, out, counter);
-}
-
-__global__ void k_axpby(double a, const double* __restrict__ x, double b, double* __restrict__ y, int64_t n) {
-    GRID_STRIDE(i, n) y[i] = a * x[i] + b * y[i];
-}
-
 template <class T>
 __global__ void k_scale(T* __restrict__ x, double a, int64_t n) {
     GRID_STRIDE(i, n) x[i] = (T)((double)x[i] * a);
@@ -197,8 +225,7 @@ __global__ void k_sub(const T* __restrict__ b, const T* __restrict__ ax, T* __re
 }
 
 // a += b
-template <class T>
-__global__ void k_accumulate(T* __restrict__ a, const T* __restrict__ b, int64_t n) {
+__global__ void k_accumulate(double* __restrict__ a, const double* __restrict__ b, int n) {
     GRID_STRIDE(i, n) a[i] += b[i];
 }
 
@@ -211,20 +238,35 @@ __global__ void k_to_f32(const double* __restrict__ a, float* __restrict__ b, in
     GRID_STRIDE(i, n) b[i] = (float)a[i];
 }
 
-// CG updates: x += alpha p, r -= alpha q (alpha = num/den from the device)
-__global__ void k_cg_update(const double* __restrict__ sc, double* __restrict__ x, double* __restrict__ r,
-                            const double* __restrict__ p, const double* __restrict__ q, int64_t n) {
-    const double alpha = sc[0] / sc[1];
+// CG updates: x += alpha p, r -= alpha q (alpha = *rz / *pq), and out = r . r
+// of the new r in the order of k_dot.
+__global__ void __launch_bounds__(DOT_BLOCK)
+    k_cg_update(const double* __restrict__ rz, const double* __restrict__ pq, double* __restrict__ x,
+                double* __restrict__ r, const double* __restrict__ p, const double* __restrict__ q, int64_t n,
+                double* __restrict__ partial, double* __restrict__ out, unsigned int* __restrict__ counter) {
+    __shared__ double sh[DOT_BLOCK / 32];
+    const double alpha = *rz / *pq;
+    double acc = 0.0;
     GRID_STRIDE(i, n) {
         x[i] += alpha * p[i];
-        r[i] -= alpha * q[i];
+        const double v = r[i] - alpha * q[i];
+        r[i] = v;
+        acc += v * v;
+    }
+    acc = block_sum(acc, sh);
+    if (threadIdx.x == 0) partial[blockIdx.x] = acc;
+    if (!last_block(counter)) return;
+    acc = sum_partials(partial, (int)gridDim.x, sh);
+    if (threadIdx.x == 0) {
+        *out = acc;
+        *counter = 0u;
     }
 }
 
 // p = z + beta p (beta = rz_new / rz_old)
-__global__ void k_cg_dir(const double* __restrict__ sc, const double* __restrict__ z, double* __restrict__ p,
-                         int64_t n) {
-    const double beta = sc[2] / sc[0];
+__global__ void k_cg_dir(const double* __restrict__ rz_new, const double* __restrict__ rz_old,
+                         const double* __restrict__ z, double* __restrict__ p, int64_t n) {
+    const double beta = *rz_new / *rz_old;
     GRID_STRIDE(i, n) p[i] = z[i] + beta * p[i];
 }
 
@@ -250,14 +292,12 @@ __global__ void k_mask(T* __restrict__ x, const uint8_t* __restrict__ dir, int64
     GRID_STRIDE(i, n) if (dir[i]) x[i] = T(0);
 }
 
-__global__ void k_copy_scalar(const double* __restrict__ src, double* __restrict__ dst) { *dst = *src; }
-
 }  // namespace
 
 // ------------------------------------------------------------ Vec helper
 
 Blas::Blas(cudaStream_t s) : s(s) {
-    partial.alloc((size_t)std::max(RGRID, 148 * 8) * 64);
+    partial.alloc((size_t)BASIS_MAX_BLOCKS * (BASIS_MAX + 1));
     scal.alloc(128);
     counter.alloc(1);
     UP3D_CUDA(cudaMemsetAsync(counter.get(), 0, sizeof(unsigned int), s));
@@ -267,22 +307,56 @@ Blas::~Blas() {
     if (host) cudaFreeHost(host);
 }
 
-template <class T>
-void Blas::multidot(const T* V, int64_t ldv, int K, const T* y, int64_t n, double* out_dev, bool self_dot) {
-    const int Ktot = K + (self_dot ? 1 : 0);
-    for (int k0 = 0; k0 < Ktot; k0 += 64) {
-        int kk = std::min(64, Ktot - k0);
-        k_multidot<T><<<dim3(RGRID, (kk + MD_KT - 1) / MD_KT), RB, 0, s>>>(V + (int64_t)k0 * ldv, ldv, K - k0, kk, y,
-                                                                          n, partial.get(), out_dev + k0,
-                                                                          counter.get());
-        UP3D_CHECK_LAUNCH();
+template <class T, int KJ, int PASS>
+static void launch_basis_k(Blas& bl, const T* V, int64_t ldv, int K, double* h, T* y, int64_t n, bool self,
+                           double* out) {
+    static_assert(basis_blocks<KJ> <= BASIS_MAX_BLOCKS / 148, "partials hold BASIS_MAX_BLOCKS blocks");
+    const unsigned grid = grid_for(n, 32 * 16 / sizeof(T), (int64_t)148 * basis_blocks<KJ>);
+    k_basis<T, KJ, PASS><<<grid, DOT_BLOCK, 0, bl.s>>>(V, ldv, K, h, y, n, self, bl.partial.get(), out,
+                                                       bl.counter.get());
+    UP3D_CHECK_LAUNCH();
+}
+template <class T, int PASS>
+static void launch_basis(Blas& bl, const T* V, int64_t ldv, int K, double* h, T* y, int64_t n, bool self,
+                         double* out) {
+    switch ((K + 7) / 8) {
+        case 0:
+        case 1: return launch_basis_k<T, 1, PASS>(bl, V, ldv, K, h, y, n, self, out);
+        case 2: return launch_basis_k<T, 2, PASS>(bl, V, ldv, K, h, y, n, self, out);
+        case 3: return launch_basis_k<T, 3, PASS>(bl, V, ldv, K, h, y, n, self, out);
+        case 4: return launch_basis_k<T, 4, PASS>(bl, V, ldv, K, h, y, n, self, out);
+        case 5: return launch_basis_k<T, 5, PASS>(bl, V, ldv, K, h, y, n, self, out);
+        case 6: return launch_basis_k<T, 6, PASS>(bl, V, ldv, K, h, y, n, self, out);
+        case 7: return launch_basis_k<T, 7, PASS>(bl, V, ldv, K, h, y, n, self, out);
+        default: return launch_basis_k<T, 8, PASS>(bl, V, ldv, K, h, y, n, self, out);
     }
 }
 
 template <class T>
+void Blas::multidot(const T* V, int64_t ldv, int K, const T* y, int64_t n, double* out_dev, bool self_dot) {
+    int k0 = 0;
+    do {   // the self dot goes with the last chunk
+        const int kk = std::min(BASIS_MAX, K - k0);
+        launch_basis<T, BASIS_DOTS>(*this, V + (int64_t)k0 * ldv, ldv, kk, nullptr, const_cast<T*>(y), n,
+                                    self_dot && k0 + kk == K, out_dev + k0);
+        k0 += kk;
+    } while (k0 < K);
+}
+
+template <class T>
+void Blas::dot_dev(const T* x, const T* y, int64_t n, double* out_dev) {
+    k_dot<T><<<dot_grid(n), DOT_BLOCK, 0, s>>>(x, y, n, partial.get(), out_dev, counter.get());
+    UP3D_CHECK_LAUNCH();
+}
+
+template <class T>
 double Blas::dot(const T* x, const T* y, int64_t n) {
-    multidot(x, 0, 1, y, n, scal.get());
-    UP3D_CUDA(cudaMemcpyAsync(host, scal.get(), sizeof(double), cudaMemcpyDeviceToHost, s));
+    dot_dev(x, y, n, scal.get());
+    return read(scal.get());
+}
+
+double Blas::read(const double* dev) {
+    UP3D_CUDA(cudaMemcpyAsync(host, dev, sizeof(double), cudaMemcpyDeviceToHost, s));
     UP3D_CUDA(cudaStreamSynchronize(s));
     return host[0];
 }
@@ -290,11 +364,6 @@ double Blas::dot(const T* x, const T* y, int64_t n) {
 template <class T>
 double Blas::nrm2(const T* x, int64_t n) {
     return std::sqrt(dot(x, x, n));
-}
-
-void Blas::axpby(double a, const double* x, double b, double* y, int64_t n) {
-    k_axpby<<<grid_for(n, 256), 256, 0, s>>>(a, x, b, y, n);
-    UP3D_CHECK_LAUNCH();
 }
 
 template <class T>
@@ -310,23 +379,24 @@ void Blas::multiaxpy(const T* V, int64_t ldv, int K, const double* h_dev, T* y, 
 }
 
 template <class T>
-void Blas::axpy_dots(const T* V, int64_t ldv, int K, const double* h_dev, T* y, int64_t n, bool dots,
-                     double* out_dev) {
-    const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>((n + CG_TILE - 1) / CG_TILE, 148 * 8));
-    if (dots)
-        k_axpy_dots<T, true><<<grid, CG_TILE, 0, s>>>(V, ldv, K, h_dev, y, n, partial.get(), out_dev, counter.get());
-    else
-        k_axpy_dots<T, false><<<grid, CG_TILE, 0, s>>>(V, ldv, K, h_dev, y, n, partial.get(), out_dev, counter.get());
-    UP3D_CHECK_LAUNCH();
+void Blas::axpy_dots(const T* V, int64_t ldv, int K, double* h_dev, T* y, int64_t n, double* out_dev) {
+    launch_basis<T, BASIS_AXPY_DOTS>(*this, V, ldv, K, h_dev, y, n, false, out_dev);
+}
+
+template <class T>
+void Blas::axpy_norm(const T* V, int64_t ldv, int K, const double* h_dev, T* y, int64_t n, double* out_dev) {
+    launch_basis<T, BASIS_AXPY_NORM>(*this, V, ldv, K, const_cast<double*>(h_dev), y, n, false, out_dev);
 }
 
 #define UP3D_BLAS_INST(T)                                                                 \
     template void Blas::multidot<T>(const T*, int64_t, int, const T*, int64_t, double*, bool); \
+    template void Blas::dot_dev<T>(const T*, const T*, int64_t, double*);                \
     template double Blas::dot<T>(const T*, const T*, int64_t);                           \
     template double Blas::nrm2<T>(const T*, int64_t);                                    \
     template void Blas::scale<T>(T*, double, int64_t);                                   \
     template void Blas::multiaxpy<T>(const T*, int64_t, int, const double*, T*, int64_t); \
-    template void Blas::axpy_dots<T>(const T*, int64_t, int, const double*, T*, int64_t, bool, double*);
+    template void Blas::axpy_dots<T>(const T*, int64_t, int, double*, T*, int64_t, double*); \
+    template void Blas::axpy_norm<T>(const T*, int64_t, int, const double*, T*, int64_t, double*);
 UP3D_BLAS_INST(double)
 UP3D_BLAS_INST(float)
 #undef UP3D_BLAS_INST
@@ -498,20 +568,25 @@ int cg_solve(const Operator& op, const double* b, double* x, double rtol, double
     if (rn > tol) {
         precond_apply(M, r.get(), z.get(), n, s);
         UP3D_CUDA(cudaMemcpyAsync(p.get(), z.get(), sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
-        bl.multidot(r.get(), 0, 1, z.get(), n, sc.get() + 0);  // rz
+        // r.z of this and the last iteration take turns in sc[0], sc[1]
+        double* rz = sc.get();
+        double* rz_next = sc.get() + 1;
+        double* pq = sc.get() + 2;
+        double* rr = sc.get() + 3;
+        bl.dot_dev(r.get(), z.get(), n, rz);
         for (it = 1; it <= maxiter; ++it) {
             op.apply(p.get(), q.get(), s);
-            bl.multidot(p.get(), 0, 1, q.get(), n, sc.get() + 1);  // pq
-            k_cg_update<<<grid_for(n, 256), 256, 0, s>>>(sc.get(), x, r.get(), p.get(), q.get(), n);
+            bl.dot_dev(p.get(), q.get(), n, pq);
+            k_cg_update<<<dot_grid(n), DOT_BLOCK, 0, s>>>(rz, pq, x, r.get(), p.get(), q.get(), n, bl.partial.get(), rr,
+                                                          bl.counter.get());
             UP3D_CHECK_LAUNCH();
-            rn = bl.nrm2(r.get(), n);
+            rn = std::sqrt(bl.read(rr));
             if (rn <= tol || !std::isfinite(rn)) break;
             precond_apply(M, r.get(), z.get(), n, s);
-            bl.multidot(r.get(), 0, 1, z.get(), n, sc.get() + 2);  // rz_new
-            k_cg_dir<<<grid_for(n, 256), 256, 0, s>>>(sc.get(), z.get(), p.get(), n);
+            bl.dot_dev(r.get(), z.get(), n, rz_next);
+            k_cg_dir<<<grid_for(n, 256), 256, 0, s>>>(rz_next, rz, z.get(), p.get(), n);
             UP3D_CHECK_LAUNCH();
-            k_copy_scalar<<<1, 1, 0, s>>>(sc.get() + 2, sc.get() + 0);
-            UP3D_CHECK_LAUNCH();
+            std::swap(rz, rz_next);
         }
         if (it > maxiter) it = maxiter;
     }
@@ -571,7 +646,8 @@ int gmres_solve(const Operator& op, const T* b, T* x, double rtol, double atol, 
     DBuf<T>& r = B[2];
     DBuf<T>& tmp = B[3];
     DBuf<double>& hdev = W.d[5];
-    V.alloc((size_t)(restart + 1) * n);
+    const int64_t ld = (n + 31) & ~int64_t(31);   // basis vectors start on 128-byte lines
+    V.alloc((size_t)(restart + 1) * ld);
     w.alloc(n);
     r.alloc(n);
     tmp.alloc(n);
@@ -616,7 +692,7 @@ int gmres_solve(const Operator& op, const T* b, T* x, double rtol, double atol, 
             // [h_0 .. h_col] (CGS2: two projections onto V_0..V_col, summed),
             // |w| before and after the projections
             // pass 1 takes V_0..V_col and the new vector itself in one
-            // multidot (h and |w|^2), passes 2 and 3 are one sweep each
+            // sweep (h and |w|^2), passes 2 and 3 are one sweep each
             // (update + the next pass's dots, update + |w|^2), and the
             // normalisation writes the vector into V[col + 1].  The
             // preconditioner's output stays the one buffer w, so its
@@ -625,21 +701,22 @@ int gmres_solve(const Operator& op, const T* b, T* x, double rtol, double atol, 
             double* hpass = hdev.get() + (restart + 3);
             double* hn = hsum + col + 1;
             T* wv = w.get();
-            op.apply(V.get() + (size_t)col * n, tmp.get(), s);
+            op.apply(V.get() + (size_t)col * ld, tmp.get(), s);
             precond_apply(M, tmp.get(), wv, n, s);
-            bl.multidot(V.get(), n, col + 1, wv, n, hsum, true);
-            if (col + 1 <= 64) {
-                bl.axpy_dots(V.get(), n, col + 1, hsum, wv, n, true, hpass);
-                bl.axpy_dots(V.get(), n, col + 1, hpass, wv, n, false, hn + 1);
+            bl.multidot(V.get(), ld, col + 1, wv, n, hsum, true);
+            if (col + 1 <= BASIS_MAX) {
+                // pass 2 leaves its coefficients in hpass and adds them to hsum
+                bl.axpy_dots(V.get(), ld, col + 1, hsum, wv, n, hpass);
+                bl.axpy_norm(V.get(), ld, col + 1, hpass, wv, n, hn + 1);
             } else {
-                bl.multiaxpy(V.get(), n, col + 1, hsum, wv, n);
-                bl.multidot(V.get(), n, col + 1, wv, n, hpass);
-                bl.multiaxpy(V.get(), n, col + 1, hpass, wv, n);
-                bl.multidot(wv, 0, 0, wv, n, hn + 1, true);
+                bl.multiaxpy(V.get(), ld, col + 1, hsum, wv, n);
+                bl.multidot(V.get(), ld, col + 1, wv, n, hpass);
+                bl.multiaxpy(V.get(), ld, col + 1, hpass, wv, n);
+                bl.dot_dev(wv, wv, n, hn + 1);
+                k_accumulate<<<1, 256, 0, s>>>(hsum, hpass, col + 1);
+                UP3D_CHECK_LAUNCH();
             }
-            k_accumulate<double><<<1, 64, 0, s>>>(hsum, hpass, col + 1);
-            UP3D_CHECK_LAUNCH();
-            k_scale_unless_breakdown<T><<<grid_for(n, 256), 256, 0, s>>>(wv, V.get() + (size_t)(col + 1) * n, hn, eps, n);
+            k_scale_unless_breakdown<T><<<grid_for(n, 256), 256, 0, s>>>(wv, V.get() + (size_t)(col + 1) * ld, hn, eps, n);
             UP3D_CHECK_LAUNCH();
             UP3D_CUDA(cudaMemcpyAsync(hbuf, hsum, sizeof(double) * (col + 3), cudaMemcpyDeviceToHost, s));
             UP3D_CUDA(cudaStreamSynchronize(s));
@@ -684,7 +761,7 @@ int gmres_solve(const Operator& op, const T* b, T* x, double rtol, double atol, 
         // x += V^T y  (as x -= V (-y))
         for (auto& v : y) v = -v;
         UP3D_CUDA(cudaMemcpyAsync(hdev.get(), y.data(), sizeof(double) * (col + 1), cudaMemcpyHostToDevice, s));
-        bl.multiaxpy(V.get(), n, col + 1, hdev.get(), x, n);
+        bl.multiaxpy(V.get(), ld, col + 1, hdev.get(), x, n);
         op.residual(b, x, r.get(), tmp.get(), s);
         rnorm = bl.nrm2(r.get(), n);
         if (rnorm <= atol_eff || breakdown || !std::isfinite(rnorm)) break;

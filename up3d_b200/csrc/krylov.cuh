@@ -39,19 +39,22 @@ struct Blas {
     template <class T>
     void multidot(const T* V, int64_t ldv, int K, const T* y, int64_t n, double* out_dev, bool self_dot = false);
     template <class T>
+    void dot_dev(const T* x, const T* y, int64_t n, double* out_dev);
+    double read(const double* dev);   // one scalar to the host (synchronises the stream)
+    template <class T>
     double dot(const T* x, const T* y, int64_t n);
     template <class T>
     double nrm2(const T* x, int64_t n);
-    void axpby(double a, const double* x, double b, double* y, int64_t n);
     template <class T>
     void scale(T* x, double a, int64_t n);
     template <class T>
     void multiaxpy(const T* V, int64_t ldv, int K, const double* h_dev, T* y, int64_t n);
-    // y -= V h (K <= 64) in one sweep that also forms V^T y (dots) or y.y
-    // (!dots) of the new y into out_dev
+    // y -= V h (K <= 64) in one sweep that also forms out = V^T y of the new
+    // y and adds it to h, or out = y . y
     template <class T>
-    void axpy_dots(const T* V, int64_t ldv, int K, const double* h_dev, T* y, int64_t n, bool dots,
-                   double* out_dev);
+    void axpy_dots(const T* V, int64_t ldv, int K, double* h_dev, T* y, int64_t n, double* out_dev);
+    template <class T>
+    void axpy_norm(const T* V, int64_t ldv, int K, const double* h_dev, T* y, int64_t n, double* out_dev);
 };
 
 // y = A x (+ extra x): the P1-pattern matrix plus, for the Newton Jacobian,

@@ -25,6 +25,7 @@
 #include <cmath>
 
 #include "internal.cuh"
+#include "reduce.cuh"
 
 namespace up3d {
 
@@ -34,11 +35,9 @@ void launch_spmv(int64_t n, const int32_t* indptr, const int32_t* indices, const
 
 namespace {
 
-constexpr int NA_RB = 256;     // reduction block (as in krylov.cu)
-constexpr int NA_RGRID = 592;  // fixed partial count (as in krylov.cu)
 constexpr int64_t NA_ROWS = UP3D_NOALLOC_MAX_ROWS;
 // r, z, p, q, D^-1, then the reduction partials and the scalars
-constexpr int64_t NA_DOUBLES = 5 * NA_ROWS + NA_RGRID + 8;
+constexpr int64_t NA_DOUBLES = 5 * NA_ROWS + DOT_MAX_BLOCKS + 8;
 
 static __device__ __align__(256) double g_scratch[NA_DOUBLES];
 
@@ -46,30 +45,21 @@ static __device__ __align__(256) double g_scratch[NA_DOUBLES];
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < (n); i += (int64_t)gridDim.x * blockDim.x)
 
 // The two reduction passes of the allocating CG's dot products (krylov.cu
-// k_multidot with one vector, k_finish): per block, warp butterflies then
-// the block's warp sums in order; then one warp over the block partials.
-__global__ void __launch_bounds__(NA_RB) k_na_dot(const double* __restrict__ x, const double* __restrict__ y,
-                                                  int64_t n, double* __restrict__ partial) {
-    __shared__ double sh[NA_RB / 32];
+// k_dot), the second as its own launch.
+__global__ void __launch_bounds__(DOT_BLOCK) k_na_dot(const double* __restrict__ x, const double* __restrict__ y,
+                                                      int64_t n, double* __restrict__ partial) {
+    __shared__ double sh[DOT_BLOCK / 32];
     double acc = 0.0;
     GRID_STRIDE(i, n) acc += x[i] * y[i];
-    const double v = warp_sum(acc);
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double t = 0.0;
-#pragma unroll
-        for (int q = 0; q < NA_RB / 32; ++q) t += sh[q];
-        partial[blockIdx.x] = t;
-    }
+    acc = block_sum(acc, sh);
+    if (threadIdx.x == 0) partial[blockIdx.x] = acc;
 }
 
-__global__ void k_na_finish(const double* __restrict__ partial, int nb, double* __restrict__ out) {
-    if (threadIdx.x >= 32) return;
-    double acc = 0.0;
-    for (int b = threadIdx.x; b < nb; b += 32) acc += partial[b];
-    acc = warp_sum(acc);
-    if (threadIdx.x == 0) *out = acc;
+__global__ void __launch_bounds__(DOT_BLOCK) k_na_finish(const double* __restrict__ partial, int nb,
+                                                         double* __restrict__ out) {
+    __shared__ double sh[DOT_BLOCK / 32];
+    const double v = sum_partials(partial, nb, sh);
+    if (threadIdx.x == 0) *out = v;
 }
 
 __global__ void k_na_diag(int64_t n, const int32_t* __restrict__ indptr, const int32_t* __restrict__ indices,
@@ -144,13 +134,13 @@ extern "C" int up3d_cg_jacobi_noalloc(const up3d_csr* A, const double* b, double
         double* q = base + 3 * NA_ROWS;
         double* dinv = base + 4 * NA_ROWS;
         double* partial = base + 5 * NA_ROWS;
-        double* sc = partial + NA_RGRID;  // rz, pq, rz_new, norm
+        double* sc = partial + DOT_MAX_BLOCKS;  // rz, pq, rz_new, norm
         // previous calls leave their values behind: start the scalars at 0
         UP3D_CUDA(cudaMemsetAsync(sc, 0, 8 * sizeof(double), s));
         auto dot = [&](const double* u, const double* v, double* out) {
-            k_na_dot<<<NA_RGRID, NA_RB, 0, s>>>(u, v, n, partial);
+            k_na_dot<<<dot_grid(n), DOT_BLOCK, 0, s>>>(u, v, n, partial);
             UP3D_CHECK_LAUNCH();
-            k_na_finish<<<1, 1024, 0, s>>>(partial, NA_RGRID, out);
+            k_na_finish<<<1, DOT_BLOCK, 0, s>>>(partial, (int)dot_grid(n), out);
             UP3D_CHECK_LAUNCH();
         };
         auto nrm = [&](const double* u) {
