@@ -721,10 +721,25 @@ __global__ void k_gj_elim(double* __restrict__ a, double* __restrict__ inv, int6
 
 // ------------------------------------------------------------ device kernels
 
-template <class T>
-__global__ void k_jacobi_first(const T* __restrict__ dinv, const T* __restrict__ b, T* __restrict__ x, T w,
-                               int64_t n) {
-    GRID_STRIDE(i, n) x[i] = w * dinv[i] * b[i];
+// The kernels of the cycle take part in overlapped launches (pdl_wait) and
+// read the smoothing weight from the device, so that a captured cycle stays
+// valid when the values are refreshed.  Vectors are plain pointers, not
+// __restrict__ (read-only loads): the kernel before may still be writing them
+// when a kernel starts.
+
+// x = w D^-1 b from b = b_in (kept in b_out unless null)
+template <class T, class TI>
+__global__ void __launch_bounds__(256)
+    k_jacobi_first(const T* __restrict__ dinv, const TI* b_in, T* b_out, T* x, const double* __restrict__ omega,
+                   int64_t n) {
+    pdl_trigger();
+    pdl_wait();
+    const T w = (T)*omega;
+    GRID_STRIDE(i, n) {
+        const T b = (T)b_in[i];
+        if (b_out) b_out[i] = b;
+        x[i] = w * dinv[i] * b;
+    }
 }
 
 // Row loop shared by the CSR kernels below: TPR = 0 is one warp per 32
@@ -736,7 +751,7 @@ constexpr int rows_block = TPR == 0 ? CSR_WARP_BLOCK : CSR_ROWS_BLOCK;
 template <class T, int TPR, int BLOCK, class Epi>
 __device__ __forceinline__ void csr_rows_loop(int64_t n, const int32_t* __restrict__ Ap,
                                               const int32_t* __restrict__ Ai, const T* __restrict__ Ax,
-                                              const T* __restrict__ x, Epi epi) {
+                                              const T* x, Epi epi) {
     const int64_t warp = (blockIdx.x * (int64_t)BLOCK + threadIdx.x) >> 5;
     const int64_t n_warps = ((int64_t)gridDim.x * BLOCK) >> 5;
     auto term = [&](int32_t c, T v) { return v * x[c]; };
@@ -836,27 +851,32 @@ __global__ void __launch_bounds__(256)
 template <class T, bool RESID, int TPR>
 __global__ void __launch_bounds__(rows_block<TPR>)
     k_jacobi_sweep(int64_t n, const int32_t* __restrict__ Ap, const int32_t* __restrict__ Ai,
-                   const T* __restrict__ Ax, const T* __restrict__ dinv, const T* __restrict__ b,
-                   const T* __restrict__ x, T* __restrict__ out, T w) {
+                   const T* __restrict__ Ax, const T* __restrict__ dinv, const T* b, const T* x, T* out,
+                   const double* __restrict__ omega) {
+    pdl_trigger();
+    pdl_wait();
+    const T w = (T)*omega;
     csr_rows_loop<T, TPR, rows_block<TPR>>(n, Ap, Ai, Ax, x, [&](int64_t r, T acc) {
         const T res = b[r] - acc;
         out[r] = RESID ? res : x[r] + w * dinv[r] * res;
     });
 }
 
-// The same sweep on the sliced rows, one row per lane.
+// The same sweep on the sliced rows, one row per lane; the first entries are
+// on their way while the kernel before drains.
 template <class T, bool RESID>
 __global__ void __launch_bounds__(SELL_BLOCK)
     k_jacobi_sell(int64_t n, const int32_t* __restrict__ Sp, const int32_t* __restrict__ Si,
-                  const T* __restrict__ Sx, const T* __restrict__ dinv, const T* __restrict__ b,
-                  const T* __restrict__ x, T* __restrict__ out, T w) {
+                  const T* __restrict__ Sx, const T* __restrict__ dinv, const T* b, const T* x, T* out,
+                  const double* __restrict__ omega) {
+    pdl_trigger();
     const int64_t r = blockIdx.x * (int64_t)SELL_BLOCK + threadIdx.x;
     const int lane = threadIdx.x & 31;
     if (r - lane >= n) return;   // warp-uniform
-    const T acc = sell_row_sum<T>(Sp, Si, Sx, x, r >> 5, lane);
+    const T acc = sell_row_sum<T>(Sp, Si, Sx, x, r >> 5, lane, pdl_wait);
     if (r >= n) return;
     const T res = b[r] - acc;
-    out[r] = RESID ? res : x[r] + w * dinv[r] * res;
+    out[r] = RESID ? res : x[r] + (T)*omega * dinv[r] * res;
 }
 
 // Column indices of the sliced rows from the CSR ones (-1 on the padding),
@@ -885,28 +905,22 @@ __global__ void k_sell_values(int64_t n, const int32_t* __restrict__ Ap, const d
 template <class T, bool ADD, int TPR>
 __global__ void __launch_bounds__(rows_block<TPR>)
     k_spmv_rect(int64_t n, const int32_t* __restrict__ Ap, const int32_t* __restrict__ Ai, const T* __restrict__ Ax,
-                const T* __restrict__ x, T* __restrict__ y) {
+                const T* x, T* y) {
+    pdl_trigger();
+    pdl_wait();
     csr_rows_loop<T, TPR, rows_block<TPR>>(n, Ap, Ai, Ax, x,
                                            [&](int64_t r, T acc) { y[r] = ADD ? y[r] + acc : acc; });
 }
 
 template <class T, bool RESID>
-void launch_sweep(int64_t n, int64_t nnz, const int32_t* Ap, const int32_t* Ai, const T* Ax, const T* dinv,
-                  const T* b, const T* x, T* out, T w, cudaStream_t s) {
-    if (use_warp_rows(n, nnz)) {
-        k_jacobi_sweep<T, RESID, 0><<<csr_rows_grid(n, CSR_WARP_BLOCK), CSR_WARP_BLOCK, 0, s>>>(n, Ap, Ai, Ax, dinv, b, x, out, w);
-    } else {
-        switch (lanes_per_row(nnz, n)) {
-            case 4: k_jacobi_sweep<T, RESID, 4><<<lanes_grid(n, 4), 256, 0, s>>>(n, Ap, Ai, Ax, dinv, b, x, out, w); break;
-            case 8: k_jacobi_sweep<T, RESID, 8><<<lanes_grid(n, 8), 256, 0, s>>>(n, Ap, Ai, Ax, dinv, b, x, out, w); break;
-            case 16:
-                k_jacobi_sweep<T, RESID, 16><<<lanes_grid(n, 16), 256, 0, s>>>(n, Ap, Ai, Ax, dinv, b, x, out, w);
-                break;
-            default:
-                k_jacobi_sweep<T, RESID, 32><<<lanes_grid(n, 32), 256, 0, s>>>(n, Ap, Ai, Ax, dinv, b, x, out, w);
-        }
-    }
-    UP3D_CHECK_LAUNCH();
+void launch_sweep(bool overlap, int64_t n, int64_t nnz, const int32_t* Ap, const int32_t* Ai, const T* Ax,
+                  const T* dinv, const T* b, const T* x, T* out, const double* omega, cudaStream_t s) {
+    const int tpr = use_warp_rows(n, nnz) ? 0 : lanes_per_row(nnz, n);
+    auto kern = tpr == 0 ? k_jacobi_sweep<T, RESID, 0> : tpr == 4 ? k_jacobi_sweep<T, RESID, 4>
+                : tpr == 8 ? k_jacobi_sweep<T, RESID, 8> : tpr == 16 ? k_jacobi_sweep<T, RESID, 16>
+                : k_jacobi_sweep<T, RESID, 32>;
+    launch_kernel(overlap, kern, tpr == 0 ? csr_rows_grid(n, CSR_WARP_BLOCK) : lanes_grid(n, tpr),
+                  tpr == 0 ? CSR_WARP_BLOCK : CSR_ROWS_BLOCK, s, n, Ap, Ai, Ax, dinv, b, x, out, omega);
 }
 
 void launch_pw_step(int64_t n, int64_t nnz, const int32_t* Ap, const int32_t* Ai, const double* Ax, const double* sq,
@@ -921,25 +935,21 @@ void launch_pw_step(int64_t n, int64_t nnz, const int32_t* Ap, const int32_t* Ai
 }
 
 template <class T, bool ADD>
-void launch_rect(int64_t n, int64_t nnz, const int32_t* Ap, const int32_t* Ai, const T* Ax, const T* x, T* y,
-                 cudaStream_t s) {
-    if (use_warp_rows(n, nnz)) {
-        k_spmv_rect<T, ADD, 0><<<csr_rows_grid(n, CSR_WARP_BLOCK), CSR_WARP_BLOCK, 0, s>>>(n, Ap, Ai, Ax, x, y);
-    } else {
-        switch (lanes_per_row(nnz, n)) {
-            case 4: k_spmv_rect<T, ADD, 4><<<lanes_grid(n, 4), 256, 0, s>>>(n, Ap, Ai, Ax, x, y); break;
-            case 8: k_spmv_rect<T, ADD, 8><<<lanes_grid(n, 8), 256, 0, s>>>(n, Ap, Ai, Ax, x, y); break;
-            case 16: k_spmv_rect<T, ADD, 16><<<lanes_grid(n, 16), 256, 0, s>>>(n, Ap, Ai, Ax, x, y); break;
-            default: k_spmv_rect<T, ADD, 32><<<lanes_grid(n, 32), 256, 0, s>>>(n, Ap, Ai, Ax, x, y);
-        }
-    }
-    UP3D_CHECK_LAUNCH();
+void launch_rect(bool overlap, int64_t n, int64_t nnz, const int32_t* Ap, const int32_t* Ai, const T* Ax, const T* x,
+                 T* y, cudaStream_t s) {
+    const int tpr = use_warp_rows(n, nnz) ? 0 : lanes_per_row(nnz, n);
+    auto kern = tpr == 0 ? k_spmv_rect<T, ADD, 0> : tpr == 4 ? k_spmv_rect<T, ADD, 4>
+                : tpr == 8 ? k_spmv_rect<T, ADD, 8> : tpr == 16 ? k_spmv_rect<T, ADD, 16> : k_spmv_rect<T, ADD, 32>;
+    launch_kernel(overlap, kern, tpr == 0 ? csr_rows_grid(n, CSR_WARP_BLOCK) : lanes_grid(n, tpr),
+                  tpr == 0 ? CSR_WARP_BLOCK : CSR_ROWS_BLOCK, s, n, Ap, Ai, Ax, x, y);
 }
 
 // x = Cinv b (dense, one warp per row), FP64, inputs/outputs of type T
 template <class T>
-__global__ void k_dense_solve(const double* __restrict__ Cinv, int64_t n, const T* __restrict__ b,
-                              T* __restrict__ x) {
+__global__ void __launch_bounds__(256)
+    k_dense_solve(const double* __restrict__ Cinv, int64_t n, const T* b, T* x) {
+    pdl_trigger();
+    pdl_wait();
     const int lane = threadIdx.x & 31;
     const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t n_warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -1046,7 +1056,7 @@ struct Level {
     DBuf<T> sell_x;
     DBuf<T> own_A, own_P, own_R, own_dinv;  // FP32 values (unused for FP64)
     DBuf<T> x, b, r;
-    T w_smooth = T(0);
+    const double* omega = nullptr;          // smoothing weight (device)
 };
 
 // Symbolic structure and FP64 values of one level.
@@ -1082,30 +1092,26 @@ struct Amg {
     // numeric scratch
     DBuf<double> pw_yz, pw_scal, omega_dev, gj_fac, dense_a, fcol;
     DBuf<int> flags;
-    std::vector<double> omega;
     DBuf<double> cinv;
     std::vector<Level<double>*> Ld;
     std::vector<Level<float>*> Lf;
     up3d_amg_info info{};
-    // one V-cycle as a CUDA graph per (input, output) pair: captured on a
-    // private stream at first use, replayed on the caller's stream
-    struct Graph {
-        const void* r;
-        void* z;
-        bool f32;  // FP32 input and output
-        cudaGraphExec_t exec;
-        long long launches;
+    // the V-cycle of each precision between its first smoothing (which reads
+    // the caller's vector) and its last (which writes the caller's) as a
+    // CUDA graph on the levels' own buffers: captured once on a private
+    // stream, replayed for every vector and every refresh of the values
+    struct Body {
+        cudaGraphExec_t exec = nullptr;
+        long long launches = 0;
+        void* x = nullptr;   // the level-0 iterate after the body, and the other buffer
+        void* other = nullptr;
     };
-    DBuf<double> io64_in, io64_out;  // FP32 input/output through an FP64 hierarchy
-    std::vector<Graph> graphs;
+    Body body64, body32;
     cudaStream_t capture_stream = nullptr;
     int device = 0;
-    void drop_graphs() {
-        for (auto& g : graphs) cudaGraphExecDestroy(g.exec);
-        graphs.clear();
-    }
     ~Amg() {
-        drop_graphs();
+        for (Body* b : {&body64, &body32})
+            if (b->exec) cudaGraphExecDestroy(b->exec);
         if (capture_stream) cudaStreamDestroy(capture_stream);
         for (auto* l : Ld) delete l;
         for (auto* l : Lf) delete l;
@@ -1118,49 +1124,45 @@ namespace {
 // One sweep (or residual) of a level's operator: the sliced rows where the
 // level has them, else the CSR rows.
 template <class T, bool RESID>
-void smooth(const Level<T>& lv, const T* x, T* out, cudaStream_t s) {
+void smooth(bool overlap, const Level<T>& lv, const T* x, T* out, cudaStream_t s) {
     const int64_t n = lv.A.n;
-    if (!lv.sell_p) {
-        launch_sweep<T, RESID>(n, lv.A.nnz, lv.A.p.get(), lv.A.i.get(), lv.A.x.get(), lv.dinv.get(), lv.b.get(), x, out,
-                               lv.w_smooth, s);
-        return;
-    }
-    k_jacobi_sell<T, RESID><<<sell_grid(n), SELL_BLOCK, 0, s>>>(n, lv.sell_p, lv.sell_i, lv.sell_x.get(),
-                                                               lv.dinv.get(), lv.b.get(), x, out, lv.w_smooth);
-    UP3D_CHECK_LAUNCH();
+    if (lv.sell_p)
+        launch_kernel(overlap, k_jacobi_sell<T, RESID>, sell_grid(n), SELL_BLOCK, s, n, lv.sell_p, lv.sell_i,
+                      lv.sell_x.get(), lv.dinv.get(), lv.b.get(), x, out, lv.omega);
+    else
+        launch_sweep<T, RESID>(overlap, n, lv.A.nnz, lv.A.p.get(), lv.A.i.get(), lv.A.x.get(), lv.dinv.get(),
+                               lv.b.get(), x, out, lv.omega, s);
 }
 
+// The V-cycle on level l from its b to its x; on the finest level (top)
+// without the first and the last smoothing.  Its kernels overlap: the first
+// that a caller launches must be ordered behind everything before it.
 template <class T>
-void vcycle(Amg& a, std::vector<Level<T>*>& L, size_t l, cudaStream_t s) {
+void vcycle(Amg& a, std::vector<Level<T>*>& L, size_t l, bool top, cudaStream_t s) {
     Level<T>& lv = *L[l];
     const int64_t n = lv.A.n;
     if (l + 1 == L.size()) {
         // coarsest: dense FP64 solve
-        if (std::is_same<T, double>::value) {
-            k_dense_solve<T><<<grid_for(32 * n, 256), 256, 0, s>>>(a.cinv.get(), n, lv.b.get(), lv.x.get());
-        } else {
-            k_dense_solve<T><<<grid_for(32 * n, 256), 256, 0, s>>>(a.cinv.get(), n, lv.b.get(), lv.x.get());
-        }
-        UP3D_CHECK_LAUNCH();
+        launch_kernel(true, k_dense_solve<T>, grid_for(32 * n, 256), 256, s, a.cinv.get(), n, lv.b.get(), lv.x.get());
         return;
     }
-    const unsigned g1 = grid_for(n, 256);
     // pre-smoothing from x = 0
-    k_jacobi_first<T><<<g1, 256, 0, s>>>(lv.dinv.get(), lv.b.get(), lv.x.get(), lv.w_smooth, n);
-    UP3D_CHECK_LAUNCH();
+    if (!top)
+        launch_kernel(true, k_jacobi_first<T, T>, grid_for(n, 256), 256, s, lv.dinv.get(), lv.b.get(), nullptr,
+                      lv.x.get(), lv.omega, n);
     for (int k = 1; k < a.pre; ++k) {
-        smooth<T, false>(lv, lv.x.get(), lv.r.get(), s);
+        smooth<T, false>(true, lv, lv.x.get(), lv.r.get(), s);
         std::swap(lv.x.p, lv.r.p);
     }
     // residual, restriction
-    smooth<T, true>(lv, lv.x.get(), lv.r.get(), s);
+    smooth<T, true>(true, lv, lv.x.get(), lv.r.get(), s);
     Level<T>& cv = *L[l + 1];
-    launch_rect<T, false>(lv.R.n, lv.R.nnz, lv.R.p.get(), lv.R.i.get(), lv.R.x.get(), lv.r.get(), cv.b.get(), s);
-    vcycle<T>(a, L, l + 1, s);
+    launch_rect<T, false>(true, lv.R.n, lv.R.nnz, lv.R.p.get(), lv.R.i.get(), lv.R.x.get(), lv.r.get(), cv.b.get(), s);
+    vcycle<T>(a, L, l + 1, false, s);
     // prolongation
-    launch_rect<T, true>(lv.P.n, lv.P.nnz, lv.P.p.get(), lv.P.i.get(), lv.P.x.get(), cv.x.get(), lv.x.get(), s);
-    for (int k = 0; k < a.post; ++k) {
-        smooth<T, false>(lv, lv.x.get(), lv.r.get(), s);
+    launch_rect<T, true>(true, lv.P.n, lv.P.nnz, lv.P.p.get(), lv.P.i.get(), lv.P.x.get(), cv.x.get(), lv.x.get(), s);
+    for (int k = top ? 1 : 0; k < a.post; ++k) {
+        smooth<T, false>(true, lv, lv.x.get(), lv.r.get(), s);
         std::swap(lv.x.p, lv.r.p);
     }
 }
@@ -1263,10 +1265,6 @@ void numeric(Amg& a, cudaStream_t s) {
         }
     }
     int sing = 0;
-    a.omega.assign(L > 1 ? L - 1 : 0, 0.0);
-    if (L > 1)
-        UP3D_CUDA(cudaMemcpyAsync(a.omega.data(), a.omega_dev.get(), sizeof(double) * (L - 1),
-                                  cudaMemcpyDeviceToHost, s));
     UP3D_CUDA(cudaMemcpyAsync(&sing, singular, sizeof(int), cudaMemcpyDeviceToHost, s));
     UP3D_CUDA(cudaStreamSynchronize(s));
     if (sing) {
@@ -1296,7 +1294,7 @@ void numeric(Amg& a, cudaStream_t s) {
 }
 
 // Narrows the FP64 level values into the FP32 cycle (the FP64 cycle views
-// them in place) and sets the smoothing weights.
+// them in place) and fills the slices.
 template <class T>
 void fill_levels(Amg& a, std::vector<Level<T>*>& Lv, cudaStream_t s) {
     for (size_t l = 0; l < a.sym.size(); ++l) {
@@ -1315,7 +1313,6 @@ void fill_levels(Amg& a, std::vector<Level<T>*>& Lv, cudaStream_t s) {
                 convert<T>(F.R.x.get(), lv.R.x.get(), F.R.nnz, s);
                 convert<T>(F.dinv.get(), lv.dinv.get(), F.A.n, s);
             }
-            lv.w_smooth = (T)a.omega[l];
         }
     }
 }
@@ -1355,6 +1352,7 @@ void make_levels(Amg& a, std::vector<Level<T>*>& Lv, cudaStream_t s) {
         lv->b.alloc(n);
         lv->r.alloc(n);
         if (l + 1 < a.sym.size()) {
+            lv->omega = a.omega_dev.get() + l;
             view(lv->P, F.P, lv->own_P);
             view(lv->R, F.R, lv->own_R);
             if constexpr (std::is_same<T, double>::value) {
@@ -1378,112 +1376,91 @@ __global__ void k_diff_u8(int64_t n, const uint8_t* __restrict__ a, const uint8_
 
 }  // namespace
 
-// One V-cycle z = M r as a sequence of launches on stream s.
-void amg_cycle(Amg& a, const double* r, double* z, cudaStream_t s) {
-    if (a.fp64) {
-        Level<double>& f = *a.Ld[0];
-        const int64_t n = f.A.n;
-        UP3D_CUDA(cudaMemcpyAsync(f.b.get(), r, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
-        vcycle<double>(a, a.Ld, 0, s);
-        UP3D_CUDA(cudaMemcpyAsync(z, f.x.get(), sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
+template <class A, class B>
+static void convert_copy(const A* src, B* dst, int64_t n, cudaStream_t s) {
+    if constexpr (std::is_same<A, B>::value) {
+        UP3D_CUDA(cudaMemcpyAsync(dst, src, sizeof(A) * n, cudaMemcpyDeviceToDevice, s));
     } else {
-        Level<float>& f = *a.Lf[0];
-        const int64_t n = f.A.n;
-        k_d2f<<<grid_for(n, 256), 256, 0, s>>>(r, f.b.get(), n);
-        UP3D_CHECK_LAUNCH();
-        vcycle<float>(a, a.Lf, 0, s);
-        k_f2d<<<grid_for(n, 256), 256, 0, s>>>(f.x.get(), z, n);
+        if constexpr (std::is_same<A, double>::value) k_d2f<<<grid_for(n, 256), 256, 0, s>>>(src, dst, n);
+        else k_f2d<<<grid_for(n, 256), 256, 0, s>>>(src, dst, n);
         UP3D_CHECK_LAUNCH();
     }
 }
 
-// The cycle's level buffers swap between sweeps; restoring them after each
-// cycle keeps every cycle (and every captured graph) on the same buffers.
+// Captures the body of the cycle at precision T.
 template <class T>
-std::vector<std::pair<T*, T*>> save_buffers(std::vector<Level<T>*>& L) {
-    std::vector<std::pair<T*, T*>> v;
-    for (auto* l : L) v.emplace_back(l->x.p, l->r.p);
-    return v;
-}
-template <class T>
-void restore_buffers(std::vector<Level<T>*>& L, const std::vector<std::pair<T*, T*>>& v) {
-    for (size_t i = 0; i < L.size(); ++i) {
-        L[i]->x.p = v[i].first;
-        L[i]->r.p = v[i].second;
-    }
-}
-
-// One V-cycle with FP32 input and output.
-void amg_cycle_f32(Amg& a, const float* r, float* z, cudaStream_t s) {
-    if (a.fp32) {
-        Level<float>& f = *a.Lf[0];
-        const int64_t n = f.A.n;
-        UP3D_CUDA(cudaMemcpyAsync(f.b.get(), r, sizeof(float) * n, cudaMemcpyDeviceToDevice, s));
-        vcycle<float>(a, a.Lf, 0, s);
-        UP3D_CUDA(cudaMemcpyAsync(z, f.x.get(), sizeof(float) * n, cudaMemcpyDeviceToDevice, s));
-    } else {
-        const int64_t n = a.Ld[0]->A.n;
-        k_f2d<<<grid_for(n, 256), 256, 0, s>>>(r, a.io64_in.get(), n);
-        UP3D_CHECK_LAUNCH();
-        amg_cycle(a, a.io64_in.get(), a.io64_out.get(), s);
-        k_d2f<<<grid_for(n, 256), 256, 0, s>>>(a.io64_out.get(), z, n);
-        UP3D_CHECK_LAUNCH();
-    }
-}
-
-// Replays the cached graph of one V-cycle for (r, z), capturing it first.
-void apply_graph(Amg& a, const void* r, void* z, bool f32, cudaStream_t s) {
-    for (auto& g : a.graphs)
-        if (g.r == r && g.z == z && g.f32 == f32) {
-            UP3D_CUDA(cudaGraphLaunch(g.exec, s));
-            count_launch((int)g.launches);
-            return;
-        }
-    if (f32 && !a.fp32) {
-        const int64_t n = a.Ld[0]->A.n;
-        a.io64_in.alloc(n);  // before the capture
-        a.io64_out.alloc(n);
-    }
+static void capture_body(Amg& a, std::vector<Level<T>*>& L, Amg::Body& body) {
     if (!a.capture_stream) UP3D_CUDA(cudaStreamCreateWithFlags(&a.capture_stream, cudaStreamNonBlocking));
-    auto sd = save_buffers(a.Ld);
-    auto sf = save_buffers(a.Lf);
+    // the levels' buffers swap between sweeps: put back afterwards
+    std::vector<std::pair<T*, T*>> saved;
+    for (auto* l : L) saved.emplace_back(l->x.p, l->r.p);
+    auto restore = [&] {
+        for (size_t i = 0; i < L.size(); ++i) {
+            L[i]->x.p = saved[i].first;
+            L[i]->r.p = saved[i].second;
+        }
+    };
     const long long l0 = g_launches.load();
     cudaGraph_t graph = nullptr;
     UP3D_CUDA(cudaStreamBeginCapture(a.capture_stream, cudaStreamCaptureModeThreadLocal));
     try {
-        if (f32) amg_cycle_f32(a, static_cast<const float*>(r), static_cast<float*>(z), a.capture_stream);
-        else amg_cycle(a, static_cast<const double*>(r), static_cast<double*>(z), a.capture_stream);
+        vcycle<T>(a, L, 0, true, a.capture_stream);
     } catch (...) {
         cudaStreamEndCapture(a.capture_stream, &graph);
         if (graph) cudaGraphDestroy(graph);
-        restore_buffers(a.Ld, sd);
-        restore_buffers(a.Lf, sf);
+        restore();
         throw;
     }
+    body.x = L[0]->x.p;
+    body.other = L[0]->r.p;
+    restore();
     UP3D_CUDA(cudaStreamEndCapture(a.capture_stream, &graph));
-    restore_buffers(a.Ld, sd);
-    restore_buffers(a.Lf, sf);
-    const long long launches = g_launches.load() - l0;
-    g_launches.fetch_sub(launches);  // counted at each replay instead
+    body.launches = g_launches.load() - l0;
+    g_launches.fetch_sub(body.launches);  // counted at each replay instead
     cudaGraphExec_t exec = nullptr;
     const cudaError_t e = cudaGraphInstantiate(&exec, graph, 0);
     cudaGraphDestroy(graph);
     UP3D_CUDA(e);
-    if (a.graphs.size() >= 16) {
-        cudaGraphExecDestroy(a.graphs.front().exec);
-        a.graphs.erase(a.graphs.begin());
+    body.exec = exec;
+}
+
+// One V-cycle z = M r at precision T on stream s.
+template <class T, class TIO>
+static void apply_cycle(Amg& a, std::vector<Level<T>*>& L, Amg::Body& body, const TIO* r, TIO* z, cudaStream_t s) {
+    Level<T>& f = *L[0];
+    const int64_t n = f.A.n;
+    if (L.size() == 1) {   // the dense solve alone
+        convert_copy(r, f.b.get(), n, s);
+        launch_kernel(false, k_dense_solve<T>, grid_for(32 * n, 256), 256, s, a.cinv.get(), n, f.b.get(), f.x.get());
+        convert_copy(f.x.get(), z, n, s);
+        return;
     }
-    a.graphs.push_back({r, z, f32, exec, launches});
-    UP3D_CUDA(cudaGraphLaunch(exec, s));
-    count_launch((int)launches);
+    if (!body.exec) capture_body<T>(a, L, body);
+    launch_kernel(false, k_jacobi_first<T, TIO>, grid_for(n, 256), 256, s, f.dinv.get(), r, f.b.get(), f.x.get(),
+                  f.omega, n);
+    UP3D_CUDA(cudaGraphLaunch(body.exec, s));
+    count_launch((int)body.launches);
+    T* x = static_cast<T*>(body.x);
+    T* last = static_cast<T*>(body.other);
+    if (a.post == 0) {
+        convert_copy(x, z, n, s);
+        return;
+    }
+    if constexpr (std::is_same<T, TIO>::value) last = z;
+    smooth<T, false>(false, f, x, last, s);
+    if constexpr (!std::is_same<T, TIO>::value) convert_copy(last, z, n, s);
 }
 
 void amg_apply(void* p, const double* r, double* z, cudaStream_t s) {
-    apply_graph(*static_cast<Amg*>(p), r, z, false, s);
+    Amg& a = *static_cast<Amg*>(p);
+    if (a.fp64) apply_cycle<double>(a, a.Ld, a.body64, r, z, s);
+    else apply_cycle<float>(a, a.Lf, a.body32, r, z, s);
 }
 
 void amg_apply_f32(void* p, const float* r, float* z, cudaStream_t s) {
-    apply_graph(*static_cast<Amg*>(p), r, z, true, s);
+    Amg& a = *static_cast<Amg*>(p);
+    if (a.fp32) apply_cycle<float>(a, a.Lf, a.body32, r, z, s);
+    else apply_cycle<double>(a, a.Ld, a.body64, r, z, s);
 }
 
 void amg_destroy(void* p) { delete static_cast<Amg*>(p); }
@@ -1668,7 +1645,6 @@ void amg_refresh(void* p, const up3d_csr& A, cudaStream_t s) {
     numeric(a, s);
     if (a.fp32) fill_levels<float>(a, a.Lf, s);
     if (a.fp64) fill_levels<double>(a, a.Ld, s);
-    a.drop_graphs();  // the smoothing weights are launch arguments of the graphs
 }
 
 const up3d_amg_info* amg_info(void* p) { return &static_cast<Amg*>(p)->info; }

@@ -125,15 +125,17 @@ inline bool use_sell(int64_t n, int64_t nnz, int64_t padded) {
 }
 inline unsigned sell_grid(int64_t n) { return (unsigned)((n + SELL_BLOCK - 1) / SELL_BLOCK); }
 
-// Sum of the slice's row `lane`, entries in row order.
-template <class T>
+// Sum of the slice's row `lane`, entries in row order.  `ready` is called
+// once the first batch of entries has been asked for and before the vector
+// is read.
+template <class T, class Ready>
 __device__ __forceinline__ T sell_row_sum(const int32_t* __restrict__ Sp, const int32_t* __restrict__ Si,
-                                          const T* __restrict__ Sx, const T* __restrict__ x, int64_t q, int lane) {
+                                          const T* __restrict__ Sx, const T* x, int64_t q, int lane, Ready ready) {
     const int32_t s = Sp[q], w = (Sp[q + 1] - s) >> 5;
     const int32_t* si = Si + s + lane;
     const T* sx = Sx + s + lane;
     T acc = T(0);
-    for (int32_t k0 = 0; k0 < w; k0 += SELL_BATCH) {   // warp-uniform
+    for (int32_t k0 = 0; k0 < w || k0 == 0; k0 += SELL_BATCH) {   // warp-uniform
         int32_t c[SELL_BATCH];
         T v[SELL_BATCH];
 #pragma unroll
@@ -141,6 +143,7 @@ __device__ __forceinline__ T sell_row_sum(const int32_t* __restrict__ Sp, const 
             c[j] = k0 + j < w ? ld_stream(si + (k0 + j) * 32) : -1;
             v[j] = k0 + j < w ? ld_stream(sx + (k0 + j) * 32) : T(0);
         }
+        if (k0 == 0) ready();
 #pragma unroll
         for (int j = 0; j < SELL_BATCH; ++j)
             if (c[j] >= 0) acc = fma(v[j], x[c[j]], acc);

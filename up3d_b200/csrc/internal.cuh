@@ -67,6 +67,30 @@ inline unsigned grid_for(int64_t n, int block, int64_t cap = 148 * 32) {
     return (unsigned)g;
 }
 
+// ------------------------------------------------------------ overlapped launches
+// A kernel that starts with pdl_trigger / pdl_wait may be launched while the
+// kernel before it on the stream drains (programmatic dependent launch):
+// what it does before pdl_wait must not touch anything an earlier kernel
+// of the chain writes.  Launched without the attribute, both are no-ops.
+
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <class... P, class... A>
+void launch_kernel(bool overlap, void (*kern)(P...), unsigned grid, int block, cudaStream_t s, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = overlap ? 1 : 0;
+    UP3D_CUDA(cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...));
+    UP3D_CHECK_LAUNCH();
+}
+
 // ------------------------------------------------------------ device buffer
 
 // Device blocks of the library's buffers (pool.cu): cudaMalloc'd, cached
