@@ -142,46 +142,101 @@ __device__ __forceinline__ void stream_extent(const int4 c, const double4* __res
     }
 }
 
-// rho_tilde_kernel_sweep (kernels/upwind.py:345-454).
-__global__ void k_rho_tilde_kernel(const int4* __restrict__ conn, const double4* __restrict__ X,
-                                   const double4* __restrict__ cen, const int64_t* __restrict__ nb_off,
-                                   const int32_t* __restrict__ nb_idx, const double* __restrict__ grad,
-                                   const double* __restrict__ q2, const double* __restrict__ rho, int64_t E, Flow F,
-                                   double reach_frac, double sig_s, double sig_p, double* __restrict__ nu_out,
-                                   double* __restrict__ rt_out, up3d_monitors* mon) {
+// Longest neighbourhood of each slice of 32 elements (times 32), and the
+// slices filled from the lists.
+__global__ void k_slice_widths(int64_t E, const int64_t* __restrict__ nb_off, int64_t* __restrict__ width) {
+    GRID_STRIDE(e, (E + 31) / 32 * 32) {   // whole warps
+        const int n = e < E ? (int)(nb_off[e + 1] - nb_off[e]) : 0;
+        const int w = __reduce_max_sync(0xffffffffu, n);
+        if ((e & 31) == 0) width[e >> 5] = 32 * (int64_t)w;
+    }
+}
+__global__ void k_slice_fill(int64_t E, const int64_t* __restrict__ nb_off, const int32_t* __restrict__ nb_idx,
+                             const int64_t* __restrict__ sp, int32_t* __restrict__ si) {
+    GRID_STRIDE(e, (E + 31) / 32 * 32) {
+        const int64_t q = e >> 5, s = sp[q] + (e & 31);
+        const int w = (int)((sp[q + 1] - sp[q]) >> 5);
+        const int64_t o = e < E ? nb_off[e] : 0;
+        const int n = e < E ? (int)(nb_off[e + 1] - o) : 0;
+        for (int j = 0; j < w; ++j) si[s + 32 * (int64_t)j] = j < n ? nb_idx[o + j] : -1;
+    }
+}
+
+// rho_tilde_kernel_sweep (kernels/upwind.py:345-454).  One thread per element,
+// the warp's neighbour lists interleaved (slices).
+//
+// The weights only matter where the switch can act: with the element and
+// every neighbour subcritical the sampled M^2, an average of theirs, is too,
+// and the density is the element's own.  So the neighbours' speeds are
+// looked at first (8 bytes each, no centroid, no exponential), against M_c^2
+// less a margin far above the average's rounding; a speed past the vacuum
+// limit or a NaN takes the full sum.  The sum runs at 64 registers for the
+// warps in flight: it is bound by the latency of its gathers and FP64 work.
+// 3.6 M tets, a supersonic pocket over the bump: 870 -> 253 us; with most
+// elements supersonic the full sum is what counts (1.8 M tets: 275 us, issue
+// slots 59 % busy, FP64 pipe 48 %; at 90 registers 42 % and 34 %).
+constexpr int NB_BATCH = 8;   // speeds asked for at once
+__global__ void __launch_bounds__(256, 4)
+    k_rho_tilde_kernel(const int4* __restrict__ conn, const double4* __restrict__ X, const double4* __restrict__ cen,
+                       const int64_t* __restrict__ sp, const int32_t* __restrict__ si,
+                       const double* __restrict__ grad, const double* __restrict__ q2,
+                       const double* __restrict__ rho, int64_t E, Flow F, double reach_frac, double sig_s,
+                       double sig_p, double* __restrict__ nu_out, double* __restrict__ rt_out, up3d_monitors* mon) {
     WMon acc;
+    const double mc2_low = F.mc2 * (1.0 - 1e-12);
     GRID_STRIDE(e, E) {
         const double gx = grad[3 * e], gy = grad[3 * e + 1], gz = grad[3 * e + 2];
         const double gmag = sqrt(dot3r(gx, gy, gz, gx, gy, gz));
         const double nu_e = switch_of(mach2_of(q2[e], F), F);
         const double re = rho[e];
         double nu = nu_e, rt = re;
-        if (gmag > 0.0) {
+        const int64_t q = e >> 5, s0 = sp[q];
+        const int w = (int)((sp[q + 1] - s0) >> 5);
+        const int32_t* list = si + s0 + (e & 31);
+        bool need = nu_e != 0.0;
+        for (int j0 = 0; j0 < w && !need; j0 += NB_BATCH) {
+            int32_t c[NB_BATCH];
+            double qc[NB_BATCH];
+#pragma unroll
+            for (int j = 0; j < NB_BATCH; ++j) c[j] = j0 + j < w ? list[32 * (j0 + j)] : -1;
+#pragma unroll
+            for (int j = 0; j < NB_BATCH; ++j) qc[j] = c[j] >= 0 ? q2[c[j]] : 0.0;
+#pragma unroll
+            for (int j = 0; j < NB_BATCH; ++j) {
+                const double base = base_of(qc[j], F);
+                need |= !(base > 0.0 && qc[j] * F.m2inf <= mc2_low * base);
+            }
+        }
+        if (need && gmag > 0.0) {
             const double vx = __ddiv_rn(gx, gmag), vy = __ddiv_rn(gy, gmag), vz = __ddiv_rn(gz, gmag);
             double pmin, pmax;
             stream_extent(conn[e], X, vx, vy, vz, pmin, pmax);
             const double extent = rsub(pmax, pmin);
             const double target = rmul(reach_frac, extent);
-            const double ss = rmul(sig_s, extent), sp = rmul(sig_p, extent);
+            const double ss = rmul(sig_s, extent), sd = rmul(sig_p, extent);
             const double inv2ss = __ddiv_rn(1.0, radd(rmul(2.0, rmul(ss, ss)), 1e-300));
-            const double inv2sp = __ddiv_rn(1.0, radd(rmul(2.0, rmul(sp, sp)), 1e-300));
+            const double inv2sp = __ddiv_rn(1.0, radd(rmul(2.0, rmul(sd, sd)), 1e-300));
             const double4 ce = cen[e];
             double w_sum = 0.0, rho_acc = 0.0, m2_acc = 0.0;
-            const int64_t j1 = nb_off[e + 1];
-            for (int64_t j = nb_off[e]; j < j1; ++j) {
-                const int32_t c = nb_idx[j];
-                const double4 cc = cen[c];
-                const double dx = rsub(cc.x, ce.x), dy = rsub(cc.y, ce.y), dz = rsub(cc.z, ce.z);
+            int32_t next = w > 0 ? list[0] : -1;
+            for (int j = 0; j < w; ++j) {
+                const int32_t c = next;
+                if (c < 0) break;
+                next = j + 1 < w ? list[32 * (j + 1)] : -1;
+                double cx, cy, cz, unused;
+                ld4(reinterpret_cast<const double*>(cen + c), cx, cy, cz, unused);
+                const double dx = rsub(cx, ce.x), dy = rsub(cy, ce.y), dz = rsub(cz, ce.z);
                 const double up = -dot3r(vx, vy, vz, dx, dy, dz);
                 if (up <= 0.0) continue;
+                const double rc = rho[c], qc = q2[c];
                 const double d2 = dot3r(dx, dy, dz, dx, dy, dz);
                 double perp2 = rsub(d2, rmul(up, up));
                 if (perp2 < 0.0) perp2 = 0.0;
                 const double du = rsub(up, target);
-                const double w = exp(-radd(rmul(rmul(du, du), inv2ss), rmul(perp2, inv2sp)));
-                w_sum = radd(w_sum, w);
-                rho_acc = radd(rho_acc, rmul(w, rho[c]));
-                m2_acc = radd(m2_acc, rmul(w, mach2_of(q2[c], F)));
+                const double wt = exp(-radd(rmul(rmul(du, du), inv2ss), rmul(perp2, inv2sp)));
+                w_sum = radd(w_sum, wt);
+                rho_acc = radd(rho_acc, rmul(wt, rc));
+                m2_acc = radd(m2_acc, rmul(wt, mach2_of(qc, F)));
             }
             if (w_sum > 0.0) {
                 const double rho_up = __ddiv_rn(rho_acc, w_sum), m2_up = __ddiv_rn(m2_acc, w_sum);
@@ -341,25 +396,48 @@ static int64_t neighborhood_offsets(const int4* fn, int64_t E, int depth, int64_
     return total;
 }
 
-// Builds (or reuses) the mesh's neighbourhood CSR of the given depth.
-// Synchronises the stream (the total sizes the index array).
+// The slices of the mesh's neighbourhood lists.  Synchronises the stream.
+static void neighborhood_slices(up3d_mesh* m, DBuf<unsigned char>& tmp, cudaStream_t s) {
+    const int64_t E = m->E, nq = (E + 31) / 32;
+    m->nb_sp.alloc(nq + 1);
+    UP3D_CUDA(cudaMemsetAsync(m->nb_sp.get(), 0, sizeof(int64_t), s));
+    if (E == 0) return;
+    DBuf<int64_t> width;
+    width.alloc(nq);
+    k_slice_widths<<<grid_for(E, 256), 256, 0, s>>>(E, m->nb_off.get(), width.get());
+    UP3D_CHECK_LAUNCH();
+    size_t bytes = 0;
+    UP3D_CUDA(cub::DeviceScan::InclusiveSum(nullptr, bytes, width.get(), m->nb_sp.get() + 1, nq, s));
+    tmp.alloc(bytes);
+    UP3D_CUDA(cub::DeviceScan::InclusiveSum(tmp.get(), bytes, width.get(), m->nb_sp.get() + 1, nq, s));
+    int64_t total = 0;
+    UP3D_CUDA(cudaMemcpyAsync(&total, m->nb_sp.get() + nq, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+    UP3D_CUDA(cudaStreamSynchronize(s));
+    m->nb_si.alloc(total > 0 ? total : 1);
+    k_slice_fill<<<grid_for(E, 256), 256, 0, s>>>(E, m->nb_off.get(), m->nb_idx.get(), m->nb_sp.get(), m->nb_si.get());
+    UP3D_CHECK_LAUNCH();
+    UP3D_CUDA(cudaStreamSynchronize(s));
+}
+
+// Builds (or reuses) the mesh's neighbourhood CSR of the given depth, and
+// its slices.  Synchronises the stream (the totals size the index arrays).
 void ensure_neighborhoods(up3d_mesh* m, int depth, cudaStream_t s) {
     if (m->nb_depth == depth) return;
     const int64_t E = m->E;
     m->nb_depth = 0;
     m->nb_off.alloc(E + 1);
+    DBuf<unsigned char> tmp;
     if (depth > NB_MAX_DEPTH) {
         m->nb_total = neighborhoods_host(m->fnbr.get(), E, depth, m->nb_off.get(), &m->nb_idx, nullptr, s);
-        m->nb_depth = depth;
-        return;
+    } else {
+        const int64_t total = neighborhood_offsets(m->fnbr.get(), E, depth, m->nb_off.get(), tmp, s);
+        m->nb_idx.alloc(total > 0 ? total : 1);
+        k_neighborhoods<true><<<grid_for(E, 128), 128, 0, s>>>(m->fnbr.get(), E, depth, nullptr, m->nb_off.get(),
+                                                              m->nb_idx.get());
+        UP3D_CHECK_LAUNCH();
+        m->nb_total = total;
     }
-    DBuf<unsigned char> tmp;
-    const int64_t total = neighborhood_offsets(m->fnbr.get(), E, depth, m->nb_off.get(), tmp, s);
-    m->nb_idx.alloc(total > 0 ? total : 1);
-    k_neighborhoods<true><<<grid_for(E, 128), 128, 0, s>>>(m->fnbr.get(), E, depth, nullptr, m->nb_off.get(),
-                                                          m->nb_idx.get());
-    UP3D_CHECK_LAUNCH();
-    m->nb_total = total;
+    neighborhood_slices(m, tmp, s);
     m->nb_depth = depth;
 }
 
@@ -433,7 +511,7 @@ int up3d_rho_tilde_kernel(up3d_mesh* m, const double* grad, const double* q2, co
         ensure_neighborhoods(m, depth, s);
         if (mon) UP3D_CUDA(cudaMemsetAsync(mon, 0, sizeof(up3d_monitors), s));
         k_rho_tilde_kernel<<<grid_for(m->E, 256), 256, 0, s>>>(
-            m->conn.get(), m->nodes4.get(), m->cen.get(), m->nb_off.get(), m->nb_idx.get(), grad, q2, rho, m->E,
+            m->conn.get(), m->nodes4.get(), m->cen.get(), m->nb_sp.get(), m->nb_si.get(), grad, q2, rho, m->E,
             make_flow(*flow), reach_frac, sigma_s_frac, sigma_p_frac, nu, rho_tilde, mon);
         UP3D_CHECK_LAUNCH();
     });
