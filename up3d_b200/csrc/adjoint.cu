@@ -13,15 +13,13 @@
 //   pass 1 (per element e): c_e = V_e (g_e . h_e), h_e = sum_i lam_i B_e,i;
 //     t_e = c_e s_e + w_e (weight on q2_e), a_e = c_e s_u (weight on q2 of
 //     u(e)), and c_e d rho~_e / dM by forward-mode differentiation;
-//   the a_e are summed per upstream element in ascending e (stable sort);
+//   the a_e are chained per upstream element and summed in integers;
 //   pass 2 (per element k): dL/dB_k,j = rho~ V (phi_j h + lam_j g)
 //     + Q_k (2/u^2) phi_j g with Q_k = t_k + sum a, dL/dV_k = rho~ (g . h),
 //     then through B = D^-1 (rows), V = |det D| / 6 with D = [x1-x0, x2-x0,
 //     x3-x0]:  dL/dD = -B^T G B^T + dL/dV V B^T;
 //   node gathers over the node -> element entries (fixed order).
 // Everything is deterministic (no atomics on values).
-
-#include <cub/cub.cuh>
 
 #include "elem.cuh"
 #include "internal.cuh"
@@ -51,52 +49,67 @@ __device__ __forceinline__ Dual dpow(Dual a, double p) {
     return {v, p * pow(a.v, p - 1.0) * a.d};
 }
 
+// a^2.5 (air) by the square root, as rho_drho does
+__device__ __forceinline__ Dual dpow25(Dual a) {
+    const double s = sqrt(a.v);
+    return {a.v * a.v * s, 2.5 * (a.v * s) * a.d};
+}
+
 struct FlowM {  // the Mach-independent flow constants
     double gamma, hgm, expo, mc2, C, floor_, mcap2;
+    bool air;   // gamma == 1.4
 };
 
-// density of the limited speed, as a function of M (q2n fixed): the
-// limiter cap q2(M_cap) moves with M (physics/isentropic.py:262-314)
-__device__ Dual rho_dual(double q2n, Dual m2, const FlowM& F, Dual& q2l, Dual& b) {
+// the limited speed and the isentropic base as functions of M (q2n fixed):
+// the limiter cap q2(M_cap) moves with M (physics/isentropic.py:262-314)
+__device__ __forceinline__ void base_dual(double q2n, Dual m2, const FlowM& F, Dual& q2l, Dual& b) {
     const Dual cap = (dconst(F.mcap2) * (dconst(1.0) + dconst(F.hgm) * m2)) /
                      (m2 * dconst(1.0 + F.hgm * F.mcap2));
     q2l = q2n < cap.v ? dconst(q2n) : cap;
     b = dconst(1.0) + dconst(F.hgm) * m2 * (dconst(1.0) - q2l);
     if (b.v < 1e-10) b = dconst(1e-10);
-    return dpow(b, F.expo);
 }
+__device__ __forceinline__ Dual rho_dual(Dual b, const FlowM& F) { return F.air ? dpow25(b) : dpow(b, F.expo); }
 
 // nu = C max(0, 1 - M_c^2 / max(M^2, M_c^2)) of the local Mach number
-__device__ Dual nu_dual(Dual q2l, Dual b, Dual m2, const FlowM& F) {
+__device__ __forceinline__ Dual nu_dual(Dual q2l, Dual b, Dual m2, const FlowM& F) {
     const Dual ml2 = q2l * m2 / b;
     if (ml2.v > F.mc2) return dconst(F.C) * (dconst(1.0) - dconst(F.mc2) / ml2);
     return dconst(0.0);
 }
 
-// d rho~ / dM at fixed speeds, upstream and (frozen) branch; br < 0: live
-__device__ double drho_tilde_dM(double q2n_e, double q2n_u, bool self_up, int br, double m_inf, const FlowM& F) {
+// d rho~ / dM at fixed speeds, upstream and (frozen) branch; br < 0: live.
+// The upstream density only enters where the switch is on.
+__device__ __forceinline__ double drho_tilde_dM(double q2n_e, double q2n_u, bool self_up, int br, double m_inf,
+                                                const FlowM& F) {
+    if (br == 3) return 0.0;
     const Dual M = {m_inf, 1.0};
     const Dual m2 = M * M;
     Dual q2e, be, q2u, bu;
-    const Dual rho_e = rho_dual(q2n_e, m2, F, q2e, be);
-    if (br == 3) return 0.0;
+    base_dual(q2n_e, m2, F, q2e, be);
+    const Dual rho_e = rho_dual(be, F);
     if (br == 0) return rho_e.d;
-    const Dual rho_u = self_up ? rho_e : rho_dual(q2n_u, m2, F, q2u, bu);
     if (self_up) {
         q2u = q2e;
         bu = be;
+    } else {
+        base_dual(q2n_u, m2, F, q2u, bu);
     }
-    Dual rt;
-    if (br == 1 || br == 2) {
-        const Dual nu = br == 1 ? nu_dual(q2e, be, m2, F) : nu_dual(q2u, bu, m2, F);
+    Dual nu;
+    if (br == 1) {
+        nu = nu_dual(q2e, be, m2, F);
+    } else if (br == 2) {
+        nu = nu_dual(q2u, bu, m2, F);
+    } else {   // live: nu = max(nu_e, nu_u), floored result
+        const Dual nu_e = nu_dual(q2e, be, m2, F), nu_u = nu_dual(q2u, bu, m2, F);
+        nu = nu_e.v >= nu_u.v ? nu_e : nu_u;
+    }
+    Dual rt = rho_e;
+    if (nu.v != 0.0 || nu.d != 0.0) {
+        const Dual rho_u = self_up ? rho_e : rho_dual(bu, F);
         rt = rho_e - nu * (rho_e - rho_u);
-        return rt.d;
     }
-    // live: nu = max(nu_e, nu_u), floored result
-    const Dual nu_e = nu_dual(q2e, be, m2, F), nu_u = nu_dual(q2u, bu, m2, F);
-    const Dual nu = nu_e.v >= nu_u.v ? nu_e : nu_u;
-    rt = rho_e - nu * (rho_e - rho_u);
-    return rt.v > F.floor_ ? rt.d : 0.0;
+    return br >= 0 || rt.v > F.floor_ ? rt.d : 0.0;
 }
 
 // ------------------------------------------------------------ passes
@@ -108,15 +121,20 @@ __device__ __forceinline__ void lam_grad(const int4 c, const double* b, const do
 }
 
 // Pass 1: per element, the weights on its own speed (t), on its upstream
-// element's speed (a), rho~, and c_e d rho~/dM summed per block.
-__global__ void __launch_bounds__(256)
+// element's speed (a, chained per upstream element where not zero), rho~, and
+// c_e d rho~/dM summed per block.
+// AIR: gamma == 1.4, compiled without the pow calls, whose registers halve the
+// warps in flight.
+template <bool AIR>
+__global__ void __launch_bounds__(256, AIR ? 3 : 2)
     k_vjp_elem(const int4* __restrict__ conn, const double* __restrict__ B, const double* __restrict__ V,
                const double* __restrict__ phi, Flow F, FlowM FM, double m_inf, double u2,
                const int64_t* __restrict__ up, const int8_t* __restrict__ br, int64_t E,
                const double* __restrict__ lam, const double* __restrict__ w, double* __restrict__ t_out,
-               double* __restrict__ a_out, double* __restrict__ rt_out, int32_t* __restrict__ key,
-               int32_t* __restrict__ val, double* __restrict__ partial) {
+               double* __restrict__ a_out, double* __restrict__ rt_out, int32_t* __restrict__ head,
+               int32_t* __restrict__ next, double* __restrict__ partial) {
     __shared__ double sh[8];
+    F.air = FM.air = AIR;
     double dm = 0.0;
     GRID_STRIDE(e, E) {
         double g[3], b[12];
@@ -162,10 +180,12 @@ __global__ void __launch_bounds__(256)
             if (cval != 0.0) dm += cval * drho_tilde_dM(q2n, q2nu, u == e, bb, m_inf, FM);
         }
         t_out[e] = cval * se + (w ? w[e] : 0.0);
-        a_out[e] = u != e ? cval * su : 0.0;
         rt_out[e] = rt;
-        key[e] = (int32_t)u;
-        val[e] = (int32_t)e;
+        const double a = u != e ? cval * su : 0.0;
+        if (a != 0.0) {   // into the chain of u
+            a_out[e] = a;
+            next[e] = atomicExch(head + u, (int32_t)e);
+        }
     }
     dm = warp_sum(dm);
     if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = dm;
@@ -185,16 +205,27 @@ __global__ void k_vjp_sum_partials(const double* __restrict__ partial, int nb, d
     if (threadIdx.x == 0) *out = s;
 }
 
-// A[k] = sum of a_e over the elements e (ascending) whose upstream is k.
-__global__ void k_vjp_upstream_sums(const int32_t* __restrict__ key, const int32_t* __restrict__ val,
-                                    const double* __restrict__ a, int64_t E, double* __restrict__ A) {
-    GRID_STRIDE(i, E) {
-        const int32_t k = key[i];
-        if (i > 0 && key[i - 1] == k) continue;
-        double s = 0.0;
-        for (int64_t j = i; j < E && key[j] == k; ++j) s += a[val[j]];
-        A[k] = s;
+// Sum of a_e over the chain starting at element i (in whatever order the
+// chain was built): the values as integers on a scale that gives the
+// largest 62 bits, added in 128 bits, so the sum is exact to 2^-62 of the
+// largest and the same for every order.  A stable sort by upstream element
+// and per-run sums, in its place, took 50 of the 283 us of a residual forward
+// and backward at 450 k tets.
+__device__ __forceinline__ double chain_sum(const int32_t* __restrict__ next, const double* __restrict__ a, int32_t i) {
+    if (i < 0) return 0.0;
+    const double first = a[i];
+    if (next[i] < 0) return first;
+    double big = 0.0, plain = 0.0;
+    for (int32_t j = i; j >= 0; j = next[j]) {
+        big = fmax(big, fabs(a[j]));
+        plain += a[j];
     }
+    if (!(big > 0.0 && big < INFINITY && plain - plain == 0.0)) return plain;   // infinities and NaN propagate
+    const int shift = 61 - ilogb(big);
+    __int128 sum = 0;
+    for (int32_t j = i; j >= 0; j = next[j]) sum += (long long)rint(ldexp(a[j], shift));
+    const double hi = (double)(long long)(sum >> 64), lo = (double)(unsigned long long)sum;
+    return ldexp(hi * 18446744073709551616.0 + lo, -shift);
 }
 
 // Pass 2: per element, dL/dB and dL/dV through the inverse edge matrix to
@@ -202,8 +233,9 @@ __global__ void k_vjp_upstream_sums(const int32_t* __restrict__ key, const int32
 __global__ void __launch_bounds__(256)
     k_vjp_geom(const int4* __restrict__ conn, const double* __restrict__ B, const double* __restrict__ V,
                const double* __restrict__ phi, double u2, int64_t E, const double* __restrict__ lam,
-               const double* __restrict__ w, const double* __restrict__ t, const double* __restrict__ A,
-               const double* __restrict__ rt, double* __restrict__ dx, double* __restrict__ dphi) {
+               const double* __restrict__ w, const double* __restrict__ t, const double* __restrict__ a,
+               const int32_t* __restrict__ head, const int32_t* __restrict__ next, const double* __restrict__ rt,
+               double* __restrict__ dx, double* __restrict__ dphi) {
     GRID_STRIDE(e, E) {
         double g[3], b[12];
         int4 c;
@@ -218,7 +250,7 @@ __global__ void __launch_bounds__(256)
             l[3] = lam[c.w];
         }
         const double Ve = V[e], r = rt[e];
-        const double Q = t[e] + A[e];
+        const double Q = t[e] + chain_sum(next, a, head[e]);
         const double q2w = 2.0 * Q / u2;
         double G[4][3];
 #pragma unroll
@@ -267,21 +299,38 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-// Node sums over the node -> element entries in their fixed order.
-__global__ void k_vjp_gather(int64_t N, const int32_t* __restrict__ ent_off, const uint32_t* __restrict__ ent,
-                             const double* __restrict__ dx, const double* __restrict__ dphi_e,
-                             double* __restrict__ dX, double* __restrict__ dphi) {
-    GRID_STRIDE(n, N) {
+// Node sums over the node -> element entries, eight lanes per node: lane
+// `sub` adds the entries sub, sub + 8, ..., then a fixed tree over the lanes
+// (one thread per node: 27 us at 450 k tets).
+__global__ void __launch_bounds__(256)
+    k_vjp_gather(int64_t N, const int32_t* __restrict__ ent_off, const uint32_t* __restrict__ ent,
+                 const double* __restrict__ dx, const double* __restrict__ dphi_e, double* __restrict__ dX,
+                 double* __restrict__ dphi) {
+    constexpr int LPR = 8, RPW = 32 / LPR;
+    const int sub = threadIdx.x & (LPR - 1);
+    const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+    const int64_t n_warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    for (int64_t base = warp * RPW; base < N; base += n_warps * RPW) {   // warp-uniform
+        const int64_t n = base + (threadIdx.x & 31) / LPR;
         double sx = 0.0, sy = 0.0, sz = 0.0, sp = 0.0;
-        for (int32_t k = ent_off[n]; k < ent_off[n + 1]; ++k) {
-            const uint32_t x = ent[k];
-            const int64_t e = x >> 2;
-            const int i = x & 3;
-            sx += dx[12 * e + 3 * i];
-            sy += dx[12 * e + 3 * i + 1];
-            sz += dx[12 * e + 3 * i + 2];
-            if (dphi) sp += dphi_e[4 * e + i];
+        if (n < N)
+            for (int32_t k = ent_off[n] + sub; k < ent_off[n + 1]; k += LPR) {
+                const uint32_t x = ent[k];
+                const int64_t e = x >> 2;
+                const int i = x & 3;
+                sx += dx[12 * e + 3 * i];
+                sy += dx[12 * e + 3 * i + 1];
+                sz += dx[12 * e + 3 * i + 2];
+                if (dphi) sp += dphi_e[4 * e + i];
+            }
+#pragma unroll
+        for (int o = LPR / 2; o > 0; o >>= 1) {
+            sx += __shfl_down_sync(0xffffffffu, sx, o, LPR);
+            sy += __shfl_down_sync(0xffffffffu, sy, o, LPR);
+            sz += __shfl_down_sync(0xffffffffu, sz, o, LPR);
+            sp += __shfl_down_sync(0xffffffffu, sp, o, LPR);
         }
+        if (sub != 0 || n >= N) continue;
         if (dX) {
             dX[3 * n] = sx;
             dX[3 * n + 1] = sy;
@@ -315,47 +364,35 @@ int up3d_residual_vjp(up3d_mesh* m, const double* phi, const up3d_flow* flow, co
         const int64_t E = m->E, N = m->N;
         const Flow F = make_flow(*flow);
         FlowM FM{flow->gamma, 0.5 * (flow->gamma - 1.0), 1.0 / (flow->gamma - 1.0),
-                 flow->m_crit * flow->m_crit, flow->upwind_c, flow->rho_floor, flow->m_cap * flow->m_cap};
+                 flow->m_crit * flow->m_crit, flow->upwind_c, flow->rho_floor, flow->m_cap * flow->m_cap,
+                 flow->gamma == 1.4};
         const double u2 = flow->u_inf * flow->u_inf;
         m->adj_t.alloc(E);
         m->adj_a.alloc(E);
         m->adj_rt.alloc(E);
-        m->adj_A.alloc(E);
         m->adj_dx.alloc(12 * E);
         m->adj_dphi.alloc(4 * E);
-        m->adj_key.alloc(E);
-        m->adj_key_s.alloc(E);
-        m->adj_val.alloc(E);
-        m->adj_val_s.alloc(E);
+        m->adj_head.alloc(E);
+        m->adj_next.alloc(E);
         const unsigned grid = grid_for(E, 256, (int64_t)148 * 8);
         m->adj_part.alloc(grid + 1);
-        k_vjp_elem<<<grid, 256, 0, s>>>(m->conn.get(), m->B.get(), m->V.get(), phi, F, FM, flow->m_inf, u2,
+        UP3D_CUDA(cudaMemsetAsync(m->adj_head.get(), 0xff, sizeof(int32_t) * E, s));   // -1: empty chains
+        auto elem = F.air ? k_vjp_elem<true> : k_vjp_elem<false>;
+        elem<<<grid, 256, 0, s>>>(m->conn.get(), m->B.get(), m->V.get(), phi, F, FM, flow->m_inf, u2,
                                         upstream, branch, E, lam, w_q2, m->adj_t.get(), m->adj_a.get(),
-                                        m->adj_rt.get(), m->adj_key.get(), m->adj_val.get(), m->adj_part.get());
+                                        m->adj_rt.get(), m->adj_head.get(), m->adj_next.get(), m->adj_part.get());
         UP3D_CHECK_LAUNCH();
         if (dM) {
             k_vjp_sum_partials<<<1, 32, 0, s>>>(m->adj_part.get(), (int)grid, dM);
             UP3D_CHECK_LAUNCH();
         }
-        // upstream sums: stable sort by upstream element, then per-key runs
-        int end_bit = 1;
-        while ((1ll << end_bit) < E) ++end_bit;
-        size_t bytes = 0;
-        UP3D_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, bytes, m->adj_key.get(), m->adj_key_s.get(),
-                                                  m->adj_val.get(), m->adj_val_s.get(), E, 0, end_bit, s));
-        m->cub_tmp.alloc(bytes);
-        UP3D_CUDA(cub::DeviceRadixSort::SortPairs(m->cub_tmp.get(), bytes, m->adj_key.get(), m->adj_key_s.get(),
-                                                  m->adj_val.get(), m->adj_val_s.get(), E, 0, end_bit, s));
-        UP3D_CUDA(cudaMemsetAsync(m->adj_A.get(), 0, sizeof(double) * E, s));
-        k_vjp_upstream_sums<<<grid_for(E, 256), 256, 0, s>>>(m->adj_key_s.get(), m->adj_val_s.get(),
-                                                             m->adj_a.get(), E, m->adj_A.get());
-        UP3D_CHECK_LAUNCH();
         k_vjp_geom<<<grid_for(E, 256), 256, 0, s>>>(m->conn.get(), m->B.get(), m->V.get(), phi, u2, E, lam, w_q2,
-                                                    m->adj_t.get(), m->adj_A.get(), m->adj_rt.get(),
+                                                    m->adj_t.get(), m->adj_a.get(), m->adj_head.get(),
+                                                    m->adj_next.get(), m->adj_rt.get(),
                                                     m->adj_dx.get(), dphi ? m->adj_dphi.get() : nullptr);
         UP3D_CHECK_LAUNCH();
         if (dX || dphi) {
-            k_vjp_gather<<<grid_for(N, 256), 256, 0, s>>>(N, m->ent_off.get(), m->ent.get(), m->adj_dx.get(),
+            k_vjp_gather<<<grid_for(N, 32, (int64_t)m->n_sms * 64), 256, 0, s>>>(N, m->ent_off.get(), m->ent.get(), m->adj_dx.get(),
                                                           m->adj_dphi.get(), dX, dphi);
             UP3D_CHECK_LAUNCH();
         }

@@ -215,11 +215,11 @@ struct up3d_mesh {
     up3d::DBuf<int32_t> t3c_seg, t3c_cnt;   // segment offsets / lengths
     up3d::DBuf<int64_t> t3c_nruns;
     // adjoint (residual vector-Jacobian products), grown on demand
-    up3d::DBuf<double> adj_t, adj_a, adj_rt, adj_A;   // (E) each
+    up3d::DBuf<double> adj_t, adj_a, adj_rt;          // (E) each
     up3d::DBuf<double> adj_dx;                        // (E, 12) per-element node gradients
     up3d::DBuf<double> adj_dphi;                      // (E, 4)
     up3d::DBuf<double> adj_part;                      // reduction partials
-    up3d::DBuf<int32_t> adj_key, adj_key_s, adj_val, adj_val_s;  // (E) upstream -> element sort
+    up3d::DBuf<int32_t> adj_head, adj_next;           // (E) each: chains of elements per upstream element
     up3d::DBuf<up3d::Flow> flows_ws;   // per-case flows of batched evaluations
     up3d::DBuf<up3d_monitors> mon_ws;  // (1)
     up3d::DBuf<int64_t> i64_ws;        // small scalars
