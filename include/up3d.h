@@ -221,6 +221,12 @@ int up3d_jacobian_data(up3d_mesh* mesh, const double* phi, const double* rho_til
 int up3d_jacobian_export(up3d_mesh* mesh, const double* data, int32_t* indptr,
                          int32_t* indices, double* merged, up3d_stream stream);
 
+/* The same with newton_nnz read back (synchronous), for callers that size
+ * indices and merged by the most there can be: the P1 nnz plus the extras
+ * (up3d_monitors.n_term3_extra, or up3d_jacobian's n_extra). */
+int up3d_jacobian_merge(up3d_mesh* mesh, const double* data, int32_t* indptr, int32_t* indices,
+                        double* merged, int64_t* newton_nnz, up3d_stream stream);
+
 /* newton_nnz of the last Jacobian (kernels/jacobian.py:358): the P1 nnz, or,
  * when Term 3 is active, the non-zeros of the merged matrix.  Synchronous. */
 int up3d_jacobian_nnz(up3d_mesh* mesh, const double* data, int64_t* newton_nnz,

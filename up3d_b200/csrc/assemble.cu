@@ -282,18 +282,21 @@ __global__ void k_prep_matrix(const double* __restrict__ B, const double* __rest
 // assemble_newton_jacobian (kernels/jacobian.py:323-338, :410-414): the
 // limiter mask gates s_e by lim[e] and s_u by lim[upstream[e]]; Term-2 and
 // Term-3 weights 2 inv_u2 s V; Term-3 vectors of active elements
-// (s_u != 0).  `grad` holds grad(phi) of every element.
-__global__ void k_prep_jacobian(const double* __restrict__ B, const double* __restrict__ V,
-                                const double* __restrict__ grad, const double* __restrict__ rt,
-                                const double* __restrict__ se, const double* __restrict__ su,
-                                const int64_t* __restrict__ up, const uint8_t* __restrict__ lim, double inv_u2,
-                                int64_t E, double* __restrict__ loc, double* __restrict__ t3v,
-                                uint8_t* __restrict__ t3flag, int32_t* __restrict__ up32) {
+// (s_u != 0), counted into *n_active.  grad(phi) of the element, and of an
+// active element's upstream, is formed here (the reference's scratch
+// velocities, :328-332).
+__global__ void k_prep_jacobian(const int4* __restrict__ conn, const double* __restrict__ B,
+                                const double* __restrict__ V, const double* __restrict__ phi,
+                                const double* __restrict__ rt, const double* __restrict__ se,
+                                const double* __restrict__ su, const int64_t* __restrict__ up,
+                                const uint8_t* __restrict__ lim, double inv_u2, int64_t E, double* __restrict__ loc,
+                                double* __restrict__ t3v, uint8_t* __restrict__ t3flag, int32_t* __restrict__ up32,
+                                unsigned long long* __restrict__ n_active) {
+    unsigned long long count = 0;
     GRID_STRIDE(e, E) {
-        double b[12];
-        load_B(B, e, b);
-        double g[3] = {grad[3 * e], grad[3 * e + 1], grad[3 * e + 2]};
-        double gB[4];
+        double b[12], g[3], gB[4];
+        int4 c;
+        elem_grad_B(conn, B, phi, e, g, b, c);
         gB_of(g, b, gB);
         int64_t u = safe_up(up[e], e, E);
         double s_e = se[e], s_u = su[e];
@@ -306,16 +309,19 @@ __global__ void k_prep_jacobian(const double* __restrict__ B, const double* __re
         const double w3 = 2.0 * inv_u2 * s_u * Ve;
         const bool active = s_u != 0.0;
         if (active) {
-            double bu[12], f[4];
-            load_B(B, u, bu);
-            double gu[3] = {grad[3 * u], grad[3 * u + 1], grad[3 * u + 2]};
+            double bu[12], gu[3], f[4];
+            int4 cu;
+            elem_grad_B(conn, B, phi, u, gu, bu, cu);
             gB_of(gu, bu, f);
             store_t3(t3v, e, w3, gB, f);
+            ++count;
         }
         t3flag[e] = active ? 1 : 0;
         up32[e] = (int32_t)u;
         store_local(loc, e, b, gB, rt[e] * Ve, w2, false);
     }
+    count = warp_sum_u64(count);
+    if ((threadIdx.x & 31) == 0 && count) atomicAdd(n_active, count);
 }
 
 // ------------------------------------------------------------ fused sweep
@@ -991,11 +997,25 @@ __global__ void __launch_bounds__(256)
 // (e << 4 | i << 2 | k) and destination at 4 ent_off[n] + position: the P1
 // slot, or -1 - (the extra's rank in its row); unused positions of the
 // row's region get INT32_MAX.
+//
+// row_on: rows with an incident active element (k_t3_mark).  A warp looks at
+// 32 of its rows' flags at a time and walks the entries of the flagged ones
+// only: with a supersonic pocket nine rows in ten have none (3.6 M tets: 137 us
+// when every row's entries were read).
+__global__ void k_t3_mark(int64_t E, const uint8_t* __restrict__ flag, const int4* __restrict__ conn,
+                          uint8_t* __restrict__ row_on) {
+    GRID_STRIDE(e, E) {
+        if (!flag[e]) continue;
+        const int4 c = conn[e];
+        row_on[c.x] = row_on[c.y] = row_on[c.z] = row_on[c.w] = 1;
+    }
+}
+
 template <int WARPS, bool RECORD>
 __global__ void __launch_bounds__(WARPS * 32)
     k_t3_rows(int64_t N, int cap, const int32_t* __restrict__ ent_off, const uint32_t* __restrict__ ent,
-              const uint8_t* __restrict__ flag, const int32_t* __restrict__ up, const int4* __restrict__ conn,
-              const double* __restrict__ t3v, const int32_t* __restrict__ indptr,
+              const uint8_t* __restrict__ row_on, const uint8_t* __restrict__ flag, const int32_t* __restrict__ up,
+              const int4* __restrict__ conn, const double* __restrict__ t3v, const int32_t* __restrict__ indptr,
               const int32_t* __restrict__ indices, double* __restrict__ data, int32_t* __restrict__ xs_col,
               double* __restrict__ xs_val, int32_t* __restrict__ x_cnt, uint32_t* __restrict__ rec_code,
               int32_t* __restrict__ rec_key) {
@@ -1014,142 +1034,160 @@ __global__ void __launch_bounds__(WARPS * 32)
     const unsigned lt = (1u << lane) - 1u;
     const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t n_warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t n = warp; n < N; n += n_warps) {
-        const int32_t eb = ent_off[n], deg = ent_off[n + 1] - eb;
-        // 1. the row's entries in (element, k) order
-        int P = 0;
-        for (int base = 0; base < deg; base += 32) {
-            const int j = base + lane;
-            uint32_t x = 0;
-            bool act = false;
-            if (j < deg) {
-                x = ent[eb + j];
-                act = flag[x >> 2] != 0;
-            }
-            const unsigned m = __ballot_sync(0xffffffffu, act);
-            if (act) {
-                const int64_t e = x >> 2;
-                const int i = x & 3;
-                const int4 cu = conn[up[e]];
-                const double* t = t3v + 8 * e;
-                const double ai = t[i];
-                const int pos = P + 4 * __popc(m & lt);
-                if (RECORD) {
-                    uint32_t* rc = rec_code + 4 * (int64_t)eb + pos;
+    for (int64_t first = warp; first < N; first += 32 * n_warps) {   // warp-uniform
+        const int64_t mine = first + lane * n_warps;
+        const bool on = mine < N && row_on[mine];
+        if (!RECORD && mine < N && !on) x_cnt[mine] = 0;
+        unsigned todo = __ballot_sync(0xffffffffu, RECORD ? mine < N : on);
+        for (; todo; todo &= todo - 1) {
+            const int64_t n = first + (__ffs(todo) - 1) * n_warps;
+            const int32_t eb = ent_off[n], deg = ent_off[n + 1] - eb;
+            // 1. the row's entries in (element, k) order
+            int P = 0;
+            for (int base = 0; base < deg; base += 32) {
+                const int j = base + lane;
+                uint32_t x = 0;
+                bool act = false;
+                if (j < deg) {
+                    x = ent[eb + j];
+                    act = flag[x >> 2] != 0;
+                }
+                const unsigned m = __ballot_sync(0xffffffffu, act);
+                if (act) {
+                    const int64_t e = x >> 2;
+                    const int i = x & 3;
+                    const int4 cu = conn[up[e]];
+                    const double* t = t3v + 8 * e;
+                    const double ai = t[i];
+                    const int pos = P + 4 * __popc(m & lt);
+                    if (RECORD) {
+                        uint32_t* rc = rec_code + 4 * (int64_t)eb + pos;
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) rc[k] = ((uint32_t)e << 4) | (uint32_t)(i << 2) | (uint32_t)k;
-                }
-                col0[pos] = cu.x;
-                col0[pos + 1] = cu.y;
-                col0[pos + 2] = cu.z;
-                col0[pos + 3] = cu.w;
-                val0[pos] = ai * t[4];
-                val0[pos + 1] = ai * t[5];
-                val0[pos + 2] = ai * t[6];
-                val0[pos + 3] = ai * t[7];
-            }
-            P += 4 * __popc(m);
-        }
-        if (P == 0) {
-            if (lane == 0) x_cnt[n] = 0;
-            if (RECORD)
-                for (int p = lane; p < 4 * deg; p += 32) rec_key[4 * (int64_t)eb + p] = INT32_MAX;
-            continue;
-        }
-        __syncwarp();
-        // 2. the distinct columns in order of first appearance, each with the
-        //    sequential sum of its entries in (element, k) order: chunks of 32
-        //    entries, equal columns grouped by match_any, the group's lowest
-        //    lane adding the group's values in lane (= entry) order to the
-        //    column's running sum -- the reference's duplicate summation order
-        int D = 0;
-        for (int base = 0; base < P; base += 32) {
-            const int p = base + lane;
-            const bool valid = p < P;
-            const int32_t c = valid ? col0[p] : -1 - lane;  // idle lanes: distinct dummies
-            const unsigned grp = __match_any_sync(0xffffffffu, c);
-            const bool leader = valid && (__ffs(grp) - 1) == lane;
-            int idx = -1;
-            if (leader)
-                for (int d = 0; d < D; ++d)
-                    if (col1[d] == c) {
-                        idx = d;
-                        break;
+                        for (int k = 0; k < 4; ++k) rc[k] = ((uint32_t)e << 4) | (uint32_t)(i << 2) | (uint32_t)k;
                     }
-            const unsigned newm = __ballot_sync(0xffffffffu, leader && idx < 0);
-            if (leader) {
-                double acc_c = 0.0;
-                if (idx < 0) idx = D + __popc(newm & lt);
-                else acc_c = val1[idx];
-                unsigned gm = grp;
-                while (gm) {
-                    const int j = __ffs(gm) - 1;
-                    gm &= gm - 1;
-                    acc_c += val0[base + j];
-                    if (RECORD) eidx[base + j] = (int16_t)idx;
+                    col0[pos] = cu.x;
+                    col0[pos + 1] = cu.y;
+                    col0[pos + 2] = cu.z;
+                    col0[pos + 3] = cu.w;
+                    val0[pos] = ai * t[4];
+                    val0[pos + 1] = ai * t[5];
+                    val0[pos + 2] = ai * t[6];
+                    val0[pos + 3] = ai * t[7];
                 }
-                col1[idx] = c;
-                val1[idx] = acc_c;
+                P += 4 * __popc(m);
             }
-            D += __popc(newm);
+            if (P == 0) {
+                if (lane == 0) x_cnt[n] = 0;
+                if (RECORD)
+                    for (int p = lane; p < 4 * deg; p += 32) rec_key[4 * (int64_t)eb + p] = INT32_MAX;
+                continue;
+            }
             __syncwarp();
-        }
-        // 3. per distinct column: into the P1 slot, else an extra; extras are
-        //    written in column order (rank among the row's extra columns)
-        const int32_t rb = indptr[n], L = indptr[n + 1] - rb;
-        for (int d = lane; d < D; d += 32) {
-            const int32_t c = col1[d];
-            int32_t lo = 0, hi = L;
-            while (lo < hi) {
-                const int32_t mid = (lo + hi) >> 1;
-                if (indices[rb + mid] < c) lo = mid + 1;
-                else hi = mid;
+            // 2. the distinct columns in order of first appearance, each with the
+            //    sequential sum of its entries in (element, k) order: chunks of 32
+            //    entries, equal columns grouped by match_any, the group's lowest
+            //    lane adding the group's values in lane (= entry) order to the
+            //    column's running sum -- the reference's duplicate summation order
+            int D = 0;
+            for (int base = 0; base < P; base += 32) {
+                const int p = base + lane;
+                const bool valid = p < P;
+                const int32_t c = valid ? col0[p] : -1 - lane;  // idle lanes: distinct dummies
+                const unsigned grp = __match_any_sync(0xffffffffu, c);
+                const bool leader = valid && (__ffs(grp) - 1) == lane;
+                int idx = -1;
+                if (leader)
+                    for (int d = 0; d < D; ++d)
+                        if (col1[d] == c) {
+                            idx = d;
+                            break;
+                        }
+                const unsigned newm = __ballot_sync(0xffffffffu, leader && idx < 0);
+                if (leader) {
+                    double acc_c = 0.0;
+                    if (idx < 0) idx = D + __popc(newm & lt);
+                    else acc_c = val1[idx];
+                    unsigned gm = grp;
+                    while (gm) {
+                        const int j = __ffs(gm) - 1;
+                        gm &= gm - 1;
+                        acc_c += val0[base + j];
+                        if (RECORD) eidx[base + j] = (int16_t)idx;
+                    }
+                    col1[idx] = c;
+                    val1[idx] = acc_c;
+                }
+                D += __popc(newm);
+                __syncwarp();
             }
-            const bool in_pattern = lo < L && indices[rb + lo] == c;
-            if (in_pattern) data[rb + lo] += val1[d];
-            if (RECORD && in_pattern) dd[d] = rb + lo;
-            col0[d] = in_pattern ? INT32_MAX : c;  // extra columns, for the ranks
-        }
-        __syncwarp();
-        int X = 0;
-        for (int base = 0; base < D; base += 32) {
-            const int d = base + lane;
-            const bool extra = d < D && col0[d] != INT32_MAX;
-            if (extra) {
-                const int32_t c = col0[d];
-                int r = 0;
-                for (int q = 0; q < D; ++q) r += col0[q] < c;
-                const int64_t o = 4 * (int64_t)eb + r;
-                xs_col[o] = c;
-                xs_val[o] = val1[d];
-                if (RECORD) dd[d] = -1 - r;
+            // 3. per distinct column: into the P1 slot, else an extra; extras are
+            //    written in column order (rank among the row's extra columns)
+            const int32_t rb = indptr[n], L = indptr[n + 1] - rb;
+            for (int d = lane; d < D; d += 32) {
+                const int32_t c = col1[d];
+                int32_t lo = 0, hi = L;
+                while (lo < hi) {
+                    const int32_t mid = (lo + hi) >> 1;
+                    if (indices[rb + mid] < c) lo = mid + 1;
+                    else hi = mid;
+                }
+                const bool in_pattern = lo < L && indices[rb + lo] == c;
+                if (in_pattern) data[rb + lo] += val1[d];
+                if (RECORD && in_pattern) dd[d] = rb + lo;
+                col0[d] = in_pattern ? INT32_MAX : c;  // extra columns, for the ranks
             }
-            X += __popc(__ballot_sync(0xffffffffu, extra));
-        }
-        if (lane == 0) x_cnt[n] = X;
-        __syncwarp();
-        if (RECORD) {
-            for (int p = lane; p < 4 * deg; p += 32) rec_key[4 * (int64_t)eb + p] = p < P ? dd[eidx[p]] : INT32_MAX;
             __syncwarp();
+            int X = 0;
+            for (int base = 0; base < D; base += 32) {
+                const int d = base + lane;
+                const bool extra = d < D && col0[d] != INT32_MAX;
+                if (extra) {
+                    const int32_t c = col0[d];
+                    int r = 0;
+                    for (int q = 0; q < D; ++q) r += col0[q] < c;
+                    const int64_t o = 4 * (int64_t)eb + r;
+                    xs_col[o] = c;
+                    xs_val[o] = val1[d];
+                    if (RECORD) dd[d] = -1 - r;
+                }
+                X += __popc(__ballot_sync(0xffffffffu, extra));
+            }
+            if (lane == 0) x_cnt[n] = X;
+            __syncwarp();
+            if (RECORD) {
+                for (int p = lane; p < 4 * deg; p += 32) rec_key[4 * (int64_t)eb + p] = p < P ? dd[eidx[p]] : INT32_MAX;
+                __syncwarp();
+            }
         }
     }
 }
 
-// Extras of every row, compacted in (row, column) order: one warp per row,
-// coalesced copies.
+// Extras of every row, compacted in (row, column) order: a warp looks at the
+// counts of 32 of its rows at a time and copies the non-empty ones, coalesced.
 __global__ void k_t3_compact(int64_t N, const int32_t* __restrict__ ent_off, const int32_t* __restrict__ x_ptr,
                              const int32_t* __restrict__ xs_col, const double* __restrict__ xs_val,
                              int32_t* __restrict__ x_row, int32_t* __restrict__ x_col, double* __restrict__ x_val) {
     const int lane = threadIdx.x & 31;
     const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t n_warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t n = warp; n < N; n += n_warps) {
-        const int32_t o = x_ptr[n], cnt = x_ptr[n + 1] - o;
-        const int64_t src = 4 * (int64_t)ent_off[n];
-        for (int32_t j = lane; j < cnt; j += 32) {
-            x_row[o + j] = (int32_t)n;
-            x_col[o + j] = xs_col[src + j];
-            x_val[o + j] = xs_val[src + j];
+    for (int64_t first = warp; first < N; first += 32 * n_warps) {   // warp-uniform
+        const int64_t mine = first + lane * n_warps;
+        int32_t o = 0, cnt = 0, eo = 0;
+        if (mine < N) {
+            o = x_ptr[mine];
+            cnt = x_ptr[mine + 1] - o;
+            if (cnt) eo = ent_off[mine];
+        }
+        for (unsigned todo = __ballot_sync(0xffffffffu, cnt > 0); todo; todo &= todo - 1) {
+            const int src_lane = __ffs(todo) - 1;
+            const int64_t n = first + src_lane * n_warps;
+            const int32_t on = __shfl_sync(0xffffffffu, o, src_lane), cn = __shfl_sync(0xffffffffu, cnt, src_lane);
+            const int64_t src = 4 * (int64_t)__shfl_sync(0xffffffffu, eo, src_lane);
+            for (int32_t j = lane; j < cn; j += 32) {
+                x_row[on + j] = (int32_t)n;
+                x_col[on + j] = xs_col[src + j];
+                x_val[on + j] = xs_val[src + j];
+            }
         }
     }
 }
@@ -1197,13 +1235,6 @@ __global__ void k_t3_sig_diff(int64_t E, const uint8_t* __restrict__ flag, const
     if ((threadIdx.x & 31) == 0 && c) atomicAdd(out, c);
 }
 
-__global__ void k_count_flags(const uint8_t* __restrict__ f, int64_t n, unsigned long long* out) {
-    unsigned long long c = 0;
-    GRID_STRIDE(i, n) c += (f[i] != 0);
-    c = warp_sum_u64(c);
-    if ((threadIdx.x & 31) == 0 && c) atomicAdd(out, c);
-}
-
 __global__ void k_count_nonzero(const double* __restrict__ v, int64_t n, unsigned long long* out) {
     unsigned long long c = 0;
     GRID_STRIDE(i, n) c += (v[i] != 0.0);
@@ -1213,37 +1244,81 @@ __global__ void k_count_nonzero(const double* __restrict__ v, int64_t n, unsigne
 
 // Merged row lengths / fill of (P1 data + extras), optionally dropping
 // exact zeros (scipy's CSR addition does, kernels/jacobian.py:355-357).
+// Eight lanes per row, eight entries at a time: an entry's place is the kept
+// entries of its own list before it (a ballot) plus the kept entries of the
+// other list in lower columns (eight shuffles per chunk; dropped entries
+// stand as column INT32_MAX).  One thread per row, merging serially, took
+// 187 us for the fill on the 625 k-row Jacobian.
 template <bool FILL>
-__global__ void k_merge_rows(int64_t N, const int32_t* __restrict__ indptr, const int32_t* __restrict__ indices,
-                             const double* __restrict__ data, const int32_t* __restrict__ xptr,
-                             const int32_t* __restrict__ xcol, const double* __restrict__ xval, bool drop_zeros,
-                             int32_t* __restrict__ out_ptr, int32_t* __restrict__ out_idx,
-                             double* __restrict__ out_val) {
-    GRID_STRIDE(n, N) {
-        int32_t a = indptr[n], ae = indptr[n + 1];
-        int32_t b = xptr ? xptr[n] : 0, be = xptr ? xptr[n + 1] : 0;
-        int32_t pos = FILL ? out_ptr[n] : 0;
-        int32_t cnt = 0;
-        while (a < ae || b < be) {
-            int32_t col;
-            double v;
-            if (b >= be || (a < ae && indices[a] < xcol[b])) {
-                col = indices[a];
-                v = data[a++];
-            } else {
-                col = xcol[b];
-                v = xval[b++];
+__global__ void __launch_bounds__(256)
+    k_merge_rows(int64_t N, const int32_t* __restrict__ indptr, const int32_t* __restrict__ indices,
+                 const double* __restrict__ data, const int32_t* __restrict__ xptr, const int32_t* __restrict__ xcol,
+                 const double* __restrict__ xval, bool drop_zeros, int32_t* __restrict__ out_ptr,
+                 int32_t* __restrict__ out_idx, double* __restrict__ out_val) {
+    constexpr int G = 8, RPW = 32 / G;
+    const int lane = threadIdx.x & 31, sub = lane & (G - 1), shift = lane & ~(G - 1);
+    const unsigned below = (1u << sub) - 1u;
+    const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+    const int64_t n_warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    for (int64_t base = warp * RPW; base < N; base += n_warps * RPW) {   // warp-uniform
+        const int64_t n = base + lane / G;
+        int32_t a = 0, la = 0, b = 0, lb = 0;
+        if (n < N) {
+            a = indptr[n];
+            la = indptr[n + 1] - a;
+            if (xptr) {
+                b = xptr[n];
+                lb = xptr[n + 1] - b;
             }
-            if (drop_zeros && v == 0.0) continue;
-            if (FILL) {
-                out_idx[pos + cnt] = col;
-                out_val[pos + cnt] = v;
-            }
-            ++cnt;
         }
-        if (!FILL) out_ptr[n] = cnt;
+        const int la_max = __reduce_max_sync(0xffffffffu, la), lb_max = __reduce_max_sync(0xffffffffu, lb);
+        // entry k0 + sub of a list: its column, INT32_MAX when past the end or dropped
+        auto entry = [&](const int32_t* col, const double* val, int32_t o, int32_t len, int k, double& v) {
+            if (k >= len) return INT32_MAX;
+            v = val[o + k];
+            if (drop_zeros && v == 0.0) return INT32_MAX;
+            return FILL ? col[o + k] : 0;
+        };
+        // the kept entries of the other list in columns below c
+        auto lower = [&](const int32_t* col, const double* val, int32_t o, int32_t len, int most, int32_t c) {
+            int cnt = 0;
+            for (int k0 = 0; k0 < most; k0 += G) {
+                double v;
+                const int32_t x = entry(col, val, o, len, k0 + sub, v);
+#pragma unroll
+                for (int j = 0; j < G; ++j) cnt += __shfl_sync(0xffffffffu, x, j, G) < c;
+            }
+            return cnt;
+        };
+        int kept = 0;
+        const int32_t out = FILL && n < N ? out_ptr[n] : 0;
+        auto list = [&](const int32_t* col, const double* val, int32_t o, int32_t len, int most, const int32_t* col2,
+                        const double* val2, int32_t o2, int32_t len2, int most2) {
+            int before = 0;
+            for (int k0 = 0; k0 < most; k0 += G) {
+                double v = 0.0;
+                const int32_t c = entry(col, val, o, len, k0 + sub, v);
+                const bool keep = c != INT32_MAX;
+                const unsigned m = (__ballot_sync(0xffffffffu, keep) >> shift) & ((1u << G) - 1u);
+                if (FILL) {
+                    int place = before + __popc(m & below);
+                    if (most2 > 0) place += lower(col2, val2, o2, len2, most2, c);
+                    if (keep) {
+                        out_idx[out + place] = c;
+                        out_val[out + place] = v;
+                    }
+                }
+                before += __popc(m);
+            }
+            kept += before;
+        };
+        list(indices, data, a, la, la_max, xcol, xval, b, lb, lb_max);
+        list(xcol, xval, b, lb, lb_max, indices, data, a, la, la_max);
+        if (!FILL && n < N && sub == 0) out_ptr[n] = kept;
     }
 }
+
+__global__ void k_set_i64(int64_t* __restrict__ dst, int64_t v) { *dst = v; }
 
 template <class T>
 void scan(up3d_mesh* m, const T* in, T* out, int64_t n, cudaStream_t s) {
@@ -1293,24 +1368,16 @@ void launch_row_residual(const up3d_mesh* m, double* R, cudaStream_t s) {
 // Builds Term 3 from the active flags and vectors: folds the in-pattern
 // part into `data`, keeps the extras (sorted by row, col) in the mesh
 // workspace, and returns (n_active, n_extra).  Synchronises the stream.
-// `known_active` >= 0 is the active count already known to the caller (0
-// skips everything).
+// `known_active` is the active count, known to the caller (0 skips
+// everything).
 constexpr int T3_WARPS = 4;
 static void build_term3(up3d_mesh* m, double* data, cudaStream_t s, int64_t& n_active, int64_t& n_extra,
-                        int64_t known_active = -1, const int32_t* upstream = nullptr) {
+                        int64_t known_active, const int32_t* upstream = nullptr) {
     if (!upstream) upstream = m->up32.get();
     const int64_t E = m->E, N = m->N, Z = m->nnz;
     n_extra = 0;
     m->last_extra = 0;
     m->i64_ws.alloc(8);
-    if (known_active < 0) {
-        unsigned long long* c = reinterpret_cast<unsigned long long*>(m->i64_ws.get());
-        UP3D_CUDA(cudaMemsetAsync(c, 0, sizeof(unsigned long long), s));
-        k_count_flags<<<grid_for(E, 256), 256, 0, s>>>(m->t3_flag.get(), E, c);
-        UP3D_CHECK_LAUNCH();
-        UP3D_CUDA(cudaMemcpyAsync(&known_active, c, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-        UP3D_CUDA(cudaStreamSynchronize(s));
-    }
     n_active = known_active;
     m->last_active = n_active;
     if (n_active == 0) return;
@@ -1323,10 +1390,7 @@ static void build_term3(up3d_mesh* m, double* data, cudaStream_t s, int64_t& n_a
         k_t3_sig_diff<<<grid_for(E, 256), 256, 0, s>>>(E, m->t3_flag.get(), upstream, m->t3c_flag.get(),
                                                       m->t3c_up.get(), c);
         UP3D_CHECK_LAUNCH();
-        unsigned long long diff = 1;
-        UP3D_CUDA(cudaMemcpyAsync(&diff, c, sizeof(diff), cudaMemcpyDeviceToHost, s));
-        UP3D_CUDA(cudaStreamSynchronize(s));
-        same = diff == 0;
+        same = read_back(c, s) == 0;
     }
     if (same && m->t3c_state == 2) {
         // values only: the P1 slots and extras of the recorded pattern
@@ -1357,17 +1421,19 @@ static void build_term3(up3d_mesh* m, double* data, cudaStream_t s, int64_t& n_a
         m->t3c_code_tmp.alloc(16 * E);
         m->t3c_key_tmp.alloc(16 * E);
     }
+    m->t3_row_on.alloc(N);
+    UP3D_CUDA(cudaMemsetAsync(m->t3_row_on.get(), 0, N, s));
+    k_t3_mark<<<grid_for(E, 256), 256, 0, s>>>(E, m->t3_flag.get(), m->conn.get(), m->t3_row_on.get());
+    UP3D_CHECK_LAUNCH();
     UP3D_CUDA(cudaMemsetAsync(m->extra_cnt.get() + N, 0, sizeof(int32_t), s));
     kern<<<grid_for(32 * N, T3_WARPS * 32, (int64_t)148 * 32), T3_WARPS * 32, smem, s>>>(
-        N, cap, m->ent_off.get(), m->ent.get(), m->t3_flag.get(), upstream, m->conn.get(), m->t3v.get(),
+        N, cap, m->ent_off.get(), m->ent.get(), m->t3_row_on.get(), m->t3_flag.get(), upstream, m->conn.get(),
+        m->t3v.get(),
         m->indptr.get(), m->indices.get(), data, m->x_col.get(), m->x_val.get(), m->extra_cnt.get(),
         record ? m->t3c_code_tmp.get() : nullptr, record ? m->t3c_key_tmp.get() : nullptr);
     UP3D_CHECK_LAUNCH();
     scan(m, m->extra_cnt.get(), m->x_ptr.get(), N + 1, s);
-    int32_t total = 0;
-    UP3D_CUDA(cudaMemcpyAsync(&total, m->x_ptr.get() + N, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-    UP3D_CUDA(cudaStreamSynchronize(s));
-    n_extra = total;
+    n_extra = read_back(m->x_ptr.get() + N, s);
     m->last_extra = n_extra;
     if (n_extra > 0) {
         m->x_row_c.alloc(n_extra);
@@ -1406,9 +1472,7 @@ static void build_term3(up3d_mesh* m, double* data, cudaStream_t s, int64_t& n_a
         m->cub_tmp.alloc(bytes);
         UP3D_CUDA(cub::DeviceRunLengthEncode::Encode(m->cub_tmp.get(), bytes, m->t3c_key.get(), m->t3c_key_tmp.get(),
                                                      m->t3c_cnt.get(), m->t3c_nruns.get(), n_valid, s));
-        int64_t nruns = 0;
-        UP3D_CUDA(cudaMemcpyAsync(&nruns, m->t3c_nruns.get(), sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-        UP3D_CUDA(cudaStreamSynchronize(s));
+        const int64_t nruns = read_back(m->t3c_nruns.get(), s);
         UP3D_CUDA(cudaMemsetAsync(m->t3c_cnt.get() + nruns, 0, sizeof(int32_t), s));
         scan(m, m->t3c_cnt.get(), m->t3c_seg.get(), nruns + 1, s);
         // keep the run keys (destinations) where the values kernel reads them
@@ -1428,6 +1492,28 @@ static void build_term3(up3d_mesh* m, double* data, cudaStream_t s, int64_t& n_a
     m->t3c_extra = n_extra;
 }
 
+// The merged CSR of the last Jacobian.
+static void export_merged(up3d_mesh* m, const double* data, int32_t* indptr, int32_t* indices, double* merged,
+                          cudaStream_t s) {
+    UP3D_REQUIRE(m && data && indptr && indices && merged, UP3D_ERR_ARGUMENT,
+                 "up3d_jacobian_export: null argument");
+    const bool has_x = m->last_extra > 0;
+    const int32_t* xptr = has_x ? m->x_ptr.get() : nullptr;
+    m->extra_cnt.alloc(m->N + 1);
+    int32_t* cnt = m->extra_cnt.get();
+    UP3D_CUDA(cudaMemsetAsync(cnt + m->N, 0, sizeof(int32_t), s));
+    const unsigned grid = grid_for(m->N, 32, (int64_t)m->n_sms * 64);
+    k_merge_rows<false><<<grid, 256, 0, s>>>(m->N, m->indptr.get(), m->indices.get(), data, xptr,
+                                                           m->x_col_c.get(), m->x_val_c.get(),
+                                                           m->last_drop_zeros, cnt, nullptr, nullptr);
+    UP3D_CHECK_LAUNCH();
+    scan(m, cnt, indptr, m->N + 1, s);
+    k_merge_rows<true><<<grid, 256, 0, s>>>(m->N, m->indptr.get(), m->indices.get(), data, xptr,
+                                                          m->x_col_c.get(), m->x_val_c.get(),
+                                                          m->last_drop_zeros, indptr, indices, merged);
+    UP3D_CHECK_LAUNCH();
+}
+
 static int64_t merged_nnz(up3d_mesh* m, const double* data, cudaStream_t s) {
     if (m->last_active == 0) return m->nnz;
     m->i64_ws.alloc(8);
@@ -1439,10 +1525,7 @@ static int64_t merged_nnz(up3d_mesh* m, const double* data, cudaStream_t s) {
         k_count_nonzero<<<grid_for(m->last_extra, 256), 256, 0, s>>>(m->x_val_c.get(), m->last_extra, c);
         UP3D_CHECK_LAUNCH();
     }
-    unsigned long long h = 0;
-    UP3D_CUDA(cudaMemcpyAsync(&h, c, sizeof(h), cudaMemcpyDeviceToHost, s));
-    UP3D_CUDA(cudaStreamSynchronize(s));
-    return (int64_t)h;
+    return (int64_t)read_back(c, s);
 }
 
 }  // namespace up3d
@@ -1492,22 +1575,17 @@ int up3d_jacobian(up3d_mesh* m, const double* phi, const double* rt, const doubl
         UP3D_REQUIRE(m && phi && rt && se && su && upstream && data, UP3D_ERR_ARGUMENT,
                      "up3d_jacobian: null argument");
         cudaStream_t s = S(stream);
-        m->grad_ws.alloc(3 * m->E);
-        m->q2_ws.alloc(m->E);
-        // scratch velocities (the reference recomputes grad into a fresh array,
-        // kernels/jacobian.py:328-332)
-        DBuf<double> grad, q2;
-        grad.alloc(3 * m->E);
-        q2.alloc(m->E);
-        launch_velocities(m, phi, grad.get(), q2.get(), s);
         const double inv_u2 = 1.0 / (u_inf * u_inf);
-        k_prep_jacobian<<<grid_for(m->E, 256), 256, 0, s>>>(m->B.get(), m->V.get(), grad.get(), rt, se, su, upstream,
-                                                           lim, inv_u2, m->E, m->loc.get(), m->t3v.get(),
-                                                           m->t3_flag.get(), m->up32.get());
+        m->i64_ws.alloc(8);
+        unsigned long long* count = reinterpret_cast<unsigned long long*>(m->i64_ws.get());
+        UP3D_CUDA(cudaMemsetAsync(count, 0, sizeof(unsigned long long), s));
+        k_prep_jacobian<<<grid_for(m->E, 256), 256, 0, s>>>(m->conn.get(), m->B.get(), m->V.get(), phi, rt, se, su,
+                                                           upstream, lim, inv_u2, m->E, m->loc.get(), m->t3v.get(),
+                                                           m->t3_flag.get(), m->up32.get(), count);
         UP3D_CHECK_LAUNCH();
         launch_row_gather(m, nullptr, data, s);
         int64_t na = 0, nx = 0;
-        build_term3(m, data, s, na, nx);
+        build_term3(m, data, s, na, nx, read_back(reinterpret_cast<const int64_t*>(count), s));
         m->last_drop_zeros = na > 0;
         if (n_active) *n_active = na;
         if (n_extra) *n_extra = nx;
@@ -1523,24 +1601,15 @@ int up3d_jacobian_data(up3d_mesh* m, const double* phi, const double* rt, const 
 
 int up3d_jacobian_export(up3d_mesh* m, const double* data, int32_t* indptr, int32_t* indices, double* merged,
                          up3d_stream stream) {
+    return guarded([&] { export_merged(m, data, indptr, indices, merged, S(stream)); });
+}
+
+int up3d_jacobian_merge(up3d_mesh* m, const double* data, int32_t* indptr, int32_t* indices, double* merged,
+                        int64_t* newton_nnz, up3d_stream stream) {
     return guarded([&] {
-        UP3D_REQUIRE(m && data && indptr && indices && merged, UP3D_ERR_ARGUMENT,
-                     "up3d_jacobian_export: null argument");
-        cudaStream_t s = S(stream);
-        const bool has_x = m->last_extra > 0;
-        const int32_t* xptr = has_x ? m->x_ptr.get() : nullptr;
-        m->extra_cnt.alloc(m->N + 1);
-        int32_t* cnt = m->extra_cnt.get();
-        UP3D_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int32_t) * (m->N + 1), s));
-        k_merge_rows<false><<<grid_for(m->N, 256), 256, 0, s>>>(m->N, m->indptr.get(), m->indices.get(), data, xptr,
-                                                               m->x_col_c.get(), m->x_val_c.get(),
-                                                               m->last_drop_zeros, cnt, nullptr, nullptr);
-        UP3D_CHECK_LAUNCH();
-        scan(m, cnt, indptr, m->N + 1, s);
-        k_merge_rows<true><<<grid_for(m->N, 256), 256, 0, s>>>(m->N, m->indptr.get(), m->indices.get(), data, xptr,
-                                                              m->x_col_c.get(), m->x_val_c.get(),
-                                                              m->last_drop_zeros, indptr, indices, merged);
-        UP3D_CHECK_LAUNCH();
+        UP3D_REQUIRE(newton_nnz, UP3D_ERR_ARGUMENT, "up3d_jacobian_merge: null argument");
+        export_merged(m, data, indptr, indices, merged, S(stream));
+        *newton_nnz = read_back(indptr + m->N, S(stream));
     });
 }
 
@@ -1753,17 +1822,15 @@ static void fused_evaluate(up3d_mesh* m, const double* phi, const Flow& F, doubl
     if (jac) {
         // the element sweep counted the active elements: Term 3 is
         // built only when there are any (flags already written)
-        int64_t known = 0;
-        UP3D_CUDA(cudaMemcpyAsync(&known, &mo->n_term3_active, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-        UP3D_CUDA(cudaStreamSynchronize(s));
+        const int64_t known = read_back(&mo->n_term3_active, s);
         int64_t na = 0, nx = 0;
         prof_begin(PROF_TERM3, s);
         build_term3(m, data, s, na, nx, known, up_dst);
         prof_end(PROF_TERM3, s, 0);
         m->last_drop_zeros = na > 0;
         if (nx) {
-            UP3D_CUDA(cudaMemcpyAsync(&mo->n_term3_extra, &nx, sizeof(int64_t), cudaMemcpyHostToDevice, s));
-            UP3D_CUDA(cudaStreamSynchronize(s));
+            k_set_i64<<<1, 1, 0, s>>>(&mo->n_term3_extra, nx);
+            UP3D_CHECK_LAUNCH();
         }
     }
 }
@@ -1963,11 +2030,9 @@ int up3d_residual_jacobian_batched(up3d_mesh* m, const double* phi, int n_cases,
             UP3D_CUDA(cudaMemsetAsync(bad, 0, sizeof(int), s));
             k_check_cases<<<grid_for(m->E, 256), 256, 0, s>>>(case_of, m->E, n_cases, bad);
             UP3D_CHECK_LAUNCH();
-            int hbad = 0;
             UP3D_CUDA(cudaMemcpyAsync(m->flows_ws.get(), host.data(), sizeof(Flow) * n_cases,
                                       cudaMemcpyHostToDevice, s));
-            UP3D_CUDA(cudaMemcpyAsync(&hbad, bad, sizeof(int), cudaMemcpyDeviceToHost, s));
-            UP3D_CUDA(cudaStreamSynchronize(s));
+            const int hbad = read_back(bad, s);   // also: `host` may go out of scope
             m->batch_cases = 0;
             UP3D_REQUIRE(!hbad, UP3D_ERR_VALUE, "up3d_residual_jacobian_batched: case index out of range");
             m->batch_cases = n_cases;

@@ -122,6 +122,21 @@ struct DBuf {
     T* get() const { return p; }
 };
 
+// One scalar from the device (synchronises the stream), through a word of
+// page-locked memory of the calling thread: into pageable memory the copy is
+// staged by the driver.  Without such memory the plain copy is made.
+int64_t* host_word();
+template <class T>
+T read_back(const T* dev, cudaStream_t s) {
+    static_assert(sizeof(T) <= sizeof(int64_t), "a scalar");
+    int64_t plain = 0;
+    int64_t* w = host_word();
+    if (!w) w = &plain;
+    UP3D_CUDA(cudaMemcpyAsync(w, dev, sizeof(T), cudaMemcpyDeviceToHost, s));
+    UP3D_CUDA(cudaStreamSynchronize(s));
+    return *reinterpret_cast<T*>(w);
+}
+
 // ------------------------------------------------------------ mesh handle
 
 // Local element data written by the element sweeps and gathered by rows:
@@ -197,6 +212,7 @@ struct up3d_mesh {
     up3d::DBuf<unsigned char> cub_tmp;
     // Term 3 (grown on demand)
     up3d::DBuf<uint8_t> t3_flag;       // (E) active elements
+    up3d::DBuf<uint8_t> t3_row_on;     // (N) rows with an incident active element
     up3d::DBuf<int32_t> x_col;         // (16E) per-row extras scratch at 4 ent_off[n]
     up3d::DBuf<double> x_val;
     up3d::DBuf<int32_t> x_ptr;         // (N+1) extras row pointer

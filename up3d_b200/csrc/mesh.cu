@@ -335,6 +335,24 @@ int32_t device_max(up3d_mesh* m, const int32_t* in, int64_t n, cudaStream_t s) {
 
 }  // namespace
 
+// The thread's page-locked word (portable: any device's copies may target
+// it); given back when the thread ends.
+int64_t* host_word() {
+    struct Word {
+        int64_t* p = nullptr;
+        Word() {
+            void* v = nullptr;
+            if (cudaHostAlloc(&v, sizeof(int64_t), cudaHostAllocPortable) == cudaSuccess) p = static_cast<int64_t*>(v);
+            else cudaGetLastError();
+        }
+        ~Word() {
+            if (p) cudaFreeHost(p);
+        }
+    };
+    static thread_local Word w;
+    return w.p;
+}
+
 void set_error(const std::string& msg) { g_last_error = msg; }
 int fail(int status, const std::string& msg) {
     g_last_error = msg;

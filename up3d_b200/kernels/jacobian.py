@@ -157,20 +157,26 @@ class PicardOperator:
         d_up = L.to_device(upstream, t.int64)
         d_lim = None if lim_mask is None else L.to_device(lim_mask, t.uint8)
         data = t.empty(self._mesh.nnz, dtype=t.float64, device="cuda")
-        na, nx, nnz = ctypes.c_int64(), ctypes.c_int64(), ctypes.c_int64()
+        na, nx = ctypes.c_int64(), ctypes.c_int64()
         L.call("up3d_jacobian", self._mesh.handle, d_phi.data_ptr(), d_rt.data_ptr(), d_se.data_ptr(),
                d_su.data_ptr(), d_up.data_ptr(), float(u_inf), L.ptr(d_lim), data.data_ptr(),
-               ctypes.byref(na), ctypes.byref(nx), ctypes.byref(nnz), L.stream_ptr())
+               ctypes.byref(na), ctypes.byref(nx), None, L.stream_ptr())
         self.n_term3_active = int(na.value)
         self.n_term3_extra = int(nx.value)
-        self.newton_nnz = int(nnz.value)
         if self.n_term3_active == 0:
+            self.newton_nnz = self._mesh.nnz
             return self._csr_result(self._mesh.indptr, self._mesh.indices, data, host)
         indptr = t.empty(self.n_nodes + 1, dtype=t.int32, device="cuda")
-        indices = t.empty(self.newton_nnz, dtype=t.int32, device="cuda")
-        merged = t.empty(self.newton_nnz, dtype=t.float64, device="cuda")
-        L.call("up3d_jacobian_export", self._mesh.handle, data.data_ptr(), indptr.data_ptr(),
-               indices.data_ptr(), merged.data_ptr(), L.stream_ptr())
+        # the merged matrix drops exact zeros: room for every entry, cut to
+        # what there is
+        most = self._mesh.nnz + self.n_term3_extra
+        indices = t.empty(most, dtype=t.int32, device="cuda")
+        merged = t.empty(most, dtype=t.float64, device="cuda")
+        nnz = ctypes.c_int64()
+        L.call("up3d_jacobian_merge", self._mesh.handle, data.data_ptr(), indptr.data_ptr(),
+               indices.data_ptr(), merged.data_ptr(), ctypes.byref(nnz), L.stream_ptr())
+        self.newton_nnz = int(nnz.value)
+        indices, merged = indices[:self.newton_nnz], merged[:self.newton_nnz]
         return self._csr_result(indptr, indices, merged, host)
 
     def assemble_residual(self, phi, rho_tilde=None):

@@ -81,13 +81,17 @@ class ResidualJacobian:
         if mon["n_term3_active"] == 0:
             return DeviceCSR(self.mesh.indptr, self.mesh.indices, self.data,
                              (self.mesh.n_nodes, self.mesh.n_nodes))
-        if newton_nnz is None:
-            newton_nnz = self.newton_nnz()
+        # the merged matrix drops exact zeros: room for every entry, cut to
+        # what there is
+        most = self.mesh.nnz + mon["n_term3_extra"] if newton_nnz is None else newton_nnz
         indptr = t.empty(self.mesh.n_nodes + 1, dtype=t.int32, device="cuda")
-        indices = t.empty(newton_nnz, dtype=t.int32, device="cuda")
-        data = t.empty(newton_nnz, dtype=t.float64, device="cuda")
-        L.call("up3d_jacobian_export", self.mesh.handle, self.data.data_ptr(), indptr.data_ptr(),
-               indices.data_ptr(), data.data_ptr(), L.stream_ptr())
+        indices = t.empty(most, dtype=t.int32, device="cuda")
+        data = t.empty(most, dtype=t.float64, device="cuda")
+        nnz = ctypes.c_int64()
+        L.call("up3d_jacobian_merge", self.mesh.handle, self.data.data_ptr(), indptr.data_ptr(),
+               indices.data_ptr(), data.data_ptr(), ctypes.byref(nnz), L.stream_ptr())
+        if newton_nnz is None:
+            indices, data = indices[:nnz.value], data[:nnz.value]
         return DeviceCSR(indptr, indices, data, (self.mesh.n_nodes, self.mesh.n_nodes))
 
     def evaluate_host(self, phi_host, flow: FlowParams, R_host, J_host) -> None:
