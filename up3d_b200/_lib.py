@@ -14,6 +14,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import sys
 from pathlib import Path
 
 import numpy as np
@@ -251,15 +252,25 @@ def torch():
     return _t
 
 
+_cuda = None   # torch, once a CUDA device was found (a device that was there stays)
+
+
 def require_cuda():
-    t = torch()
-    if not t.cuda.is_available():
-        raise RuntimeError("up3d_b200 needs a CUDA device; none is visible (no CPU fallback)")
-    return t
+    global _cuda
+    if _cuda is None:
+        t = torch()
+        if not t.cuda.is_available():
+            raise RuntimeError("up3d_b200 needs a CUDA device; none is visible (no CPU fallback)")
+        _cuda = t
+    return _cuda
 
 
 def stream_ptr():
-    return torch().cuda.current_stream().cuda_stream
+    t = torch()
+    raw = getattr(t._C, "_cuda_getCurrentRawStream", None)   # without building a Stream object
+    if raw is None:
+        return t.cuda.current_stream().cuda_stream
+    return raw(t.cuda.current_device())
 
 
 def ptr(t) -> int | None:
@@ -274,21 +285,21 @@ def ptr(t) -> int | None:
 
 
 def is_torch(x) -> bool:
-    try:
-        import torch as _t
-        return isinstance(x, _t.Tensor)
-    except ImportError:
-        return False
+    t = sys.modules.get("torch")   # a tensor exists only where torch was imported
+    return t is not None and isinstance(x, t.Tensor)
 
 
 def to_device(x, dtype, device=None):
     """numpy / torch -> contiguous CUDA tensor of `dtype` (no copy when it
     already is one)."""
     t = require_cuda()
-    dev = device if device is not None else t.device("cuda", t.cuda.current_device())
     if is_torch(x):
-        y = x.to(device=dev, dtype=dtype)
-        return y.contiguous()
+        if (device is None and x.dtype == dtype and x.is_cuda and x.is_contiguous()
+                and x.get_device() == t.cuda.current_device()):
+            return x
+        dev = device if device is not None else t.device("cuda", t.cuda.current_device())
+        return x.to(device=dev, dtype=dtype).contiguous()
+    dev = device if device is not None else t.device("cuda", t.cuda.current_device())
     arr = np.ascontiguousarray(x)
     return t.from_numpy(arr).to(device=dev, dtype=dtype, non_blocking=False).contiguous()
 
