@@ -35,18 +35,10 @@ namespace {
 
 constexpr int RG_WARPS = 8;   // warps per block of the row gather
 
-// Minimum resident blocks per SM (launch bounds), tuned at 3.6M tets on
-// B200: the Jacobian sweep runs fastest at 2 (128 registers, no spills).
+// Minimum resident blocks per SM of the row gather (launch bounds).
 #ifndef UP3D_ROW_MINB
 #define UP3D_ROW_MINB 8
 #endif
-#ifndef UP3D_ELEM_MINB
-#define UP3D_ELEM_MINB 3
-#endif
-#ifndef UP3D_ELEM_MINB_JAC
-#define UP3D_ELEM_MINB_JAC 2
-#endif
-
 // ------------------------------------------------------------ element math
 
 __device__ __forceinline__ void gB_of(const double g[3], const double* __restrict__ b, double gB[4]) {
@@ -69,9 +61,11 @@ __device__ __forceinline__ double jij(const double* b, const double gB[4], doubl
 }
 
 // Writes [R_0, J_00, ..., R_3, J_33, J_01, J_02, J_03, J_12, J_13, J_23].
-__device__ __forceinline__ void store_local(double* __restrict__ loc, int64_t e, const double* b,
-                                            const double gB[4], double w1, double w2, bool with_r) {
-    double2* p = reinterpret_cast<double2*>(loc + (size_t)LOC_STRIDE * e);
+__device__ __forceinline__ double2* loc_of(double* __restrict__ loc, int64_t e) {
+    return reinterpret_cast<double2*>(loc + (size_t)LOC_STRIDE * e);
+}
+__device__ __forceinline__ void store_local(double2* __restrict__ p, const double* b, const double gB[4], double w1,
+                                            double w2, bool with_r) {
 #pragma unroll
     for (int i = 0; i < 4; ++i)
         p[i] = make_double2(with_r ? w1 * gB[i] : 0.0, jij(b, gB, w1, w2, i, i));
@@ -275,7 +269,7 @@ __global__ void k_prep_matrix(const double* __restrict__ B, const double* __rest
         double b[12];
         load_B(B, e, b);
         const double z[4] = {0.0, 0.0, 0.0, 0.0};
-        store_local(loc, e, b, z, (rt ? rt[e] : 1.0) * V[e], 0.0, false);
+        store_local(loc_of(loc, e), b, z, (rt ? rt[e] : 1.0) * V[e], 0.0, false);
     }
 }
 
@@ -318,7 +312,7 @@ __global__ void k_prep_jacobian(const int4* __restrict__ conn, const double* __r
         }
         t3flag[e] = active ? 1 : 0;
         up32[e] = (int32_t)u;
-        store_local(loc, e, b, gB, rt[e] * Ve, w2, false);
+        store_local(loc_of(loc, e), b, gB, rt[e] * Ve, w2, false);
     }
     count = warp_sum_u64(count);
     if ((threadIdx.x & 31) == 0 && count) atomicAdd(n_active, count);
@@ -326,9 +320,9 @@ __global__ void k_prep_jacobian(const int4* __restrict__ conn, const double* __r
 
 // ------------------------------------------------------------ fused sweep
 
-struct MonAcc {
+struct MonAcc {   // one thread's counts: below 2^31 with the elements
     double nu_max = 0.0;
-    unsigned long long sup = 0, flo = 0, lim = 0, act = 0;
+    unsigned sup = 0, flo = 0, lim = 0, act = 0;
 };
 
 __device__ __forceinline__ void flush(MonAcc a, up3d_monitors* mon) {
@@ -344,6 +338,26 @@ __device__ __forceinline__ void flush(MonAcc a, up3d_monitors* mon) {
     }
 }
 
+// A warp's 32 consecutive records leave through a slab of shared memory as
+// one bulk store of contiguous bytes: a lane storing its own 112 bytes puts a
+// line per lane through the load/store unit (3.6 M tets: 275 -> 265 us).
+__device__ __forceinline__ void slab_free(int lane) {  // the last store has read the slab
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+    __syncwarp();
+}
+__device__ __forceinline__ void slab_store(double* dst, const double2* src, unsigned bytes, int lane) {
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncwarp();
+    if (lane == 0) {
+        asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst),
+                     "r"((unsigned)__cvta_generic_to_shared(src)), "r"(bytes)
+                     : "memory");
+        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+    }
+}
+__device__ __forceinline__ void slab_done(int lane) {  // written, before the block ends
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+}
 // eval_residual + assemble_coupled, per element (pyfp3d/solve/newton.py:
 // 345-372, :435-452): gradient, limiter, density, upstream walk (or the
 // frozen selection), the upstream element's state recomputed in place, the
@@ -356,137 +370,168 @@ __device__ __forceinline__ void flush(MonAcc a, up3d_monitors* mon) {
 // taking the flow of its case, flows[case_of[e]] (an index outside
 // [0, n_cases) reads case 0: the host validates the indices, and a table
 // reused without validation can never be read out of bounds).
+// AIR: gamma == 1.4 in every flow (no pow, and the registers it takes).
 // NT threads per block, MB resident blocks per SM that the register
 // allocation must allow.
-template <bool FROZEN, bool JAC, bool BATCH, int NT, int MB>
+// What bounds it: the latency of the walk's dependent loads at the few warps
+// that its registers leave (3.6 M tets, 20 warps per SM: issue slots 30 %,
+// FP64 pipe 32 %, load/store wavefronts 68 % busy), so registers and
+// wavefronts are what pays: 304 us with int64 ids and pow, 287 with neither,
+// 275 without the switch of subcritical pairs, 264 with the records stored in
+// bulk; residual only 238 -> 214.  14.7 M tets: 1187 -> 1092 us.  Tried and
+// slower: the walk as a kernel of its own (297), B_e kept in the slab instead
+// of formed again (259 against 256, residual only 230 against 214), the next
+// tile's records prefetched into L2 (256 at 3.6 M, but 1240 at 14.7 M).
+template <bool FROZEN, bool JAC, bool BATCH, bool AIR, int NT, int MB>
 __global__ void __launch_bounds__(NT, MB)
-    k_fused_elem(const int4* __restrict__ conn, const int4* __restrict__ fn, const double* __restrict__ disp, const double4* __restrict__ X,
-                 const double* __restrict__ phi, Flow F0, double u2, const int64_t* __restrict__ up_fz,
+    k_fused_elem(const int4* __restrict__ conn, const int4* __restrict__ fn, const double* __restrict__ disp,
+                 const double4* __restrict__ X, const double* __restrict__ phi, Flow F0, double u2,
+                 const int64_t* __restrict__ up_fz,
                  const int8_t* __restrict__ br_fz, int64_t E, double* __restrict__ loc, double* __restrict__ res,
                  double* __restrict__ t3v, uint8_t* __restrict__ t3flag, int32_t* __restrict__ up_out,
                  double* __restrict__ rt_out, up3d_monitors* mon, const Flow* __restrict__ flows,
                  const int32_t* __restrict__ case_of, int n_cases, int8_t* __restrict__ br_out) {
+    constexpr int LOC2 = LOC_STRIDE / 2;
+    __shared__ double2 slab[JAC ? NT * LOC2 : 1];  // the local records of each warp's 32 elements
+    const int lane = threadIdx.x & 31;
+    double2* const mine = slab + (JAC ? (threadIdx.x - lane) * LOC2 : 0);
     MonAcc acc;
-    // tiles of blockDim elements, block-strided over the grid
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < E; base += stride) {
-        const int64_t e = base + threadIdx.x;
-        if (e >= E) continue;
-        int ci = 0;
-        if (BATCH) {
-            ci = case_of[e];
-            ci = (unsigned)ci < (unsigned)n_cases ? ci : 0;
-        }
-        const Flow& F = BATCH ? flows[ci] : F0;
-        // only grad phi_e stays live through the walk; the element's own
-        // state and gB_j = grad . B_j are formed after it (B_e recomputed
-        // from the coordinates, L1/L2 hits)
-        const int4 ce = conn[e];
-        double g[3], Ve;
-        {
-            double bb[12];
-            geom_B(X, ce, bb, Ve);
-            grad_from_B(ce, bb, phi, g);
-        }
-        // frozen (upstream, branch) per element; a negative branch keeps the
-        // element live (several cases in one mesh, frozen one by one)
-        const int brf = FROZEN ? (int)br_fz[e] : -1;
-        const bool frz = FROZEN && brf >= 0;
-        int64_t u = frz ? safe_up(up_fz[e], e, E) : upstream_walk(fn, disp, X, conn, e, E, g);
-        double q2n = __ddiv_rn(dot3r(g[0], g[1], g[2], g[0], g[1], g[2]), u2);
-        double q2l = q2n < F.q2cap ? q2n : F.q2cap;
-        bool lim_e = q2l == q2n;
-        double rho_e, drho_e;
-        rho_drho(q2l, F, rho_e, drho_e);
-        // upstream state, and its Term-3 factors grad_u . B_u,k
-        double q2lu = q2l, rho_u = rho_e;
-        bool lim_u = lim_e;
-        if (u != e) {
-            double gu[3];
+    // tiles of NT elements, block-strided over the grid; element ids in 32
+    // bits (E < 2^29), which with the counts costs 12 registers less
+    const int n = (int)E;
+    for (int e0 = blockIdx.x * NT + (threadIdx.x - lane); e0 < n; e0 += gridDim.x * NT) {
+        if (JAC) slab_free(lane);
+        const int e = e0 + lane;
+        if (e < n) {
+            int ci = 0;
+            if (BATCH) {
+                ci = case_of[e];
+                ci = (unsigned)ci < (unsigned)n_cases ? ci : 0;
+            }
+            const Flow& F = BATCH ? flows[ci] : F0;
+            // only grad phi_e stays live through the walk; the element's own
+            // state and gB_j = grad . B_j are formed after it (B_e recomputed
+            // from the coordinates, L1/L2 hits)
+            const int4 ce = conn[e];
+            double g[3], Ve;
             {
-                const int4 cu = conn[u];
-                double bu[12], vu;
-                geom_B(X, cu, bu, vu);
-                grad_from_B(cu, bu, phi, gu);
+                double bb[12];
+                geom_B(X, ce, bb, Ve);
+                grad_from_B(ce, bb, phi, g);
             }
-            double q2nu = __ddiv_rn(dot3r(gu[0], gu[1], gu[2], gu[0], gu[1], gu[2]), u2);
-            q2lu = q2nu < F.q2cap ? q2nu : F.q2cap;
-            lim_u = q2lu == q2nu;
-            rho_u = rho_of(q2lu, F);
-        }
-        acc.lim += !lim_e;
-
-        double nu, rt, s_e = 0.0, s_u = 0.0;
-        if (frz) {
-            const int br = brf;
-            if (br_out) br_out[e] = (int8_t)br;
-            if (br == 3) {
-                nu = 0.0;
-                rt = F.floor_;
-                acc.flo += 1;
-            } else if (br == 0) {
-                nu = 0.0;
-                rt = rho_e;
-            } else {
-                nu = switch_of(mach2_of(br == 1 ? q2l : q2lu, F), F);
-                rt = rho_e - nu * (rho_e - rho_u);
-            }
-            if (JAC) frozen_sensitivities(br, q2l, rho_e, q2lu, rho_u, F, s_e, s_u);
-        } else {
-            const double nu_e = switch_of(mach2_of(q2l, F), F), nu_u = switch_of(mach2_of(q2lu, F), F);
-            nu = fmax(nu_e, nu_u);
-            rt = rho_e - nu * (rho_e - rho_u);
-            // the branch this live evaluation took (classify_upwind_branches,
-            // kernels/upwind.py:504-541)
-            if (br_out)
-                br_out[e] = (int8_t)(u == e ? (rho_e <= F.floor_ ? 3 : 0)
-                                            : (rt <= F.floor_ ? 3 : (nu == 0.0 ? 0 : (nu_e >= nu_u ? 1 : 2))));
-            rt = rt > F.floor_ ? rt : F.floor_;
-            acc.flo += (rt == F.floor_);
-            if (JAC) live_sensitivities(q2l, rho_e, q2lu, rho_u, u == e, F, s_e, s_u);
-        }
-        acc.nu_max = fmax(acc.nu_max, nu);
-        acc.sup += (nu > 0.0);
-
-        const double w1 = rt * Ve;
-        // B_e again (recomputed), held in registers from here
-        double b[12];
-        {
-            double vtmp;
-            geom_B(X, ce, b, vtmp);
-        }
-        double gB[4];
-        gB_of(g, b, gB);
-        if (JAC) {
-            s_e = s_e * (lim_e ? 1.0 : 0.0);
-            s_u = s_u * (lim_u ? 1.0 : 0.0);
-            const double w2 = 2.0 * F.inv_u2 * s_e * Ve;
-            const double w3 = 2.0 * F.inv_u2 * s_u * Ve;
-            const bool active = s_u != 0.0;
-            if (active) {
-                // Term-3 factors grad_u . B_u,k, recomputed for the (few)
-                // active elements only
-                double f[4] = {gB[0], gB[1], gB[2], gB[3]};
-                if (u != e) {
-                    double gu[3], bu[12];
-                    int4 cu;
-                    cu = conn[u];
-                    double vu;
+            // frozen (upstream, branch) per element; a negative branch keeps the
+            // element live (several cases in one mesh, frozen one by one)
+            const int brf = FROZEN ? (int)br_fz[e] : -1;
+            const bool frz = FROZEN && brf >= 0;
+            const int u = frz ? (int)safe_up(up_fz[e], e, E) : upstream_walk(fn, disp, X, ce, e, n, g);
+            double q2n = __ddiv_rn(dot3r(g[0], g[1], g[2], g[0], g[1], g[2]), u2);
+            double q2l = q2n < F.q2cap ? q2n : F.q2cap;
+            bool lim_e = q2l == q2n;
+            double rho_e, drho_e;
+            rho_drho<AIR>(q2l, F, rho_e, drho_e);
+            // upstream state, and its Term-3 factors grad_u . B_u,k
+            double q2lu = q2l, rho_u = rho_e;
+            bool lim_u = lim_e;
+            if (u != e) {
+                double gu[3];
+                {
+                    const int4 cu = conn[u];
+                    double bu[12], vu;
                     geom_B(X, cu, bu, vu);
                     grad_from_B(cu, bu, phi, gu);
-                    gB_of(gu, bu, f);
                 }
-                store_t3(t3v, e, w3, gB, f);
-                acc.act += 1;
+                double q2nu = __ddiv_rn(dot3r(gu[0], gu[1], gu[2], gu[0], gu[1], gu[2]), u2);
+                q2lu = q2nu < F.q2cap ? q2nu : F.q2cap;
+                lim_u = q2lu == q2nu;
             }
-            t3flag[e] = active ? 1 : 0;
-            store_local(loc, e, b, gB, w1, w2, true);
-        } else {
-            store_res(res, e, gB, w1);
+            // both elements surely subcritical: the switch is 0, no upstream
+            // density, Mach number or switch enters (four divisions and a root)
+            const bool sub = !frz && q2l <= F.q2sub && q2lu <= F.q2sub;
+            if (u != e && !sub) rho_u = rho_of<AIR>(q2lu, F);
+            acc.lim += !lim_e;
+
+            double nu, rt, s_e = 0.0, s_u = 0.0;
+            if (frz) {
+                const int br = brf;
+                if (br_out) br_out[e] = (int8_t)br;
+                if (br == 3) {
+                    nu = 0.0;
+                    rt = F.floor_;
+                    acc.flo += 1;
+                } else if (br == 0) {
+                    nu = 0.0;
+                    rt = rho_e;
+                } else {
+                    nu = switch_of(mach2_of(br == 1 ? q2l : q2lu, F), F);
+                    rt = rho_e - nu * (rho_e - rho_u);
+                }
+                if (JAC) frozen_sensitivities<AIR>(br, q2l, rho_e, q2lu, rho_u, F, s_e, s_u);
+            } else if (sub) {
+                nu = 0.0;
+                const bool floored = rho_e <= F.floor_;
+                rt = rho_e > F.floor_ ? rho_e : F.floor_;
+                acc.flo += (rt == F.floor_);
+                if (br_out) br_out[e] = floored ? 3 : 0;
+                if (JAC) s_e = floored ? 0.0 : drho_e;
+            } else {
+                const double nu_e = switch_of(mach2_of(q2l, F), F), nu_u = switch_of(mach2_of(q2lu, F), F);
+                nu = fmax(nu_e, nu_u);
+                rt = rho_e - nu * (rho_e - rho_u);
+                // the branch this live evaluation took (classify_upwind_branches,
+                // kernels/upwind.py:504-541)
+                if (br_out)
+                    br_out[e] = (int8_t)(u == e ? (rho_e <= F.floor_ ? 3 : 0)
+                                                : (rt <= F.floor_ ? 3 : (nu == 0.0 ? 0 : (nu_e >= nu_u ? 1 : 2))));
+                rt = rt > F.floor_ ? rt : F.floor_;
+                acc.flo += (rt == F.floor_);
+                if (JAC) live_sensitivities<AIR>(q2l, rho_e, q2lu, rho_u, u == e, F, s_e, s_u);
+            }
+            acc.nu_max = fmax(acc.nu_max, nu);
+            acc.sup += (nu > 0.0);
+
+            const double w1 = rt * Ve;
+            // B_e again (recomputed), held in registers from here
+            double b[12];
+            {
+                double vtmp;
+                geom_B(X, ce, b, vtmp);
+            }
+            double gB[4];
+            gB_of(g, b, gB);
+            if (JAC) {
+                s_e = s_e * (lim_e ? 1.0 : 0.0);
+                s_u = s_u * (lim_u ? 1.0 : 0.0);
+                const double w2 = 2.0 * F.inv_u2 * s_e * Ve;
+                const double w3 = 2.0 * F.inv_u2 * s_u * Ve;
+                const bool active = s_u != 0.0;
+                if (active) {
+                    // Term-3 factors grad_u . B_u,k, recomputed for the (few)
+                    // active elements only
+                    double f[4] = {gB[0], gB[1], gB[2], gB[3]};
+                    if (u != e) {
+                        double gu[3], bu[12];
+                        int4 cu;
+                        cu = conn[u];
+                        double vu;
+                        geom_B(X, cu, bu, vu);
+                        grad_from_B(cu, bu, phi, gu);
+                        gB_of(gu, bu, f);
+                    }
+                    store_t3(t3v, e, w3, gB, f);
+                    acc.act += 1;
+                }
+                t3flag[e] = active ? 1 : 0;
+                store_local(mine + LOC2 * lane, b, gB, w1, w2, true);
+            } else {
+                store_res(res, e, gB, w1);
+            }
+            up_out[e] = (int32_t)u;
+            if (rt_out) rt_out[e] = rt;
         }
-        up_out[e] = (int32_t)u;
-        if (rt_out) rt_out[e] = rt;
+        if (JAC)
+            slab_store(loc + (size_t)LOC_STRIDE * e0, mine, min(32, n - e0) * LOC_STRIDE * sizeof(double), lane);
     }
+    if (JAC) slab_done(lane);
     flush(acc, mon);
 }
 
@@ -1636,9 +1681,9 @@ __global__ void k_check_cases(const int32_t* __restrict__ case_of, int64_t E, in
 // wave (SMs x the kernel's occupancy) looping over block-sized tiles; the
 // Jacobian sweep compiled for 512 (256 x 2), 640 (128 x 5) or 768 (256 x 3)
 // resident threads per SM.
-template <bool FR, bool JA, bool BA, int NT, int MB, class... A>
+template <bool FR, bool JA, bool BA, bool AIR, int NT, int MB, class... A>
 static void launch_sweep_mb(const up3d_mesh* m, cudaStream_t s, A... args) {
-    auto kern = k_fused_elem<FR, JA, BA, NT, MB>;
+    auto kern = k_fused_elem<FR, JA, BA, AIR, NT, MB>;
     unsigned grid;
     if (m->tune.elem_persistent) {
         static int occ = 0;  // same for every device of the process (one architecture)
@@ -1655,14 +1700,24 @@ static void launch_sweep_mb(const up3d_mesh* m, cudaStream_t s, A... args) {
     UP3D_CHECK_LAUNCH();
 }
 
-template <bool FR, bool JA, bool BA, class... A>
-static void launch_sweep(const up3d_mesh* m, cudaStream_t s, A... args) {
-    if (!JA) return launch_sweep_mb<FR, JA, BA, 256, UP3D_ELEM_MINB>(m, s, args...);
+template <bool FR, bool JA, bool BA, bool AIR, class... A>
+static void launch_sweep_air(const up3d_mesh* m, cudaStream_t s, A... args) {
+    // residual only: air fits 72 registers without a spill; with the walk 28
+    // warps per SM are fastest (3.6 M tets: 24 warps 218 us, 28 warps 211 us),
+    // without it 24 (0.43 M: 21.9 and 22.5 us)
+    if (!JA) return !AIR ? launch_sweep_mb<FR, JA, BA, AIR, 256, 3>(m, s, args...)
+                         : launch_sweep_mb<FR, JA, BA, AIR, 128, FR ? 6 : 7>(m, s, args...);
     switch (m->tune.elem_threads_per_sm) {
-        case 640: launch_sweep_mb<FR, JA, BA, 128, 5>(m, s, args...); break;
-        case 768: launch_sweep_mb<FR, JA, BA, 256, 3>(m, s, args...); break;
-        default: launch_sweep_mb<FR, JA, BA, 256, UP3D_ELEM_MINB_JAC>(m, s, args...); break;
+        case 640: launch_sweep_mb<FR, JA, BA, AIR, 128, 5>(m, s, args...); break;
+        case 768: launch_sweep_mb<FR, JA, BA, AIR, 128, 6>(m, s, args...); break;
+        default: launch_sweep_mb<FR, JA, BA, AIR, 256, 2>(m, s, args...); break;
     }
+}
+
+template <bool FR, bool JA, bool BA, class... A>
+static void launch_sweep(const up3d_mesh* m, bool air, cudaStream_t s, A... args) {
+    if (air) launch_sweep_air<FR, JA, BA, true>(m, s, args...);
+    else launch_sweep_air<FR, JA, BA, false>(m, s, args...);
 }
 
 // One launch of the tiled evaluation over every tile (a persistent grid of
@@ -1782,7 +1837,7 @@ static void fused_evaluate(up3d_mesh* m, const double* phi, const Flow& F, doubl
                            int8_t* br_out = nullptr, int n_cases = 0) {
     up3d_monitors* mo = mon ? mon : m->mon_ws.get();
     UP3D_CUDA(cudaMemsetAsync(mo, 0, sizeof(up3d_monitors), s));
-    const bool jac = data != nullptr;
+    const bool jac = data != nullptr, air = flows_d ? m->batch_air : F.air;
     // the walk's result goes straight to the caller's buffer when there is
     // one (Term 3 reads it from there), else to the mesh workspace
     int32_t* up_dst = up_out ? up_out : m->up32.get();
@@ -1797,19 +1852,19 @@ static void fused_evaluate(up3d_mesh* m, const double* phi, const Flow& F, doubl
     prof_begin(PROF_ELEM, s);
     if (flows_d) {
         if (up_fz) {
-            if (jac) launch_sweep<true, true, true>(m, s, FUSED_ARGS);
-            else launch_sweep<true, false, true>(m, s, FUSED_ARGS);
+            if (jac) launch_sweep<true, true, true>(m, air, s, FUSED_ARGS);
+            else launch_sweep<true, false, true>(m, air, s, FUSED_ARGS);
         } else {
-            if (jac) launch_sweep<false, true, true>(m, s, FUSED_ARGS);
-            else launch_sweep<false, false, true>(m, s, FUSED_ARGS);
+            if (jac) launch_sweep<false, true, true>(m, air, s, FUSED_ARGS);
+            else launch_sweep<false, false, true>(m, air, s, FUSED_ARGS);
         }
     } else {
         if (up_fz) {
-            if (jac) launch_sweep<true, true, false>(m, s, FUSED_ARGS);
-            else launch_sweep<true, false, false>(m, s, FUSED_ARGS);
+            if (jac) launch_sweep<true, true, false>(m, air, s, FUSED_ARGS);
+            else launch_sweep<true, false, false>(m, air, s, FUSED_ARGS);
         } else {
-            if (jac) launch_sweep<false, true, false>(m, s, FUSED_ARGS);
-            else launch_sweep<false, false, false>(m, s, FUSED_ARGS);
+            if (jac) launch_sweep<false, true, false>(m, air, s, FUSED_ARGS);
+            else launch_sweep<false, false, false>(m, air, s, FUSED_ARGS);
         }
     }
 #undef FUSED_ARGS
@@ -1941,7 +1996,7 @@ int up3d_autotune(up3d_mesh* m, const double* phi, const up3d_flow* flow, int re
                 m->tune.elem_persistent = shapes[k][0];
                 m->tune.elem_threads_per_sm = shapes[k][1];
                 const double t = time_it([&] {
-                    launch_sweep<false, true, false>(m, s, m->conn.get(), m->fnbr.get(),
+                    launch_sweep<false, true, false>(m, F.air, s, m->conn.get(), m->fnbr.get(),
                                                      m->disp.get(), m->nodes4.get(), phi, F, u2, no_up, no_br, m->E,
                                                      m->loc.get(), m->res.get(), m->t3v.get(), m->t3_flag.get(),
                                                      m->up32.get(), no_rt, mo, no_flows, no_case, 0, no_brout);
@@ -2019,10 +2074,12 @@ int up3d_residual_jacobian_batched(up3d_mesh* m, const double* phi, int n_cases,
         cudaStream_t s = S(stream);
         if (flows) {
             std::vector<Flow> host(n_cases);
+            bool air = true;
             for (int c = 0; c < n_cases; ++c) {
                 UP3D_REQUIRE(flows[c].u_inf == flows[0].u_inf, UP3D_ERR_VALUE,
                              "up3d_residual_jacobian_batched: the cases must share u_inf");
                 host[c] = make_flow(flows[c]);
+                air &= host[c].air;
             }
             m->flows_ws.alloc(n_cases);
             m->i64_ws.alloc(8);
@@ -2036,6 +2093,7 @@ int up3d_residual_jacobian_batched(up3d_mesh* m, const double* phi, int n_cases,
             m->batch_cases = 0;
             UP3D_REQUIRE(!hbad, UP3D_ERR_VALUE, "up3d_residual_jacobian_batched: case index out of range");
             m->batch_cases = n_cases;
+            m->batch_air = air;
             m->batch_flow0 = flows[0];
         } else {
             UP3D_REQUIRE(m->batch_cases == n_cases, UP3D_ERR_VALUE,

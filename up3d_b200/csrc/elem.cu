@@ -31,6 +31,11 @@ Flow make_flow(const up3d_flow& f) {
         double mc = f.m_cap * f.m_cap;
         F.q2cap = mc * (1.0 + 0.5 * (f.gamma - 1.0) * F.m2inf) / (F.m2inf * (1.0 + 0.5 * (f.gamma - 1.0) * mc));
     }
+    // M^2(q^2) <= M_crit^2 solved for q^2, less a margin far above the
+    // roundings of mach2_of: at or below it switch_of returns C * 0
+    const double sub = F.mc2 * (1.0 + F.hgm * F.m2inf) / (F.m2inf * (1.0 + F.hgm * F.mc2)) * (1.0 - 1e-12);
+    const bool known = F.m2inf > 0.0 && F.hgm > 0.0 && F.mc2 > 0.0 && std::isfinite(F.C) && std::isfinite(sub);
+    F.q2sub = known ? sub : -1.0;
     F.air = (f.gamma == 1.4);
     return F;
 }
@@ -98,7 +103,7 @@ __global__ void k_walk(const int4* __restrict__ fn, const double* __restrict__ d
                        const double* __restrict__ grad, int64_t E, IDX* __restrict__ out) {
     GRID_STRIDE(e, E) {
         double g[3] = {grad[3 * e], grad[3 * e + 1], grad[3 * e + 2]};
-        out[e] = (IDX)upstream_walk(fn, disp, X, conn, e, E, g);
+        out[e] = (IDX)upstream_walk(fn, disp, X, conn[e], (int)e, (int)E, g);
     }
 }
 

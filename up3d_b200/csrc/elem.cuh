@@ -99,12 +99,11 @@ __device__ __forceinline__ void elem_grad_B(const int4* __restrict__ conn, const
 // precomputed per element and face (IEEE-rounded like every other walk
 // operation), so a hop is one dependent load of (fn, disp)[cur] instead of
 // fn[cur] followed by four centroid gathers.  Neighbour entries outside
-// [0, E) count as boundary faces.
-__device__ __forceinline__ int64_t upstream_walk(const int4* __restrict__ fn, const double* __restrict__ disp,
-                                                 const double4* __restrict__ X, const int4* __restrict__ conn,
-                                                 int64_t e, int64_t E, const double g[3]) {
+// [0, E) count as boundary faces.  c = conn[e]; element ids fit 32 bits.
+__device__ __forceinline__ int upstream_walk(const int4* __restrict__ fn, const double* __restrict__ disp,
+                                             const double4* __restrict__ X, const int4 c, int e, int E,
+                                             const double g[3]) {
     const double gx = g[0], gy = g[1], gz = g[2];
-    int4 c = conn[e];
     int nd[4] = {c.x, c.y, c.z, c.w};
     double pmin = 1e300, pmax = -1e300;
 #pragma unroll
@@ -116,16 +115,16 @@ __device__ __forceinline__ int64_t upstream_walk(const int4* __restrict__ fn, co
         if (p > pmax) pmax = p;
     }
     const double target = rmul(0.8, rsub(pmax, pmin));
-    int64_t cur = e;
+    int cur = e;
     double reach = 0.0;
     for (int hops = 0; hops < 4 && reach < target; ++hops) {
         const int4 f = fn[cur];
         double a[12];
-        ld_B(disp + 12 * cur, a);  // the face displacements: the same 96-byte record shape
+        ld_B(disp + 12 * (size_t)cur, a);  // the face displacements: the same 96-byte record shape
         const int nb[4] = {f.x, f.y, f.z, f.w};
         const double d[4] = {dot3r(a[0], a[1], a[2], gx, gy, gz), dot3r(a[3], a[4], a[5], gx, gy, gz),
                              dot3r(a[6], a[7], a[8], gx, gy, gz), dot3r(a[9], a[10], a[11], gx, gy, gz)};
-        int64_t best = -1;
+        int best = -1;
         double best_disp = 0.0;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
@@ -142,10 +141,11 @@ __device__ __forceinline__ int64_t upstream_walk(const int4* __restrict__ fn, co
 }
 
 // rho_tilde_sensitivities_sweep, one element (kernels/upwind.py:687-730).
+template <bool AIR = false>
 __device__ __forceinline__ void live_sensitivities(double q2e, double rho_e, double q2u, double rho_u, bool self_up,
                                                    const Flow& F, double& se, double& su) {
     double r_tmp, drho_e;
-    rho_drho(q2e, F, r_tmp, drho_e);
+    rho_drho<AIR>(q2e, F, r_tmp, drho_e);
     if (self_up) {
         se = rho_e <= F.floor_ ? 0.0 : drho_e;
         su = 0.0;
@@ -166,7 +166,7 @@ __device__ __forceinline__ void live_sensitivities(double q2e, double rho_e, dou
         return;
     }
     double drho_u;
-    rho_drho(q2u, F, r_tmp, drho_u);
+    rho_drho<AIR>(q2u, F, r_tmp, drho_u);
     double djump = rho_e - rho_u;
     if (nu_e >= nu_u) {
         double dnu_e = m2 > F.mc2 ? dswitch_of(q2e, m2, F) : 0.0;
@@ -180,6 +180,7 @@ __device__ __forceinline__ void live_sensitivities(double q2e, double rho_e, dou
 }
 
 // rho_tilde_frozen_sensitivities_sweep, one element (kernels/upwind.py:616-643).
+template <bool AIR = false>
 __device__ __forceinline__ void frozen_sensitivities(int b, double q2e, double rho_e, double q2u, double rho_u,
                                                      const Flow& F, double& se, double& su) {
     if (b == 3) {
@@ -188,14 +189,14 @@ __device__ __forceinline__ void frozen_sensitivities(int b, double q2e, double r
         return;
     }
     double r_tmp, drho_e;
-    rho_drho(q2e, F, r_tmp, drho_e);
+    rho_drho<AIR>(q2e, F, r_tmp, drho_e);
     if (b == 0) {
         se = drho_e;
         su = 0.0;
         return;
     }
     double drho_u;
-    rho_drho(q2u, F, r_tmp, drho_u);
+    rho_drho<AIR>(q2u, F, r_tmp, drho_u);
     double djump = rho_e - rho_u;
     if (b == 1) {
         double m2 = mach2_of(q2e, F);

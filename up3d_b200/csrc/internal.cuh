@@ -174,6 +174,7 @@ struct up3d_mesh {
     up3d::DBuf<int32_t> nb_si;
     int32_t nb_depth = 0;
     int64_t nb_total = 0;
+    bool batch_air = false;                    // gamma == 1.4 in all of them
     up3d_flow batch_flow0 = {};                // its case 0
 
     // geometry (device)
@@ -276,6 +277,7 @@ struct Flow {
     double floor_;
     double inv_u2;
     double q2cap;     // q^2 at M_cap (+inf when M_inf == 0)
+    double q2sub;     // q^2 surely below M_crit (its switch is exactly 0); -1: not known
     bool air;         // gamma == 1.4
 };
 
@@ -286,18 +288,22 @@ __device__ __forceinline__ double base_of(double q2, const Flow& F) {
     return radd(1.0, rmul(rmul(F.hgm, F.m2inf), rsub(1.0, q2)));
 }
 
+// AIR: gamma == 1.4 known when compiled, so that a kernel carries no pow call
+// and keeps the registers that one takes.
+template <bool AIR = false>
 __device__ __forceinline__ double rho_of(double q2, const Flow& F) {
     double b = base_of(q2, F);
     if (b < 1e-10) b = 1e-10;
-    if (F.air) return b * b * sqrt(b);
+    if (AIR || F.air) return b * b * sqrt(b);
     return pow(b, F.expo);
 }
 
 // rho and d rho / d q^2 from one base evaluation.
+template <bool AIR = false>
 __device__ __forceinline__ void rho_drho(double q2, const Flow& F, double& rho, double& drho) {
     double b = base_of(q2, F);
     if (b < 1e-10) b = 1e-10;
-    if (F.air) {
+    if (AIR || F.air) {
         double sb = sqrt(b);
         rho = b * b * sb;
         drho = -0.5 * F.m2inf * (b * sb);
