@@ -64,7 +64,9 @@ __device__ __forceinline__ T warp_row_sum(const int32_t* __restrict__ Ap, const 
             v[j] = k < e ? ld_stream(Ax + k) : T(0);
         }
 #pragma unroll
-        for (int j = 0; j < CSR_ROWS_CHUNK / 32; ++j) sh[j * 32 + lane] = c[j] >= 0 ? term(c[j], v[j]) : T(0);
+        for (int j = 0; j < CSR_ROWS_CHUNK / 32; ++j) v[j] = c[j] >= 0 ? term(c[j], v[j]) : T(0);
+#pragma unroll
+        for (int j = 0; j < CSR_ROWS_CHUNK / 32; ++j) sh[j * 32 + lane] = v[j];
         __syncwarp();
         const int32_t a = ms > c0 ? ms : c0;
         const int32_t b = me < c0 + CSR_ROWS_CHUNK ? me : c0 + CSR_ROWS_CHUNK;

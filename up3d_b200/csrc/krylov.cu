@@ -26,12 +26,21 @@ namespace {
 #define GRID_STRIDE(i, n) \
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < (n); i += (int64_t)gridDim.x * blockDim.x)
 
-// out = x . y; products and sums in FP64 whatever the vector type.
+// The kernels of an iteration are launched overlapped (each starts while the
+// one before drains: 2 us less between two of them): vectors and scalars that
+// an earlier one writes are read after pdl_wait, and not through __restrict__.
+// Results for the host go to `host`, page-locked memory, from the kernel that
+// forms them: a copy behind it costs 5 us of an iteration.
+
+// out = x . y (and *host when given); products and sums in FP64 whatever the
+// vector type.
 template <class T>
 __global__ void __launch_bounds__(DOT_BLOCK)
-    k_dot(const T* __restrict__ x, const T* __restrict__ y, int64_t n, double* __restrict__ partial,
-          double* __restrict__ out, unsigned int* __restrict__ counter) {
+    k_dot(const T* x, const T* y, int64_t n, double* __restrict__ partial, double* out, double* host,
+          unsigned int* __restrict__ counter) {
     __shared__ double sh[DOT_BLOCK / 32];
+    pdl_trigger();
+    pdl_wait();
     double acc = 0.0;
     GRID_STRIDE(i, n) acc += (double)x[i] * (double)y[i];
     acc = block_sum(acc, sh);
@@ -40,6 +49,7 @@ __global__ void __launch_bounds__(DOT_BLOCK)
     acc = sum_partials(partial, (int)gridDim.x, sh);
     if (threadIdx.x == 0) {
         *out = acc;
+        if (host) *host = acc;
         *counter = 0u;
     }
 }
@@ -71,7 +81,8 @@ constexpr int basis_blocks = KJ == 1 ? 6 : KJ == 2 ? 4 : KJ <= 4 ? 3 : 2;
 template <class T, int KJ, int PASS>
 __global__ void __launch_bounds__(DOT_BLOCK, basis_blocks<KJ>)
     k_basis(const T* __restrict__ V, int64_t ldv, int K, double* h, T* y, int64_t n, bool self,
-            double* __restrict__ partial, double* __restrict__ out, unsigned int* __restrict__ counter) {
+            double* __restrict__ partial, double* out, unsigned int* __restrict__ counter, const double* hsrc,
+            double* hdst, int hlen) {
     constexpr int VEC = 16 / sizeof(T), ROWS = 32 * VEC;
     struct alignas(16) Vec {
         T x[VEC];
@@ -80,6 +91,8 @@ __global__ void __launch_bounds__(DOT_BLOCK, basis_blocks<KJ>)
     __shared__ alignas(16) double fresh[ROWS];               // the updated y
     __shared__ double sums[8 * KJ + 1];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    pdl_trigger();
+    pdl_wait();
     double hw[KJ];
 #pragma unroll
     for (int j = 0; j < KJ; ++j) hw[j] = PASS != BASIS_DOTS && w + 8 * j < K ? h[w + 8 * j] : 0.0;
@@ -190,6 +203,10 @@ __global__ void __launch_bounds__(DOT_BLOCK, basis_blocks<KJ>)
         }
     }
     if (threadIdx.x == 0) *counter = 0u;
+    if (hdst) {   // the step's column, complete now
+        __syncthreads();
+        for (int k = threadIdx.x; k < hlen; k += DOT_BLOCK) hdst[k] = hsrc[k];
+    }
 }
 
 // y -= sum_k h[k] V_k  (h on the device, staged in shared memory 64 at a
@@ -241,15 +258,17 @@ __global__ void k_to_f32(const double* __restrict__ a, float* __restrict__ b, in
 // CG updates: x += alpha p, r -= alpha q (alpha = *rz / *pq), and out = r . r
 // of the new r in the order of k_dot.
 __global__ void __launch_bounds__(DOT_BLOCK)
-    k_cg_update(const double* __restrict__ rz, const double* __restrict__ pq, double* __restrict__ x,
-                double* __restrict__ r, const double* __restrict__ p, const double* __restrict__ q, int64_t n,
-                double* __restrict__ partial, double* __restrict__ out, unsigned int* __restrict__ counter) {
+    k_cg_update(const double* rz, const double* pq, double* x, double* r, const double* p, const double* q, int64_t n,
+                double* __restrict__ partial, double* out, double* host, unsigned int* __restrict__ counter) {
     __shared__ double sh[DOT_BLOCK / 32];
+    pdl_trigger();
+    pdl_wait();
     const double alpha = *rz / *pq;
     double acc = 0.0;
     GRID_STRIDE(i, n) {
-        x[i] += alpha * p[i];
-        const double v = r[i] - alpha * q[i];
+        const double xi = x[i], ri = r[i], pi = p[i], qi = q[i];
+        x[i] = xi + alpha * pi;
+        const double v = ri - alpha * qi;
         r[i] = v;
         acc += v * v;
     }
@@ -259,13 +278,15 @@ __global__ void __launch_bounds__(DOT_BLOCK)
     acc = sum_partials(partial, (int)gridDim.x, sh);
     if (threadIdx.x == 0) {
         *out = acc;
+        if (host) *host = acc;
         *counter = 0u;
     }
 }
 
 // p = z + beta p (beta = rz_new / rz_old)
-__global__ void k_cg_dir(const double* __restrict__ rz_new, const double* __restrict__ rz_old,
-                         const double* __restrict__ z, double* __restrict__ p, int64_t n) {
+__global__ void k_cg_dir(const double* rz_new, const double* rz_old, const double* z, double* p, int64_t n) {
+    pdl_trigger();
+    pdl_wait();
     const double beta = *rz_new / *rz_old;
     GRID_STRIDE(i, n) p[i] = z[i] + beta * p[i];
 }
@@ -309,26 +330,25 @@ Blas::~Blas() {
 
 template <class T, int KJ, int PASS>
 static void launch_basis_k(Blas& bl, const T* V, int64_t ldv, int K, double* h, T* y, int64_t n, bool self,
-                           double* out) {
+                           double* out, const double* hsrc, double* hdst, int hlen) {
     static_assert(basis_blocks<KJ> <= BASIS_MAX_BLOCKS / 148, "partials hold BASIS_MAX_BLOCKS blocks");
     const unsigned grid = grid_for(n, 32 * 16 / sizeof(T), (int64_t)148 * basis_blocks<KJ>);
-    k_basis<T, KJ, PASS><<<grid, DOT_BLOCK, 0, bl.s>>>(V, ldv, K, h, y, n, self, bl.partial.get(), out,
-                                                       bl.counter.get());
-    UP3D_CHECK_LAUNCH();
+    launch_kernel(true, k_basis<T, KJ, PASS>, grid, DOT_BLOCK, bl.s, V, ldv, K, h, y, n, self, bl.partial.get(), out,
+                  bl.counter.get(), hsrc, hdst, hlen);
 }
 template <class T, int PASS>
 static void launch_basis(Blas& bl, const T* V, int64_t ldv, int K, double* h, T* y, int64_t n, bool self,
-                         double* out) {
+                         double* out, const double* hsrc = nullptr, double* hdst = nullptr, int hlen = 0) {
     switch ((K + 7) / 8) {
         case 0:
-        case 1: return launch_basis_k<T, 1, PASS>(bl, V, ldv, K, h, y, n, self, out);
-        case 2: return launch_basis_k<T, 2, PASS>(bl, V, ldv, K, h, y, n, self, out);
-        case 3: return launch_basis_k<T, 3, PASS>(bl, V, ldv, K, h, y, n, self, out);
-        case 4: return launch_basis_k<T, 4, PASS>(bl, V, ldv, K, h, y, n, self, out);
-        case 5: return launch_basis_k<T, 5, PASS>(bl, V, ldv, K, h, y, n, self, out);
-        case 6: return launch_basis_k<T, 6, PASS>(bl, V, ldv, K, h, y, n, self, out);
-        case 7: return launch_basis_k<T, 7, PASS>(bl, V, ldv, K, h, y, n, self, out);
-        default: return launch_basis_k<T, 8, PASS>(bl, V, ldv, K, h, y, n, self, out);
+        case 1: return launch_basis_k<T, 1, PASS>(bl, V, ldv, K, h, y, n, self, out, hsrc, hdst, hlen);
+        case 2: return launch_basis_k<T, 2, PASS>(bl, V, ldv, K, h, y, n, self, out, hsrc, hdst, hlen);
+        case 3: return launch_basis_k<T, 3, PASS>(bl, V, ldv, K, h, y, n, self, out, hsrc, hdst, hlen);
+        case 4: return launch_basis_k<T, 4, PASS>(bl, V, ldv, K, h, y, n, self, out, hsrc, hdst, hlen);
+        case 5: return launch_basis_k<T, 5, PASS>(bl, V, ldv, K, h, y, n, self, out, hsrc, hdst, hlen);
+        case 6: return launch_basis_k<T, 6, PASS>(bl, V, ldv, K, h, y, n, self, out, hsrc, hdst, hlen);
+        case 7: return launch_basis_k<T, 7, PASS>(bl, V, ldv, K, h, y, n, self, out, hsrc, hdst, hlen);
+        default: return launch_basis_k<T, 8, PASS>(bl, V, ldv, K, h, y, n, self, out, hsrc, hdst, hlen);
     }
 }
 
@@ -345,18 +365,16 @@ void Blas::multidot(const T* V, int64_t ldv, int K, const T* y, int64_t n, doubl
 
 template <class T>
 void Blas::dot_dev(const T* x, const T* y, int64_t n, double* out_dev) {
-    k_dot<T><<<dot_grid(n), DOT_BLOCK, 0, s>>>(x, y, n, partial.get(), out_dev, counter.get());
-    UP3D_CHECK_LAUNCH();
+    dot_to<T>(x, y, n, out_dev, nullptr);
+}
+template <class T>
+void Blas::dot_to(const T* x, const T* y, int64_t n, double* out_dev, double* out_host) {
+    launch_kernel(true, k_dot<T>, dot_grid(n), DOT_BLOCK, s, x, y, n, partial.get(), out_dev, out_host, counter.get());
 }
 
 template <class T>
 double Blas::dot(const T* x, const T* y, int64_t n) {
-    dot_dev(x, y, n, scal.get());
-    return read(scal.get());
-}
-
-double Blas::read(const double* dev) {
-    UP3D_CUDA(cudaMemcpyAsync(host, dev, sizeof(double), cudaMemcpyDeviceToHost, s));
+    dot_to<T>(x, y, n, scal.get(), host);
     UP3D_CUDA(cudaStreamSynchronize(s));
     return host[0];
 }
@@ -384,8 +402,10 @@ void Blas::axpy_dots(const T* V, int64_t ldv, int K, double* h_dev, T* y, int64_
 }
 
 template <class T>
-void Blas::axpy_norm(const T* V, int64_t ldv, int K, const double* h_dev, T* y, int64_t n, double* out_dev) {
-    launch_basis<T, BASIS_AXPY_NORM>(*this, V, ldv, K, const_cast<double*>(h_dev), y, n, false, out_dev);
+void Blas::axpy_norm(const T* V, int64_t ldv, int K, const double* h_dev, T* y, int64_t n, double* out_dev,
+                     const double* col, double* col_host, int len) {
+    launch_basis<T, BASIS_AXPY_NORM>(*this, V, ldv, K, const_cast<double*>(h_dev), y, n, false, out_dev, col, col_host,
+                                     len);
 }
 
 #define UP3D_BLAS_INST(T)                                                                 \
@@ -396,7 +416,8 @@ void Blas::axpy_norm(const T* V, int64_t ldv, int K, const double* h_dev, T* y, 
     template void Blas::scale<T>(T*, double, int64_t);                                   \
     template void Blas::multiaxpy<T>(const T*, int64_t, int, const double*, T*, int64_t); \
     template void Blas::axpy_dots<T>(const T*, int64_t, int, double*, T*, int64_t, double*); \
-    template void Blas::axpy_norm<T>(const T*, int64_t, int, const double*, T*, int64_t, double*);
+    template void Blas::axpy_norm<T>(const T*, int64_t, int, const double*, T*, int64_t, double*, const double*, \
+                                     double*, int);
 UP3D_BLAS_INST(double)
 UP3D_BLAS_INST(float)
 #undef UP3D_BLAS_INST
@@ -424,6 +445,11 @@ struct KrylovWs {
             pin_n = n;
         }
         return pin;
+    }
+    cudaEvent_t column_done = nullptr;
+    cudaEvent_t column() {   // a GMRES step's column has reached `pin`
+        if (!column_done) UP3D_CUDA(cudaEventCreateWithFlags(&column_done, cudaEventDisableTiming));
+        return column_done;
     }
     template <class T>
     DBuf<T>* bufs();
@@ -460,7 +486,7 @@ void Operator::apply(const double* x, double* y, cudaStream_t s) const {
     }
     // y = A x (+ extra x: the Term-3 entries outside the P1 pattern), one pass
     launch_spmv2<double>(A.n, A.indptr, A.indices, A.data, extra.indptr, extra.indices, extra.data, x, y,
-                         A.dirichlet, s);
+                         A.dirichlet, s, true);
 }
 
 // FP32 operator: the FP32 copies of the values (data32, extra32).
@@ -468,7 +494,7 @@ void Operator::apply(const float* x, float* y, cudaStream_t s) const {
     UP3D_REQUIRE(!coupled, UP3D_ERR_ARGUMENT, "the coupled wake operator is FP64 only");
     UP3D_REQUIRE(data32 && (!extra.indptr || extra32), UP3D_ERR_ARGUMENT, "FP32 operator without FP32 values");
     launch_spmv2<float>(A.n, A.indptr, A.indices, data32, extra.indptr, extra.indices, extra32, x, y, A.dirichlet,
-                        s);
+                        s, true);
 }
 
 void Operator::residual(const double* b, const double* x, double* r, double* tmp, cudaStream_t s) const {
@@ -577,15 +603,14 @@ int cg_solve(const Operator& op, const double* b, double* x, double rtol, double
         for (it = 1; it <= maxiter; ++it) {
             op.apply(p.get(), q.get(), s);
             bl.dot_dev(p.get(), q.get(), n, pq);
-            k_cg_update<<<dot_grid(n), DOT_BLOCK, 0, s>>>(rz, pq, x, r.get(), p.get(), q.get(), n, bl.partial.get(), rr,
-                                                          bl.counter.get());
-            UP3D_CHECK_LAUNCH();
-            rn = std::sqrt(bl.read(rr));
+            launch_kernel(true, k_cg_update, dot_grid(n), DOT_BLOCK, s, rz, pq, x, r.get(), p.get(), q.get(), n,
+                          bl.partial.get(), rr, bl.host, bl.counter.get());
+            UP3D_CUDA(cudaStreamSynchronize(s));
+            rn = std::sqrt(*bl.host);
             if (rn <= tol || !std::isfinite(rn)) break;
             precond_apply(M, r.get(), z.get(), n, s);
             bl.dot_dev(r.get(), z.get(), n, rz_next);
-            k_cg_dir<<<grid_for(n, 256), 256, 0, s>>>(rz_next, rz, z.get(), p.get(), n);
-            UP3D_CHECK_LAUNCH();
+            launch_kernel(true, k_cg_dir, grid_for(n, 256), 256, s, rz_next, rz, z.get(), p.get(), n);
             std::swap(rz, rz_next);
         }
         if (it > maxiter) it = maxiter;
@@ -600,8 +625,9 @@ int cg_solve(const Operator& op, const double* b, double* x, double rtol, double
 // V_{col+1} *= 1 / |w| unless |w| <= eps |w_before| (Arnoldi breakdown);
 // hn = (|w_before|^2, |w|^2)
 template <class T>
-__global__ void k_scale_unless_breakdown(const T* __restrict__ w, T* __restrict__ v, const double* __restrict__ hn,
-                                         double eps, int64_t n) {
+__global__ void k_scale_unless_breakdown(const T* w, T* v, const double* hn, double eps, int64_t n) {
+    pdl_trigger();
+    pdl_wait();
     const double h0 = sqrt(hn[0]), h1 = sqrt(hn[1]);
     const bool keep = h1 <= eps * h0;   // breakdown: the vector is copied unscaled
     const double f = keep ? 1.0 : 1.0 / h1;
@@ -707,7 +733,7 @@ int gmres_solve(const Operator& op, const T* b, T* x, double rtol, double atol, 
             if (col + 1 <= BASIS_MAX) {
                 // pass 2 leaves its coefficients in hpass and adds them to hsum
                 bl.axpy_dots(V.get(), ld, col + 1, hsum, wv, n, hpass);
-                bl.axpy_norm(V.get(), ld, col + 1, hpass, wv, n, hn + 1);
+                bl.axpy_norm(V.get(), ld, col + 1, hpass, wv, n, hn + 1, hsum, hbuf, col + 3);
             } else {
                 bl.multiaxpy(V.get(), ld, col + 1, hsum, wv, n);
                 bl.multidot(V.get(), ld, col + 1, wv, n, hpass);
@@ -715,11 +741,13 @@ int gmres_solve(const Operator& op, const T* b, T* x, double rtol, double atol, 
                 bl.dot_dev(wv, wv, n, hn + 1);
                 k_accumulate<<<1, 256, 0, s>>>(hsum, hpass, col + 1);
                 UP3D_CHECK_LAUNCH();
+                UP3D_CUDA(cudaMemcpyAsync(hbuf, hsum, sizeof(double) * (col + 3), cudaMemcpyDeviceToHost, s));
             }
-            k_scale_unless_breakdown<T><<<grid_for(n, 256), 256, 0, s>>>(wv, V.get() + (size_t)(col + 1) * ld, hn, eps, n);
-            UP3D_CHECK_LAUNCH();
-            UP3D_CUDA(cudaMemcpyAsync(hbuf, hsum, sizeof(double) * (col + 3), cudaMemcpyDeviceToHost, s));
-            UP3D_CUDA(cudaStreamSynchronize(s));
+            // the host turns to the column while the vector is normalised
+            UP3D_CUDA(cudaEventRecord(W.column(), s));
+            launch_kernel(true, k_scale_unless_breakdown<T>, grid_for(n, 256), 256, s, wv,
+                          V.get() + (size_t)(col + 1) * ld, hn, eps, n);
+            UP3D_CUDA(cudaEventSynchronize(W.column()));
             for (int k = 0; k <= col; ++k) Hat(col, k) = hbuf[k];
             const double h0 = std::sqrt(hbuf[col + 1]);
             const double h1 = std::sqrt(hbuf[col + 2]);

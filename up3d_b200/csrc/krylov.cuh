@@ -13,7 +13,8 @@ void launch_spmv(int64_t n, const int32_t* indptr, const int32_t* indices, const
                  const uint8_t* dir, cudaStream_t s);
 template <class T>
 void launch_spmv2(int64_t n, const int32_t* indptr, const int32_t* indices, const T* data, const int32_t* xptr,
-                  const int32_t* xidx, const T* xdata, const T* x, T* y, const uint8_t* dir, cudaStream_t s);
+                  const int32_t* xidx, const T* xdata, const T* x, T* y, const uint8_t* dir, cudaStream_t s,
+                  bool overlap = false);
 
 // r = b - (A x + xA x) with each row's sum rounded once (linear.cu)
 void launch_residual(int64_t n, const int32_t* indptr, const int32_t* indices, const double* data,
@@ -32,7 +33,7 @@ struct Blas {
     cudaStream_t s;
     DBuf<double> partial, scal;
     DBuf<unsigned int> counter;   // blocks arrived, for the last-block reductions (re-armed by it)
-    double* host = nullptr;  // pinned scalar readback
+    double* host = nullptr;  // page-locked, written by the kernels that form a scalar
     explicit Blas(cudaStream_t s);
     ~Blas();
     // out[k] = V_k . y for k < K, then y . y at out[K] when self_dot
@@ -40,7 +41,9 @@ struct Blas {
     void multidot(const T* V, int64_t ldv, int K, const T* y, int64_t n, double* out_dev, bool self_dot = false);
     template <class T>
     void dot_dev(const T* x, const T* y, int64_t n, double* out_dev);
-    double read(const double* dev);   // one scalar to the host (synchronises the stream)
+    // the same, and to page-locked memory unless out_host is NULL
+    template <class T>
+    void dot_to(const T* x, const T* y, int64_t n, double* out_dev, double* out_host);
     template <class T>
     double dot(const T* x, const T* y, int64_t n);
     template <class T>
@@ -50,11 +53,13 @@ struct Blas {
     template <class T>
     void multiaxpy(const T* V, int64_t ldv, int K, const double* h_dev, T* y, int64_t n);
     // y -= V h (K <= 64) in one sweep that also forms out = V^T y of the new
-    // y and adds it to h, or out = y . y
+    // y and adds it to h, or out = y . y (then the len values at col, out
+    // among them, also go to page-locked memory at col_host)
     template <class T>
     void axpy_dots(const T* V, int64_t ldv, int K, double* h_dev, T* y, int64_t n, double* out_dev);
     template <class T>
-    void axpy_norm(const T* V, int64_t ldv, int K, const double* h_dev, T* y, int64_t n, double* out_dev);
+    void axpy_norm(const T* V, int64_t ldv, int K, const double* h_dev, T* y, int64_t n, double* out_dev,
+                   const double* col = nullptr, double* col_host = nullptr, int len = 0);
 };
 
 // y = A x (+ extra x): the P1-pattern matrix plus, for the Newton Jacobian,

@@ -22,7 +22,9 @@ template <class T, int TPR>
 __global__ void __launch_bounds__(TPR == 0 ? CSR_WARP_BLOCK : CSR_ROWS_BLOCK)
     k_spmv(int64_t n, const int32_t* __restrict__ indptr, const int32_t* __restrict__ indices,
            const T* __restrict__ data, const int32_t* __restrict__ xptr, const int32_t* __restrict__ xidx,
-           const T* __restrict__ xdata, const T* __restrict__ x, T* __restrict__ y, const uint8_t* __restrict__ dir) {
+           const T* __restrict__ xdata, const T* x, T* y, const uint8_t* __restrict__ dir) {
+    pdl_trigger();
+    pdl_wait();   // x may come from an overlapped launch: no __restrict__ on it
     auto term = [&](int32_t c, T v) {
         const T p = v * x[c];   // beside the mask's load, not behind it
         return (dir && dir[c]) ? T(0) : p;
@@ -119,20 +121,20 @@ void launch_residual(int64_t n, const int32_t* indptr, const int32_t* indices, c
 // enough to fill the GPU that way, else 4 lanes per row
 template <class T>
 void launch_spmv2(int64_t n, const int32_t* indptr, const int32_t* indices, const T* data, const int32_t* xptr,
-                  const int32_t* xidx, const T* xdata, const T* x, T* y, const uint8_t* dir, cudaStream_t s) {
+                  const int32_t* xidx, const T* xdata, const T* x, T* y, const uint8_t* dir, cudaStream_t s,
+                  bool overlap) {
     if (n >= CSR_ROWS_MIN_ROWS)
-        k_spmv<T, 0><<<csr_rows_grid(n, CSR_WARP_BLOCK), CSR_WARP_BLOCK, 0, s>>>(n, indptr, indices, data, xptr, xidx,
-                                                                                 xdata, x, y, dir);
+        launch_kernel(overlap, k_spmv<T, 0>, csr_rows_grid(n, CSR_WARP_BLOCK), CSR_WARP_BLOCK, s, n, indptr, indices,
+                      data, xptr, xidx, xdata, x, y, dir);
     else
-        k_spmv<T, 4><<<lanes_grid(n, 4), CSR_ROWS_BLOCK, 0, s>>>(n, indptr, indices, data, xptr, xidx, xdata, x, y,
-                                                                 dir);
-    UP3D_CHECK_LAUNCH();
+        launch_kernel(overlap, k_spmv<T, 4>, lanes_grid(n, 4), CSR_ROWS_BLOCK, s, n, indptr, indices, data, xptr,
+                      xidx, xdata, x, y, dir);
 }
 
 template <class T>
 void launch_spmv(int64_t n, const int32_t* indptr, const int32_t* indices, const T* data, const T* x, T* y,
                  const uint8_t* dir, cudaStream_t s) {
-    launch_spmv2<T>(n, indptr, indices, data, nullptr, nullptr, nullptr, x, y, dir, s);
+    launch_spmv2<T>(n, indptr, indices, data, nullptr, nullptr, nullptr, x, y, dir, s, false);
 }
 
 template void launch_spmv<double>(int64_t, const int32_t*, const int32_t*, const double*, const double*, double*,
@@ -141,9 +143,10 @@ template void launch_spmv<float>(int64_t, const int32_t*, const int32_t*, const 
                                  const uint8_t*, cudaStream_t);
 template void launch_spmv2<double>(int64_t, const int32_t*, const int32_t*, const double*, const int32_t*,
                                    const int32_t*, const double*, const double*, double*, const uint8_t*,
-                                   cudaStream_t);
+                                   cudaStream_t, bool);
 template void launch_spmv2<float>(int64_t, const int32_t*, const int32_t*, const float*, const int32_t*,
-                                  const int32_t*, const float*, const float*, float*, const uint8_t*, cudaStream_t);
+                                  const int32_t*, const float*, const float*, float*, const uint8_t*, cudaStream_t,
+                                  bool);
 
 }  // namespace up3d
 
