@@ -389,6 +389,62 @@ __device__ __forceinline__ int32_t dev_lower_bound(const int32_t* __restrict__ a
     return lo;
 }
 
+// Pattern of the finest operator from the caller's: entries of row r in
+// cnt[r + 1] (cnt[0] = 0), then, with its row offsets p, the columns and the
+// caller's entry of each.  Eight lanes per row (a lane's ballot among its
+// row's eight orders the entries).  Bound by the pattern's bytes.
+__global__ void __launch_bounds__(256)
+    k_embed_count(int64_t n, const int32_t* __restrict__ Ap, const int32_t* __restrict__ Ai,
+                  const uint8_t* __restrict__ dir, int32_t* __restrict__ cnt) {
+    const int sub = threadIdx.x & 7;
+    const int64_t step = (int64_t)gridDim.x * (blockDim.x >> 3);
+    for (int64_t base = (int64_t)blockIdx.x * (blockDim.x >> 3); base < n; base += step) {   // block-uniform
+        const int64_t r = base + (threadIdx.x >> 3);
+        int32_t c = 0;
+        if (r < n && !(dir && dir[r]))
+            for (int32_t k = Ap[r] + sub; k < Ap[r + 1]; k += 8) c += !(dir && dir[Ai[k]]);
+        for (int o = 4; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+        if (r < n && sub == 0) cnt[r + 1] = dir && dir[r] ? 1 : c;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) cnt[0] = 0;
+}
+__global__ void __launch_bounds__(256)
+    k_embed_fill(int64_t n, const int32_t* __restrict__ Ap, const int32_t* __restrict__ Ai,
+                 const uint8_t* __restrict__ dir, const int32_t* __restrict__ p, int32_t* __restrict__ out,
+                 int32_t* __restrict__ src) {
+    const int sub = threadIdx.x & 7, group = threadIdx.x & 24;
+    const int64_t step = (int64_t)gridDim.x * (blockDim.x >> 3);
+    for (int64_t base = (int64_t)blockIdx.x * (blockDim.x >> 3); base < n; base += step) {   // block-uniform
+        const int64_t r = base + (threadIdx.x >> 3);
+        int32_t k0 = 0, k1 = 0, o = 0;
+        if (r < n) {
+            o = p[r];
+            if (dir && dir[r]) {
+                if (sub == 0) {
+                    out[o] = (int32_t)r;
+                    src[o] = -1;
+                }
+            } else {
+                k0 = Ap[r];
+                k1 = Ap[r + 1];
+            }
+        }
+        const int32_t most = __reduce_max_sync(0xffffffffu, k1 - k0);
+        for (int32_t j = 0; j < most; j += 8) {
+            const int32_t k = k0 + j + sub;
+            const int32_t c = k < k1 ? Ai[k] : 0;
+            const bool keep = k < k1 && !(dir && dir[c]);
+            const unsigned m = __ballot_sync(0xffffffffu, keep) >> group & 0xffu;
+            if (keep) {
+                const int32_t at = o + __popc(m & ((1u << sub) - 1u));
+                out[at] = c;
+                src[at] = k;
+            }
+            o += __popc(m);
+        }
+    }
+}
+
 // finest operator from the caller's matrix: src[k] = caller entry, or -1
 // for the identity entry of a constrained row
 __global__ void k_embed(int64_t nnz, const int32_t* __restrict__ src, const double* __restrict__ data,
@@ -1478,13 +1534,7 @@ void* amg_setup(const up3d_csr& A, const up3d_amg_options& opt, cudaStream_t s) 
         a->post = std::max(0, opt.postsmooth);
         const int64_t n = A.n;
         UP3D_REQUIRE(n > 0, UP3D_ERR_VALUE, "AMG setup: empty matrix");
-        HostCSR h;
-        h.n = h.m = n;
-        h.p.resize(n + 1);
-        d2h(h.p.data(), A.indptr, sizeof(int32_t) * (n + 1), s);
-        const int64_t nnz = h.p[n];
-        h.i.resize(nnz);
-        d2h(h.i.data(), A.indices, sizeof(int32_t) * nnz, s);
+        const int64_t nnz = read_back(A.indptr + n, s);
         std::vector<uint8_t> skip(n, 0);
         if (A.dirichlet)
             UP3D_CUDA(cudaMemcpyAsync(skip.data(), A.dirichlet, n, cudaMemcpyDeviceToHost, s));
@@ -1501,38 +1551,33 @@ void* amg_setup(const up3d_csr& A, const up3d_amg_options& opt, cudaStream_t s) 
             UP3D_CUDA(cudaMemcpyAsync(a->in_i.get(), A.indices, sizeof(int32_t) * nnz, cudaMemcpyDeviceToDevice, s));
         if (a->has_dir) upload(a->in_dir, skip, s);
         // finest operator as the embedded free-DOF system: identity rows,
-        // constrained columns dropped; src = caller entry (-1: identity)
+        // constrained columns dropped; src = caller entry (-1: identity).
+        // Formed on the device, the host reads the pattern it works on
+        // (9.4 M entries: formed on the host, with the caller's pattern read
+        // and two arrays sent, 20-40 ms of a set-up; so 5-14)
+        auto* F0 = new SymLevel();
+        a->sym.push_back(F0);
+        const uint8_t* dir = a->has_dir ? a->in_dir.get() : nullptr;
         HostCSR e;
-        std::vector<int32_t> src;
         e.n = e.m = n;
-        e.p.assign(n + 1, 0);
-#pragma omp parallel for schedule(static)
-        for (int64_t r = 0; r < n; ++r) {
-            int32_t cnt = 0;
-            if (skip[r]) cnt = 1;
-            else
-                for (int32_t k = h.p[r]; k < h.p[r + 1]; ++k) cnt += !skip[h.i[k]];
-            e.p[r + 1] = cnt;
-        }
+        e.p.resize(n + 1);
+        F0->A.p.alloc(n + 1);
+        k_embed_count<<<grid_for(n, 32, (int64_t)148 * 64), 256, 0, s>>>(n, a->in_p.get(), a->in_i.get(), dir,
+                                                                       F0->A.p.get());
+        UP3D_CHECK_LAUNCH();
+        d2h(e.p.data(), F0->A.p.get(), sizeof(int32_t) * (n + 1), s);
         for (int64_t r = 0; r < n; ++r) e.p[r + 1] += e.p[r];
+        F0->A.n = F0->A.m = n;
+        F0->A.nnz = e.p[n];
+        F0->A.i.alloc(std::max<int64_t>(e.p[n], 1));
+        F0->A.x.alloc(std::max<int64_t>(e.p[n], 1));
+        a->emb_src.alloc(std::max<int64_t>(e.p[n], 1));
+        h2d(F0->A.p.get(), e.p.data(), sizeof(int32_t) * (n + 1), s);
+        k_embed_fill<<<grid_for(n, 32, (int64_t)148 * 64), 256, 0, s>>>(n, a->in_p.get(), a->in_i.get(), dir,
+                                                                      F0->A.p.get(), F0->A.i.get(), a->emb_src.get());
+        UP3D_CHECK_LAUNCH();
         e.i.resize(e.p[n]);
-        src.resize(e.p[n]);
-#pragma omp parallel for schedule(static)
-        for (int64_t r = 0; r < n; ++r) {
-            int32_t o = e.p[r];
-            if (skip[r]) {
-                e.i[o] = (int32_t)r;
-                src[o] = -1;
-                continue;
-            }
-            for (int32_t k = h.p[r]; k < h.p[r + 1]; ++k)
-                if (!skip[h.i[k]]) {
-                    e.i[o] = h.i[k];
-                    src[o] = k;
-                    ++o;
-                }
-        }
-        upload(a->emb_src, src, s);
+        if (e.p[n]) d2h(e.i.data(), F0->A.i.get(), sizeof(int32_t) * e.p[n], s);
         // symbolic levels
         std::vector<HostCSR> As;
         As.push_back(std::move(e));
@@ -1541,9 +1586,11 @@ void* amg_setup(const up3d_csr& A, const up3d_amg_options& opt, cudaStream_t s) 
         int64_t nmax = n;
         while (true) {
             const HostCSR& Al = As.back();
-            auto* F = new SymLevel();
-            a->sym.push_back(F);
-            F->A.upload_pattern(Al, s);
+            if (As.size() > 1) {
+                a->sym.push_back(new SymLevel());
+                a->sym.back()->A.upload_pattern(Al, s);
+            }
+            SymLevel* F = a->sym.back();
             F->a_max = longest_row(Al);
             make_slices(*F, Al, s);
             upload(F->diag, diag_slots(Al), s);
