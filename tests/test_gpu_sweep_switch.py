@@ -68,3 +68,38 @@ def test_against_the_kernels_that_form_every_switch(cells, gamma, m_inf, m_crit,
         assert (mon["n_supersonic"], mon["n_floored"]) == (sup, flo)
         only = ev.evaluate(phi, flow, jacobian=False).cpu().numpy()
         assert np.array_equal(only, got)
+
+
+@pytest.mark.parametrize("gammas", [(1.4, 1.4), (1.4, 1.3), (1.3, 1.3)])
+def test_captured_batch_follows_a_new_flow_table(gammas):
+    """A captured evaluation reads the flow table of its replay, also when
+    the gas is another than the one it was captured with."""
+    import torch
+    from up3d_b200 import _lib as L
+    from up3d_b200.mesh.kuhn import bump_channel
+    from up3d_b200.solve.batched import BatchedChannels
+    from up3d_b200.solve.fused import FlowParams
+    meshes = [bump_channel(6, 3, 3, amplitude=0.05, seed=k) for k in range(2)]
+    batch = BatchedChannels(meshes)
+    rng = np.random.default_rng(3)
+    x = np.concatenate([m.nodes[:, 0] for m in meshes])
+    phi = torch.from_numpy(1.1 * x + 0.02 * rng.standard_normal(len(x))).cuda()
+    batch.evaluate(phi, [0.8, 0.7], jacobian=False)          # air
+    side, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        batch.evaluate(phi, None, jacobian=False)
+        graph.capture_begin()
+        try:
+            batch.evaluate(phi, None, jacobian=False)
+        finally:
+            graph.capture_end()
+    torch.cuda.current_stream().wait_stream(side)
+    flows = (L.Flow * 2)(*[FlowParams(m_inf=m, gamma=g).c() for m, g in zip((0.8, 0.7), gammas)])
+    batch._flows = lambda machs: flows
+    direct = batch.evaluate(phi, [0.8, 0.7], jacobian=False).clone()
+    batch.ws.ev.R.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    scale = direct.abs().max()
+    assert float((batch.ws.ev.R - direct).abs().max()) <= 1e-14 * float(scale)

@@ -378,7 +378,7 @@ __device__ __forceinline__ void slab_done(int lane) {  // written, before the bl
 // FP64 pipe 32 %, load/store wavefronts 68 % busy), so registers and
 // wavefronts are what pays: 304 us with int64 ids and pow, 287 with neither,
 // 275 without the switch of subcritical pairs, 264 with the records stored in
-// bulk; residual only 238 -> 214.  14.7 M tets: 1187 -> 1092 us.  Tried and
+// bulk; residual only 238 -> 211.  14.7 M tets: 1187 -> 1092 us.  Tried and
 // slower: the walk as a kernel of its own (297), B_e kept in the slab instead
 // of formed again (259 against 256, residual only 230 against 214), the next
 // tile's records prefetched into L2 (256 at 3.6 M, but 1240 at 14.7 M).
@@ -1700,13 +1700,16 @@ static void launch_sweep_mb(const up3d_mesh* m, cudaStream_t s, A... args) {
     UP3D_CHECK_LAUNCH();
 }
 
+constexpr int64_t SWEEP_LARGE = 2'000'000;
 template <bool FR, bool JA, bool BA, bool AIR, class... A>
 static void launch_sweep_air(const up3d_mesh* m, cudaStream_t s, A... args) {
-    // residual only: air fits 72 registers without a spill; with the walk 28
-    // warps per SM are fastest (3.6 M tets: 24 warps 218 us, 28 warps 211 us),
-    // without it 24 (0.43 M: 21.9 and 22.5 us)
-    if (!JA) return !AIR ? launch_sweep_mb<FR, JA, BA, AIR, 256, 3>(m, s, args...)
-                         : launch_sweep_mb<FR, JA, BA, AIR, 128, FR ? 6 : 7>(m, s, args...);
+    // residual only: on a large mesh of air 28 warps per SM are fastest (72
+    // registers, no spill); on one of a few waves of blocks 24 warps, and then
+    // the form for any gas (the whole call, walk / frozen: 3.6 M tets 269 / 187
+    // against 272 / 193 us, 0.97 M 86.1 / 57.6 and 84.7 / 57.9, 0.45 M 45.2 /
+    // 29.6 against 43.2 / 28.6)
+    if (!JA) return AIR && m->E >= SWEEP_LARGE ? launch_sweep_mb<FR, JA, BA, AIR, 128, 7>(m, s, args...)
+                                               : launch_sweep_mb<FR, JA, BA, false, 256, 3>(m, s, args...);
     switch (m->tune.elem_threads_per_sm) {
         case 640: launch_sweep_mb<FR, JA, BA, AIR, 128, 5>(m, s, args...); break;
         case 768: launch_sweep_mb<FR, JA, BA, AIR, 128, 6>(m, s, args...); break;
@@ -1837,7 +1840,15 @@ static void fused_evaluate(up3d_mesh* m, const double* phi, const Flow& F, doubl
                            int8_t* br_out = nullptr, int n_cases = 0) {
     up3d_monitors* mo = mon ? mon : m->mon_ws.get();
     UP3D_CUDA(cudaMemsetAsync(mo, 0, sizeof(up3d_monitors), s));
-    const bool jac = data != nullptr, air = flows_d ? m->batch_air : F.air;
+    const bool jac = data != nullptr;
+    // a captured launch reads whatever flow table is there when it is
+    // replayed: only a direct one may count on the table's gamma
+    bool air = F.air;
+    if (flows_d) {
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        if (m->batch_air) UP3D_CUDA(cudaStreamIsCapturing(s, &capture));
+        air = m->batch_air && capture == cudaStreamCaptureStatusNone;
+    }
     // the walk's result goes straight to the caller's buffer when there is
     // one (Term 3 reads it from there), else to the mesh workspace
     int32_t* up_dst = up_out ? up_out : m->up32.get();

@@ -5,11 +5,11 @@
 //
 // Vectors live on the device; each iteration's scalars (dots, norms) are
 // reduced on the device with a fixed two-pass tree (bit-reproducible) and
-// read back once per iteration for the convergence test.  GMRES follows
+// reach the host once per iteration for the convergence test.  GMRES follows
 // scipy's algorithm (left preconditioning, Givens rotations, adaptive inner
 // tolerance, true-residual test after every cycle) with classical
 // Gram-Schmidt applied twice (CGS2) in place of modified Gram-Schmidt, so
-// each Arnoldi step is two batched multi-dot / multi-axpy passes.
+// each Arnoldi step is three sweeps over the basis.
 
 #include <cmath>
 #include <mutex>
