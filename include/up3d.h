@@ -223,9 +223,19 @@ int up3d_jacobian_export(up3d_mesh* mesh, const double* data, int32_t* indptr,
 
 /* The same with newton_nnz read back (synchronous), for callers that size
  * indices and merged by the most there can be: the P1 nnz plus the extras
- * (up3d_monitors.n_term3_extra, or up3d_jacobian's n_extra). */
+ * (up3d_monitors.n_term3_extra, or up3d_jacobian's n_extra).  The extras
+ * are the mesh's, of whichever call formed a Jacobian on it last: nothing
+ * past `capacity` entries is written (UP3D_ERR_VALUE when there are more),
+ * and UP3D_ERR_RUNTIME when `serial` is not the mesh's serial number any
+ * more (its value after the call that formed `data`; -1: not checked). */
 int up3d_jacobian_merge(up3d_mesh* mesh, const double* data, int32_t* indptr, int32_t* indices,
-                        double* merged, int64_t* newton_nnz, up3d_stream stream);
+                        double* merged, int64_t capacity, int64_t serial, int64_t* newton_nnz,
+                        up3d_stream stream);
+
+/* The mesh's count of Jacobians formed on it (up3d_jacobian,
+ * up3d_residual_jacobian[_batched] with data): a host word, valid while the
+ * mesh is. */
+int up3d_jacobian_serial(const up3d_mesh* mesh, const int64_t** serial);
 
 /* newton_nnz of the last Jacobian (kernels/jacobian.py:358): the P1 nnz, or,
  * when Term 3 is active, the non-zeros of the merged matrix.  Synchronous. */

@@ -106,7 +106,8 @@ SIGNATURES = {
     "up3d_jacobian_data": (_int, [_p, _p, _p, _p, _p, _p, _d, _p, _p, ctypes.POINTER(_i64),
                              ctypes.POINTER(_i64), ctypes.POINTER(_i64), _p]),
     "up3d_jacobian_export": (_int, [_p, _p, _p, _p, _p, _p]),
-    "up3d_jacobian_merge": (_int, [_p, _p, _p, _p, _p, ctypes.POINTER(_i64), _p]),
+    "up3d_jacobian_merge": (_int, [_p, _p, _p, _p, _p, _i64, _i64, ctypes.POINTER(_i64), _p]),
+    "up3d_jacobian_serial": (_int, [_p, ctypes.POINTER(_p)]),
     "up3d_jacobian_nnz": (_int, [_p, _p, ctypes.POINTER(_i64), _p]),
     "up3d_residual_jacobian": (_int, [_p, _p, ctypes.POINTER(Flow), _p, _p, _p, _p, _p, _p, _p, _p]),
     "up3d_residual_vjp": (_int, [_p, _p, ctypes.POINTER(Flow), _p, _p, _p, _p, _p, _p, _p, _p]),

@@ -1292,14 +1292,14 @@ __global__ void k_count_nonzero(const double* __restrict__ v, int64_t n, unsigne
 // Eight lanes per row, eight entries at a time: an entry's place is the kept
 // entries of its own list before it (a ballot) plus the kept entries of the
 // other list in lower columns (eight shuffles per chunk; dropped entries
-// stand as column INT32_MAX).  One thread per row, merging serially, took
+// stand as column INT32_MAX).  Entries past `capacity` are not written.  One thread per row, merging serially, took
 // 187 us for the fill on the 625 k-row Jacobian.
 template <bool FILL>
 __global__ void __launch_bounds__(256)
     k_merge_rows(int64_t N, const int32_t* __restrict__ indptr, const int32_t* __restrict__ indices,
                  const double* __restrict__ data, const int32_t* __restrict__ xptr, const int32_t* __restrict__ xcol,
                  const double* __restrict__ xval, bool drop_zeros, int32_t* __restrict__ out_ptr,
-                 int32_t* __restrict__ out_idx, double* __restrict__ out_val) {
+                 int32_t* __restrict__ out_idx, double* __restrict__ out_val, int64_t capacity) {
     constexpr int G = 8, RPW = 32 / G;
     const int lane = threadIdx.x & 31, sub = lane & (G - 1), shift = lane & ~(G - 1);
     const unsigned below = (1u << sub) - 1u;
@@ -1348,7 +1348,7 @@ __global__ void __launch_bounds__(256)
                 if (FILL) {
                     int place = before + __popc(m & below);
                     if (most2 > 0) place += lower(col2, val2, o2, len2, most2, c);
-                    if (keep) {
+                    if (keep && out + place < capacity) {
                         out_idx[out + place] = c;
                         out_val[out + place] = v;
                     }
@@ -1422,6 +1422,7 @@ static void build_term3(up3d_mesh* m, double* data, cudaStream_t s, int64_t& n_a
     const int64_t E = m->E, N = m->N, Z = m->nnz;
     n_extra = 0;
     m->last_extra = 0;
+    m->jac_serial += 1;
     m->i64_ws.alloc(8);
     n_active = known_active;
     m->last_active = n_active;
@@ -1537,9 +1538,10 @@ static void build_term3(up3d_mesh* m, double* data, cudaStream_t s, int64_t& n_a
     m->t3c_extra = n_extra;
 }
 
-// The merged CSR of the last Jacobian.
+// The merged CSR of the last Jacobian; at most `capacity` entries of indices
+// and merged are written.
 static void export_merged(up3d_mesh* m, const double* data, int32_t* indptr, int32_t* indices, double* merged,
-                          cudaStream_t s) {
+                          int64_t capacity, cudaStream_t s) {
     UP3D_REQUIRE(m && data && indptr && indices && merged, UP3D_ERR_ARGUMENT,
                  "up3d_jacobian_export: null argument");
     const bool has_x = m->last_extra > 0;
@@ -1550,12 +1552,12 @@ static void export_merged(up3d_mesh* m, const double* data, int32_t* indptr, int
     const unsigned grid = grid_for(m->N, 32, (int64_t)m->n_sms * 64);
     k_merge_rows<false><<<grid, 256, 0, s>>>(m->N, m->indptr.get(), m->indices.get(), data, xptr,
                                                            m->x_col_c.get(), m->x_val_c.get(),
-                                                           m->last_drop_zeros, cnt, nullptr, nullptr);
+                                                           m->last_drop_zeros, cnt, nullptr, nullptr, 0);
     UP3D_CHECK_LAUNCH();
     scan(m, cnt, indptr, m->N + 1, s);
     k_merge_rows<true><<<grid, 256, 0, s>>>(m->N, m->indptr.get(), m->indices.get(), data, xptr,
                                                           m->x_col_c.get(), m->x_val_c.get(),
-                                                          m->last_drop_zeros, indptr, indices, merged);
+                                                          m->last_drop_zeros, indptr, indices, merged, capacity);
     UP3D_CHECK_LAUNCH();
 }
 
@@ -1646,15 +1648,26 @@ int up3d_jacobian_data(up3d_mesh* m, const double* phi, const double* rt, const 
 
 int up3d_jacobian_export(up3d_mesh* m, const double* data, int32_t* indptr, int32_t* indices, double* merged,
                          up3d_stream stream) {
-    return guarded([&] { export_merged(m, data, indptr, indices, merged, S(stream)); });
+    return guarded([&] { export_merged(m, data, indptr, indices, merged, INT64_MAX, S(stream)); });
 }
 
 int up3d_jacobian_merge(up3d_mesh* m, const double* data, int32_t* indptr, int32_t* indices, double* merged,
-                        int64_t* newton_nnz, up3d_stream stream) {
+                        int64_t capacity, int64_t serial, int64_t* newton_nnz, up3d_stream stream) {
     return guarded([&] {
-        UP3D_REQUIRE(newton_nnz, UP3D_ERR_ARGUMENT, "up3d_jacobian_merge: null argument");
-        export_merged(m, data, indptr, indices, merged, S(stream));
+        UP3D_REQUIRE(m && newton_nnz, UP3D_ERR_ARGUMENT, "up3d_jacobian_merge: null argument");
+        UP3D_REQUIRE(serial < 0 || serial == m->jac_serial, UP3D_ERR_RUNTIME,
+                     "up3d_jacobian_merge: another Jacobian was formed on the mesh since; evaluate again");
+        export_merged(m, data, indptr, indices, merged, capacity, S(stream));
         *newton_nnz = read_back(indptr + m->N, S(stream));
+        UP3D_REQUIRE(*newton_nnz <= capacity, UP3D_ERR_VALUE,
+                     "up3d_jacobian_merge: the merged matrix has more entries than the arrays hold");
+    });
+}
+
+int up3d_jacobian_serial(const up3d_mesh* m, const int64_t** serial) {
+    return guarded([&] {
+        UP3D_REQUIRE(m && serial, UP3D_ERR_ARGUMENT, "up3d_jacobian_serial: null argument");
+        *serial = &m->jac_serial;
     });
 }
 

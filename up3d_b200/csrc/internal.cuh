@@ -242,6 +242,7 @@ struct up3d_mesh {
     up3d::DBuf<int64_t> i64_ws;        // small scalars
     int64_t last_extra = 0;            // extras of the last Jacobian
     int64_t last_active = 0;
+    int64_t jac_serial = 0;            // Jacobians formed on the mesh: whose extras these are
     bool last_drop_zeros = false;
 };
 

@@ -161,6 +161,7 @@ class PicardOperator:
         L.call("up3d_jacobian", self._mesh.handle, d_phi.data_ptr(), d_rt.data_ptr(), d_se.data_ptr(),
                d_su.data_ptr(), d_up.data_ptr(), float(u_inf), L.ptr(d_lim), data.data_ptr(),
                ctypes.byref(na), ctypes.byref(nx), None, L.stream_ptr())
+        serial = self._mesh.jacobian_serial.value
         self.n_term3_active = int(na.value)
         self.n_term3_extra = int(nx.value)
         if self.n_term3_active == 0:
@@ -174,7 +175,7 @@ class PicardOperator:
         merged = t.empty(most, dtype=t.float64, device="cuda")
         nnz = ctypes.c_int64()
         L.call("up3d_jacobian_merge", self._mesh.handle, data.data_ptr(), indptr.data_ptr(),
-               indices.data_ptr(), merged.data_ptr(), ctypes.byref(nnz), L.stream_ptr())
+               indices.data_ptr(), merged.data_ptr(), most, serial, ctypes.byref(nnz), L.stream_ptr())
         self.newton_nnz = int(nnz.value)
         indices, merged = indices[:self.newton_nnz], merged[:self.newton_nnz]
         return self._csr_result(indptr, indices, merged, host)

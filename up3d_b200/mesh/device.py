@@ -73,6 +73,9 @@ class DeviceMesh:
         self.indptr = device_view(ip.value, (self.n_nodes + 1,), np.int32).clone()
         self.indices = device_view(ix.value, (self.nnz,), np.int32).clone()
         self._colors = None
+        serial = ctypes.c_void_p()
+        L.call("up3d_jacobian_serial", self.handle, ctypes.byref(serial))
+        self.jacobian_serial = ctypes.c_int64.from_address(serial.value)   # Jacobians formed so far
 
     def __del__(self):
         h = getattr(self, "handle", None)

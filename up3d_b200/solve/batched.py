@@ -114,6 +114,8 @@ class BatchedChannels:
                L.ptr(self.up_fz), L.ptr(self.br_fz),
                ev.R.data_ptr(), ev.data.data_ptr() if jacobian else None, ev.rho_tilde.data_ptr(),
                ev.upstream.data_ptr(), self.branch.data_ptr(), ev.monitors.data_ptr(), L.stream_ptr())
+        if jacobian:
+            ev._serial = ev.mesh.jacobian_serial.value
         return ev.R
 
     def case_phi(self, phi, c: int):

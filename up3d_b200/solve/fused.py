@@ -46,6 +46,7 @@ class ResidualJacobian:
         self.upstream = t.empty(mesh.n_tets, dtype=t.int32, device="cuda")
         self.monitors = L.monitors_buffer()
         self._n_extra = 0
+        self._serial = -1   # the mesh's Jacobian that `data` is
         if mesh.tuning()["assembly"] == 1:
             mesh.tile_info()  # the tile plan now, not inside a timed solve
 
@@ -69,13 +70,17 @@ class ResidualJacobian:
                self.rho_tilde.data_ptr() if keep_state is True else None,
                self.upstream.data_ptr() if keep_state else None,
                self.monitors.data_ptr(), L.stream_ptr())
+        if jacobian:
+            self._serial = self.mesh.jacobian_serial.value
         return R
 
     def read_monitors(self) -> dict:
         return L.read_monitors(self.monitors)
 
     def jacobian(self, newton_nnz: int | None = None) -> DeviceCSR:
-        """The merged Newton Jacobian of the last evaluate(jacobian=True)."""
+        """The merged Newton Jacobian of the last evaluate(jacobian=True).
+        Its entries outside the P1 pattern are in the mesh's workspace:
+        RuntimeError when another Jacobian was formed on the mesh since."""
         t = L.torch()
         mon = self.read_monitors()
         if mon["n_term3_active"] == 0:
@@ -89,7 +94,7 @@ class ResidualJacobian:
         data = t.empty(most, dtype=t.float64, device="cuda")
         nnz = ctypes.c_int64()
         L.call("up3d_jacobian_merge", self.mesh.handle, self.data.data_ptr(), indptr.data_ptr(),
-               indices.data_ptr(), data.data_ptr(), ctypes.byref(nnz), L.stream_ptr())
+               indices.data_ptr(), data.data_ptr(), most, self._serial, ctypes.byref(nnz), L.stream_ptr())
         if newton_nnz is None:
             indices, data = indices[:nnz.value], data[:nnz.value]
         return DeviceCSR(indptr, indices, data, (self.mesh.n_nodes, self.mesh.n_nodes))
