@@ -13,7 +13,8 @@
 //   pass 1 (per element e): c_e = V_e (g_e . h_e), h_e = sum_i lam_i B_e,i;
 //     t_e = c_e s_e + w_e (weight on q2_e), a_e = c_e s_u (weight on q2 of
 //     u(e)), and c_e d rho~_e / dM by forward-mode differentiation;
-//   the a_e are chained per upstream element and summed in integers;
+//   the a_e are chained per upstream element and summed in integers
+//     (exact_sum.cuh);
 //   pass 2 (per element k): dL/dB_k,j = rho~ V (phi_j h + lam_j g)
 //     + Q_k (2/u^2) phi_j g with Q_k = t_k + sum a, dL/dV_k = rho~ (g . h),
 //     then through B = D^-1 (rows), V = |det D| / 6 with D = [x1-x0, x2-x0,
@@ -22,6 +23,7 @@
 // Everything is deterministic (no atomics on values).
 
 #include "elem.cuh"
+#include "exact_sum.cuh"
 #include "internal.cuh"
 
 namespace up3d {
@@ -132,7 +134,7 @@ __global__ void __launch_bounds__(256, AIR ? 3 : 2)
                const int64_t* __restrict__ up, const int8_t* __restrict__ br, int64_t E,
                const double* __restrict__ lam, const double* __restrict__ w, double* __restrict__ t_out,
                double* __restrict__ a_out, double* __restrict__ rt_out, int32_t* __restrict__ head,
-               int32_t* __restrict__ next, double* __restrict__ partial) {
+               int32_t* __restrict__ next, int32_t* __restrict__ top, double* __restrict__ partial) {
     __shared__ double sh[8];
     F.air = FM.air = AIR;
     double dm = 0.0;
@@ -185,6 +187,7 @@ __global__ void __launch_bounds__(256, AIR ? 3 : 2)
         if (a != 0.0) {   // into the chain of u
             a_out[e] = a;
             next[e] = atomicExch(head + u, (int32_t)e);
+            atomicMax(top + u, exponent_field(a));
         }
     }
     dm = warp_sum(dm);
@@ -205,27 +208,33 @@ __global__ void k_vjp_sum_partials(const double* __restrict__ partial, int nb, d
     if (threadIdx.x == 0) *out = s;
 }
 
-// Sum of a_e over the chain starting at element i (in whatever order the
-// chain was built): the values as integers on a scale that gives the
-// largest 62 bits, added in 128 bits, so the sum is exact to 2^-62 of the
-// largest and the same for every order.  A stable sort by upstream element
-// and per-run sums, in its place, took 50 of the 283 us of a residual forward
-// and backward at 450 k tets.
-__device__ __forceinline__ double chain_sum(const int32_t* __restrict__ next, const double* __restrict__ a, int32_t i) {
-    if (i < 0) return 0.0;
-    const double first = a[i];
-    if (next[i] < 0) return first;
-    double big = 0.0, plain = 0.0;
-    for (int32_t j = i; j >= 0; j = next[j]) {
-        big = fmax(big, fabs(a[j]));
-        plain += a[j];
+// Sum of a_e over the chain of element k, in whatever order the chain was
+// built: up to two terms as they are, longer chains by ExactSum, the same
+// bits for every order.  `top` holds the largest exponent field of each
+// chain, so that it is walked once: bound by a dependent load per link (0.45 M
+// elements on one chain: a stable sort by upstream element and the sums of its
+// runs 65 ms, a walk for the largest and one for the sum 89 ms, this 47 ms).
+// The sort took 50 of the 283 us of a residual forward and backward at 450 k
+// tets.
+__device__ __forceinline__ double chain_sum(const int32_t* __restrict__ head, const int32_t* __restrict__ next,
+                                            const int32_t* __restrict__ top, const double* __restrict__ a,
+                                            int64_t k) {
+    int32_t j = head[k];
+    if (j < 0) return 0.0;
+    const double first = a[j];
+    if ((j = next[j]) < 0) return first;
+    double v = a[j];
+    if ((j = next[j]) < 0) return first + v;
+    ExactSum sum(top[k]);
+    sum.add(first);
+    while (j >= 0) {   // the next link is on its way while this term is added
+        const double ahead = a[j];
+        j = next[j];
+        sum.add(v);
+        v = ahead;
     }
-    if (!(big > 0.0 && big < INFINITY && plain - plain == 0.0)) return plain;   // infinities and NaN propagate
-    const int shift = 61 - ilogb(big);
-    __int128 sum = 0;
-    for (int32_t j = i; j >= 0; j = next[j]) sum += (long long)rint(ldexp(a[j], shift));
-    const double hi = (double)(long long)(sum >> 64), lo = (double)(unsigned long long)sum;
-    return ldexp(hi * 18446744073709551616.0 + lo, -shift);
+    sum.add(v);
+    return sum.value();
 }
 
 // Pass 2: per element, dL/dB and dL/dV through the inverse edge matrix to
@@ -234,8 +243,8 @@ __global__ void __launch_bounds__(256)
     k_vjp_geom(const int4* __restrict__ conn, const double* __restrict__ B, const double* __restrict__ V,
                const double* __restrict__ phi, double u2, int64_t E, const double* __restrict__ lam,
                const double* __restrict__ w, const double* __restrict__ t, const double* __restrict__ a,
-               const int32_t* __restrict__ head, const int32_t* __restrict__ next, const double* __restrict__ rt,
-               double* __restrict__ dx, double* __restrict__ dphi) {
+               const int32_t* __restrict__ head, const int32_t* __restrict__ next,
+               const int32_t* __restrict__ top, const double* __restrict__ rt, double* __restrict__ dx, double* __restrict__ dphi) {
     GRID_STRIDE(e, E) {
         double g[3], b[12];
         int4 c;
@@ -250,7 +259,7 @@ __global__ void __launch_bounds__(256)
             l[3] = lam[c.w];
         }
         const double Ve = V[e], r = rt[e];
-        const double Q = t[e] + chain_sum(next, a, head[e]);
+        const double Q = t[e] + chain_sum(head, next, top, a, e);
         const double q2w = 2.0 * Q / u2;
         double G[4][3];
 #pragma unroll
@@ -372,23 +381,25 @@ int up3d_residual_vjp(up3d_mesh* m, const double* phi, const up3d_flow* flow, co
         m->adj_rt.alloc(E);
         m->adj_dx.alloc(12 * E);
         m->adj_dphi.alloc(4 * E);
-        m->adj_head.alloc(E);
+        m->adj_head.alloc(2 * E);
         m->adj_next.alloc(E);
+        int32_t* head = m->adj_head.get();
+        int32_t* top = head + E;
         const unsigned grid = grid_for(E, 256, (int64_t)148 * 8);
         m->adj_part.alloc(grid + 1);
-        UP3D_CUDA(cudaMemsetAsync(m->adj_head.get(), 0xff, sizeof(int32_t) * E, s));   // -1: empty chains
+        UP3D_CUDA(cudaMemsetAsync(head, 0xff, sizeof(int32_t) * 2 * E, s));   // -1: empty chains
         auto elem = F.air ? k_vjp_elem<true> : k_vjp_elem<false>;
         elem<<<grid, 256, 0, s>>>(m->conn.get(), m->B.get(), m->V.get(), phi, F, FM, flow->m_inf, u2,
                                         upstream, branch, E, lam, w_q2, m->adj_t.get(), m->adj_a.get(),
-                                        m->adj_rt.get(), m->adj_head.get(), m->adj_next.get(), m->adj_part.get());
+                                        m->adj_rt.get(), head, m->adj_next.get(), top, m->adj_part.get());
         UP3D_CHECK_LAUNCH();
         if (dM) {
             k_vjp_sum_partials<<<1, 32, 0, s>>>(m->adj_part.get(), (int)grid, dM);
             UP3D_CHECK_LAUNCH();
         }
         k_vjp_geom<<<grid_for(E, 256), 256, 0, s>>>(m->conn.get(), m->B.get(), m->V.get(), phi, u2, E, lam, w_q2,
-                                                    m->adj_t.get(), m->adj_a.get(), m->adj_head.get(),
-                                                    m->adj_next.get(), m->adj_rt.get(),
+                                                    m->adj_t.get(), m->adj_a.get(), head,
+                                                    m->adj_next.get(), top, m->adj_rt.get(),
                                                     m->adj_dx.get(), dphi ? m->adj_dphi.get() : nullptr);
         UP3D_CHECK_LAUNCH();
         if (dX || dphi) {

@@ -236,7 +236,7 @@ struct up3d_mesh {
     up3d::DBuf<double> adj_dx;                        // (E, 12) per-element node gradients
     up3d::DBuf<double> adj_dphi;                      // (E, 4)
     up3d::DBuf<double> adj_part;                      // reduction partials
-    up3d::DBuf<int32_t> adj_head, adj_next;           // (E) each: chains of elements per upstream element
+    up3d::DBuf<int32_t> adj_head, adj_next;           // (2E: chain heads, largest exponents), (E): elements per upstream element
     up3d::DBuf<up3d::Flow> flows_ws;   // per-case flows of batched evaluations
     up3d::DBuf<up3d_monitors> mon_ws;  // (1)
     up3d::DBuf<int64_t> i64_ws;        // small scalars
