@@ -296,7 +296,9 @@ int up3d_face_normals(const up3d_mesh* mesh, double* out, up3d_stream stream);
  * within `depth` face hops of each element, itself excluded, ascending;
  * built once per depth and kept on the mesh (rebuilt after
  * up3d_mesh_set_face_neighbors).  Device views of the CSR (offsets int64
- * n_tets + 1, indices int32) and the total; any output may be NULL.
+ * n_tets + 1, indices int32; they hold until another depth is built) and
+ * the total; any output may be NULL.  The indices are kept beside the form
+ * the density sweep reads only where they were asked for.
  * Depths up to 4 (at most 160 elements) are built on the device, deeper
  * ones on the host (OpenMP breadth-first search) and uploaded.
  * UP3D_ERR_VALUE for depth < 1.  Synchronises the stream when it builds. */

@@ -167,8 +167,8 @@ struct up3d_mesh {
     // face-hop neighbourhoods of the weighted "kernel" upwind mode (built on
     // request; nb_depth 0 = none)
     up3d::DBuf<int64_t> nb_off;  // (E+1)
-    up3d::DBuf<int32_t> nb_idx;  // (nb_total) ascending per element
-    // the same lists in slices of 32 elements: neighbour j of element 32 q +
+    up3d::DBuf<int32_t> nb_idx;  // (nb_total) lists, ascending per element; only once exported
+    // the lists in slices of 32 elements: neighbour j of element 32 q +
     // lane at nb_sp[q] + 32 j + lane, -1 past the element's last
     up3d::DBuf<int64_t> nb_sp;   // (ceil(E / 32) + 1)
     up3d::DBuf<int32_t> nb_si;

@@ -84,8 +84,11 @@ __global__ void k_face_normals(const int4* __restrict__ conn, const double4* __r
 // build_upstream_neighborhoods (kernels/upwind.py:313-341): the elements
 // within `depth` face hops of e, e excluded, ascending.  Breadth-first in
 // a per-thread list whose levels are its own frontiers; the list is then
-// insertion-sorted.  Count pass (cnt[e]) or fill pass (idx from off).
-template <bool FILL>
+// insertion-sorted.  Count pass (cnt[e]), or a fill pass: lists (idx from
+// off[e]), or the slices of k_rho_tilde_kernel (off: start of each 32
+// elements; interleaved, padded with -1).
+enum NbPass { NB_COUNT, NB_LISTS, NB_SLICES };
+template <NbPass PASS>
 __global__ void __launch_bounds__(128)
     k_neighborhoods(const int4* __restrict__ fn, int64_t E, int depth, int64_t* __restrict__ cnt,
                     const int64_t* __restrict__ off, int32_t* __restrict__ idx) {
@@ -108,7 +111,7 @@ __global__ void __launch_bounds__(128)
             lo = hi;
             hi = ns;
         }
-        if constexpr (!FILL) {
+        if constexpr (PASS == NB_COUNT) {
             cnt[e] = ns - 1;
         } else {
             for (int i = 2; i < ns; ++i) {
@@ -120,8 +123,14 @@ __global__ void __launch_bounds__(128)
                 }
                 seen[j + 1] = v;
             }
-            int32_t* out = idx + off[e];
-            for (int i = 1; i < ns; ++i) out[i - 1] = seen[i];
+            if constexpr (PASS == NB_LISTS) {
+                int32_t* out = idx + off[e];
+                for (int i = 1; i < ns; ++i) out[i - 1] = seen[i];
+            } else {
+                const int64_t q = e >> 5, s = off[q] + (e & 31);
+                const int w = (int)((off[q + 1] - off[q]) >> 5);
+                for (int j = 0; j < w; ++j) idx[s + 32 * (int64_t)j] = j + 1 < ns ? seen[j + 1] : -1;
+            }
         }
     }
 }
@@ -142,8 +151,8 @@ __device__ __forceinline__ void stream_extent(const int4 c, const double4* __res
     }
 }
 
-// Longest neighbourhood of each slice of 32 elements (times 32), and the
-// slices filled from the lists.
+// Longest neighbourhood of each slice of 32 elements (times 32), the slices
+// filled from lists, and lists read out of the slices.
 __global__ void k_slice_widths(int64_t E, const int64_t* __restrict__ nb_off, int64_t* __restrict__ width) {
     GRID_STRIDE(e, (E + 31) / 32 * 32) {   // whole warps
         const int n = e < E ? (int)(nb_off[e + 1] - nb_off[e]) : 0;
@@ -159,6 +168,14 @@ __global__ void k_slice_fill(int64_t E, const int64_t* __restrict__ nb_off, cons
         const int64_t o = e < E ? nb_off[e] : 0;
         const int n = e < E ? (int)(nb_off[e + 1] - o) : 0;
         for (int j = 0; j < w; ++j) si[s + 32 * (int64_t)j] = j < n ? nb_idx[o + j] : -1;
+    }
+}
+__global__ void k_slice_lists(int64_t E, const int64_t* __restrict__ nb_off, const int64_t* __restrict__ sp,
+                              const int32_t* __restrict__ si, int32_t* __restrict__ nb_idx) {
+    GRID_STRIDE(e, E) {
+        const int64_t s = sp[e >> 5] + (e & 31), o = nb_off[e];
+        const int n = (int)(nb_off[e + 1] - o);
+        for (int j = 0; j < n; ++j) nb_idx[o + j] = si[s + 32 * (int64_t)j];
     }
 }
 
@@ -383,7 +400,7 @@ static int64_t neighborhood_offsets(const int4* fn, int64_t E, int depth, int64_
                                     cudaStream_t s) {
     DBuf<int64_t> cnt;
     cnt.alloc(E);
-    k_neighborhoods<false><<<grid_for(E, 128), 128, 0, s>>>(fn, E, depth, cnt.get(), nullptr, nullptr);
+    k_neighborhoods<NB_COUNT><<<grid_for(E, 128), 128, 0, s>>>(fn, E, depth, cnt.get(), nullptr, nullptr);
     UP3D_CHECK_LAUNCH();
     UP3D_CUDA(cudaMemsetAsync(off, 0, sizeof(int64_t), s));
     size_t bytes = 0;
@@ -396,8 +413,9 @@ static int64_t neighborhood_offsets(const int4* fn, int64_t E, int depth, int64_
     return total;
 }
 
-// The slices of the mesh's neighbourhood lists.  Synchronises the stream.
-static void neighborhood_slices(up3d_mesh* m, DBuf<unsigned char>& tmp, cudaStream_t s) {
+// Offsets of the slices of the lists with offsets nb_off, and room for the
+// slices.  Synchronises the stream.
+static void slice_offsets(up3d_mesh* m, DBuf<unsigned char>& tmp, cudaStream_t s) {
     const int64_t E = m->E, nq = (E + 31) / 32;
     m->nb_sp.alloc(nq + 1);
     UP3D_CUDA(cudaMemsetAsync(m->nb_sp.get(), 0, sizeof(int64_t), s));
@@ -414,31 +432,47 @@ static void neighborhood_slices(up3d_mesh* m, DBuf<unsigned char>& tmp, cudaStre
     UP3D_CUDA(cudaMemcpyAsync(&total, m->nb_sp.get() + nq, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
     UP3D_CUDA(cudaStreamSynchronize(s));
     m->nb_si.alloc(total > 0 ? total : 1);
-    k_slice_fill<<<grid_for(E, 256), 256, 0, s>>>(E, m->nb_off.get(), m->nb_idx.get(), m->nb_sp.get(), m->nb_si.get());
-    UP3D_CHECK_LAUNCH();
-    UP3D_CUDA(cudaStreamSynchronize(s));
 }
 
-// Builds (or reuses) the mesh's neighbourhood CSR of the given depth, and
-// its slices.  Synchronises the stream (the totals size the index arrays).
+// Builds (or reuses) the mesh's neighbourhoods of the given depth: offsets
+// and slices (the lists themselves are 132 bytes an element at depth 3, kept
+// only for who asks for them: neighborhood_lists).  Synchronises the stream
+// (the totals size the arrays).
 void ensure_neighborhoods(up3d_mesh* m, int depth, cudaStream_t s) {
     if (m->nb_depth == depth) return;
     const int64_t E = m->E;
     m->nb_depth = 0;
+    m->nb_idx.release();
     m->nb_off.alloc(E + 1);
     DBuf<unsigned char> tmp;
     if (depth > NB_MAX_DEPTH) {
-        m->nb_total = neighborhoods_host(m->fnbr.get(), E, depth, m->nb_off.get(), &m->nb_idx, nullptr, s);
-    } else {
-        const int64_t total = neighborhood_offsets(m->fnbr.get(), E, depth, m->nb_off.get(), tmp, s);
-        m->nb_idx.alloc(total > 0 ? total : 1);
-        k_neighborhoods<true><<<grid_for(E, 128), 128, 0, s>>>(m->fnbr.get(), E, depth, nullptr, m->nb_off.get(),
-                                                              m->nb_idx.get());
+        DBuf<int32_t> idx;
+        m->nb_total = neighborhoods_host(m->fnbr.get(), E, depth, m->nb_off.get(), &idx, nullptr, s);
+        slice_offsets(m, tmp, s);
+        k_slice_fill<<<grid_for(E, 256), 256, 0, s>>>(E, m->nb_off.get(), idx.get(), m->nb_sp.get(), m->nb_si.get());
         UP3D_CHECK_LAUNCH();
-        m->nb_total = total;
+        UP3D_CUDA(cudaStreamSynchronize(s));   // idx goes
+    } else {
+        m->nb_total = neighborhood_offsets(m->fnbr.get(), E, depth, m->nb_off.get(), tmp, s);
+        slice_offsets(m, tmp, s);
+        k_neighborhoods<NB_SLICES><<<grid_for(E, 128), 128, 0, s>>>(m->fnbr.get(), E, depth, nullptr, m->nb_sp.get(),
+                                                                   m->nb_si.get());
+        UP3D_CHECK_LAUNCH();
+        UP3D_CUDA(cudaStreamSynchronize(s));
     }
-    neighborhood_slices(m, tmp, s);
     m->nb_depth = depth;
+}
+
+// The lists of the built neighbourhoods (until another depth is built).
+static const int32_t* neighborhood_lists(up3d_mesh* m, cudaStream_t s) {
+    if (!m->nb_idx.get()) {
+        m->nb_idx.alloc(m->nb_total > 0 ? m->nb_total : 1);
+        k_slice_lists<<<grid_for(m->E, 256), 256, 0, s>>>(m->E, m->nb_off.get(), m->nb_sp.get(), m->nb_si.get(),
+                                                         m->nb_idx.get());
+        UP3D_CHECK_LAUNCH();
+        UP3D_CUDA(cudaStreamSynchronize(s));
+    }
+    return m->nb_idx.get();
 }
 
 }  // namespace up3d
@@ -462,7 +496,7 @@ int up3d_mesh_neighborhoods(up3d_mesh* m, int depth, const int64_t** offsets, co
         UP3D_REQUIRE(depth >= 1, UP3D_ERR_VALUE, "up3d_mesh_neighborhoods: depth must be >= 1");
         ensure_neighborhoods(m, depth, S(stream));
         if (offsets) *offsets = m->nb_off.get();
-        if (indices) *indices = m->nb_idx.get();
+        if (indices) *indices = neighborhood_lists(m, S(stream));
         if (total) *total = m->nb_total;
     });
 }
@@ -494,7 +528,7 @@ int up3d_face_neighborhoods(const int32_t* fn, int64_t n, int depth, int64_t* of
             neighborhoods_host(f4, n, depth, offsets, nullptr, indices, s);
             return;
         }
-        k_neighborhoods<true><<<grid_for(n, 128), 128, 0, s>>>(f4, n, depth, nullptr, offsets, indices);
+        k_neighborhoods<NB_LISTS><<<grid_for(n, 128), 128, 0, s>>>(f4, n, depth, nullptr, offsets, indices);
         UP3D_CHECK_LAUNCH();
     });
 }

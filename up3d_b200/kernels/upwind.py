@@ -68,7 +68,6 @@ class UpwindOperator:
         self.weighted = bool(weighted)
         self.mode = mode
         self.nbr_depth = int(nbr_depth)
-        self._nb = None
         if self.weighted and mode == "kernel":
             self._neighborhoods()
         self.p_weight, self.reach_frac, self.reach_gain_max = p_weight, reach_frac, reach_gain_max
@@ -114,13 +113,13 @@ class UpwindOperator:
         self._mesh.set_face_neighbors(value)
         self._fn = value
 
-    def _neighborhoods(self):
-        """The mesh's depth-hop neighbourhood CSR (device views)."""
+    def _neighborhoods(self, lists=False):
+        """The mesh's depth-hop neighbourhood CSR (device views): offsets,
+        indices (None unless `lists`) and their number."""
         off, idx, total = ctypes.c_void_p(), ctypes.c_void_p(), ctypes.c_int64()
         L.call("up3d_mesh_neighborhoods", self._mesh.handle, self.nbr_depth, ctypes.byref(off),
-               ctypes.byref(idx), ctypes.byref(total), L.stream_ptr())
-        self._nb = (off.value, idx.value, int(total.value))
-        return self._nb
+               ctypes.byref(idx) if lists else None, ctypes.byref(total), L.stream_ptr())
+        return off.value, idx.value, int(total.value)
 
     @property
     def _nb_off(self):
@@ -135,7 +134,7 @@ class UpwindOperator:
         if not (self.weighted and self.mode == "kernel"):
             return None
         from ..mesh.device import device_view
-        _, ptr, total = self._neighborhoods()
+        _, ptr, total = self._neighborhoods(lists=True)
         idx = device_view(ptr, (total,), np.int32).to(L.torch().int64)
         return idx.cpu().numpy() if self._host else idx
 
