@@ -903,27 +903,27 @@ __global__ void __launch_bounds__(256)
 
 // out = x + w D^-1 (b - A x)   (or, with RESID, out = b - A x).  The finest
 // operator is the embedded one (identity rows, no constrained columns): no
-// mask.
-template <class T, bool RESID, int TPR>
+// mask.  TO: type of out (the caller's vector behind the last sweep).
+template <class T, bool RESID, int TPR, class TO>
 __global__ void __launch_bounds__(rows_block<TPR>)
     k_jacobi_sweep(int64_t n, const int32_t* __restrict__ Ap, const int32_t* __restrict__ Ai,
-                   const T* __restrict__ Ax, const T* __restrict__ dinv, const T* b, const T* x, T* out,
+                   const T* __restrict__ Ax, const T* __restrict__ dinv, const T* b, const T* x, TO* out,
                    const double* __restrict__ omega) {
     pdl_trigger();
     pdl_wait();
     const T w = (T)*omega;
     csr_rows_loop<T, TPR, rows_block<TPR>>(n, Ap, Ai, Ax, x, [&](int64_t r, T acc) {
         const T res = b[r] - acc;
-        out[r] = RESID ? res : x[r] + w * dinv[r] * res;
+        out[r] = (TO)(RESID ? res : x[r] + w * dinv[r] * res);
     });
 }
 
 // The same sweep on the sliced rows, one row per lane; the first entries are
 // on their way while the kernel before drains.
-template <class T, bool RESID>
+template <class T, bool RESID, class TO>
 __global__ void __launch_bounds__(SELL_BLOCK)
     k_jacobi_sell(int64_t n, const int32_t* __restrict__ Sp, const int32_t* __restrict__ Si,
-                  const T* __restrict__ Sx, const T* __restrict__ dinv, const T* b, const T* x, T* out,
+                  const T* __restrict__ Sx, const T* __restrict__ dinv, const T* b, const T* x, TO* out,
                   const double* __restrict__ omega) {
     pdl_trigger();
     const int64_t r = blockIdx.x * (int64_t)SELL_BLOCK + threadIdx.x;
@@ -932,7 +932,7 @@ __global__ void __launch_bounds__(SELL_BLOCK)
     const T acc = sell_row_sum<T>(Sp, Si, Sx, x, r >> 5, lane, pdl_wait);
     if (r >= n) return;
     const T res = b[r] - acc;
-    out[r] = RESID ? res : x[r] + (T)*omega * dinv[r] * res;
+    out[r] = (TO)(RESID ? res : x[r] + (T)*omega * dinv[r] * res);
 }
 
 // Column indices of the sliced rows from the CSR ones (-1 on the padding),
@@ -968,13 +968,13 @@ __global__ void __launch_bounds__(rows_block<TPR>)
                                            [&](int64_t r, T acc) { y[r] = ADD ? y[r] + acc : acc; });
 }
 
-template <class T, bool RESID>
+template <class T, bool RESID, class TO>
 void launch_sweep(bool overlap, int64_t n, int64_t nnz, const int32_t* Ap, const int32_t* Ai, const T* Ax,
-                  const T* dinv, const T* b, const T* x, T* out, const double* omega, cudaStream_t s) {
+                  const T* dinv, const T* b, const T* x, TO* out, const double* omega, cudaStream_t s) {
     const int tpr = use_warp_rows(n, nnz) ? 0 : lanes_per_row(nnz, n);
-    auto kern = tpr == 0 ? k_jacobi_sweep<T, RESID, 0> : tpr == 4 ? k_jacobi_sweep<T, RESID, 4>
-                : tpr == 8 ? k_jacobi_sweep<T, RESID, 8> : tpr == 16 ? k_jacobi_sweep<T, RESID, 16>
-                : k_jacobi_sweep<T, RESID, 32>;
+    auto kern = tpr == 0 ? k_jacobi_sweep<T, RESID, 0, TO> : tpr == 4 ? k_jacobi_sweep<T, RESID, 4, TO>
+                : tpr == 8 ? k_jacobi_sweep<T, RESID, 8, TO> : tpr == 16 ? k_jacobi_sweep<T, RESID, 16, TO>
+                : k_jacobi_sweep<T, RESID, 32, TO>;
     launch_kernel(overlap, kern, tpr == 0 ? csr_rows_grid(n, CSR_WARP_BLOCK) : lanes_grid(n, tpr),
                   tpr == 0 ? CSR_WARP_BLOCK : CSR_ROWS_BLOCK, s, n, Ap, Ai, Ax, dinv, b, x, out, omega);
 }
@@ -1159,8 +1159,7 @@ struct Amg {
     struct Body {
         cudaGraphExec_t exec = nullptr;
         long long launches = 0;
-        void* x = nullptr;   // the level-0 iterate after the body, and the other buffer
-        void* other = nullptr;
+        void* x = nullptr;   // the level-0 iterate after the body
     };
     Body body64, body32;
     cudaStream_t capture_stream = nullptr;
@@ -1179,14 +1178,14 @@ namespace {
 
 // One sweep (or residual) of a level's operator: the sliced rows where the
 // level has them, else the CSR rows.
-template <class T, bool RESID>
-void smooth(bool overlap, const Level<T>& lv, const T* x, T* out, cudaStream_t s) {
+template <class T, bool RESID, class TO>
+void smooth(bool overlap, const Level<T>& lv, const T* x, TO* out, cudaStream_t s) {
     const int64_t n = lv.A.n;
     if (lv.sell_p)
-        launch_kernel(overlap, k_jacobi_sell<T, RESID>, sell_grid(n), SELL_BLOCK, s, n, lv.sell_p, lv.sell_i,
+        launch_kernel(overlap, k_jacobi_sell<T, RESID, TO>, sell_grid(n), SELL_BLOCK, s, n, lv.sell_p, lv.sell_i,
                       lv.sell_x.get(), lv.dinv.get(), lv.b.get(), x, out, lv.omega);
     else
-        launch_sweep<T, RESID>(overlap, n, lv.A.nnz, lv.A.p.get(), lv.A.i.get(), lv.A.x.get(), lv.dinv.get(),
+        launch_sweep<T, RESID, TO>(overlap, n, lv.A.nnz, lv.A.p.get(), lv.A.i.get(), lv.A.x.get(), lv.dinv.get(),
                                lv.b.get(), x, out, lv.omega, s);
 }
 
@@ -1468,7 +1467,6 @@ static void capture_body(Amg& a, std::vector<Level<T>*>& L, Amg::Body& body) {
         throw;
     }
     body.x = L[0]->x.p;
-    body.other = L[0]->r.p;
     restore();
     UP3D_CUDA(cudaStreamEndCapture(a.capture_stream, &graph));
     body.launches = g_launches.load() - l0;
@@ -1496,15 +1494,12 @@ static void apply_cycle(Amg& a, std::vector<Level<T>*>& L, Amg::Body& body, cons
                   f.omega, n);
     UP3D_CUDA(cudaGraphLaunch(body.exec, s));
     count_launch((int)body.launches);
-    T* x = static_cast<T*>(body.x);
-    T* last = static_cast<T*>(body.other);
+    const T* x = static_cast<const T*>(body.x);
     if (a.post == 0) {
         convert_copy(x, z, n, s);
         return;
     }
-    if constexpr (std::is_same<T, TIO>::value) last = z;
-    smooth<T, false>(false, f, x, last, s);
-    if constexpr (!std::is_same<T, TIO>::value) convert_copy(last, z, n, s);
+    smooth<T, false>(false, f, x, z, s);   // in the caller's precision: a conversion behind it is 2 us of a small cycle
 }
 
 void amg_apply(void* p, const double* r, double* z, cudaStream_t s) {
