@@ -80,7 +80,7 @@ template <int KJ>
 constexpr int basis_blocks = KJ == 1 ? 6 : KJ == 2 ? 4 : KJ <= 4 ? 3 : 2;
 template <class T, int KJ, int PASS>
 __global__ void __launch_bounds__(DOT_BLOCK, basis_blocks<KJ>)
-    k_basis(const T* __restrict__ V, int64_t ldv, int K, double* h, T* y, int64_t n, bool self,
+    k_basis(const T* V, int64_t ldv, int K, double* h, T* y, int64_t n, bool self,
             double* __restrict__ partial, double* out, unsigned int* __restrict__ counter, const double* hsrc,
             double* hdst, int hlen) {
     constexpr int VEC = 16 / sizeof(T), ROWS = 32 * VEC;
