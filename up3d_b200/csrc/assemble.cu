@@ -392,6 +392,11 @@ __global__ void __launch_bounds__(NT, MB)
                  double* __restrict__ rt_out, up3d_monitors* mon, const Flow* __restrict__ flows,
                  const int32_t* __restrict__ case_of, int n_cases, int8_t* __restrict__ br_out) {
     constexpr int LOC2 = LOC_STRIDE / 2;
+    // the test for subcritical pairs, except in the frozen Jacobian of other
+    // gases, whose elements rarely take it and whose upstream pow is better
+    // early (gamma 1.3, 8.2 M tets, 768 threads persistent: 968 us without, 1107
+    // with it; 640 threads 1004 and 1078)
+    constexpr bool SKIP = AIR || !FROZEN || !JAC;
     __shared__ double2 slab[JAC ? NT * LOC2 : 1];  // the local records of each warp's 32 elements
     const int lane = threadIdx.x & 31;
     double2* const mine = slab + (JAC ? (threadIdx.x - lane) * LOC2 : 0);
@@ -443,11 +448,12 @@ __global__ void __launch_bounds__(NT, MB)
                 double q2nu = __ddiv_rn(dot3r(gu[0], gu[1], gu[2], gu[0], gu[1], gu[2]), u2);
                 q2lu = q2nu < F.q2cap ? q2nu : F.q2cap;
                 lim_u = q2lu == q2nu;
+                if (!SKIP) rho_u = rho_of<AIR>(q2lu, F);
             }
             // both elements surely subcritical: the switch is 0, no upstream
             // density, Mach number or switch enters (four divisions and a root)
-            const bool sub = !frz && q2l <= F.q2sub && q2lu <= F.q2sub;
-            if (u != e && !sub) rho_u = rho_of<AIR>(q2lu, F);
+            const bool sub = SKIP && !frz && q2l <= F.q2sub && q2lu <= F.q2sub;
+            if (SKIP && u != e && !sub) rho_u = rho_of<AIR>(q2lu, F);
             acc.lim += !lim_e;
 
             double nu, rt, s_e = 0.0, s_u = 0.0;
@@ -1692,7 +1698,7 @@ __global__ void k_check_cases(const int32_t* __restrict__ case_of, int64_t E, in
 // One launch of the fused element sweep in the mesh's tuned shape: one
 // thread per element (grid capped at 64 blocks per SM) or one resident
 // wave (SMs x the kernel's occupancy) looping over block-sized tiles; the
-// Jacobian sweep compiled for 512 (256 x 2), 640 (128 x 5) or 768 (256 x 3)
+// Jacobian sweep compiled for 512 (256 x 2), 640 (128 x 5) or 768 (128 x 6)
 // resident threads per SM.
 template <bool FR, bool JA, bool BA, bool AIR, int NT, int MB, class... A>
 static void launch_sweep_mb(const up3d_mesh* m, cudaStream_t s, A... args) {
@@ -1721,12 +1727,16 @@ static void launch_sweep_air(const up3d_mesh* m, cudaStream_t s, A... args) {
     // the form for any gas (the whole call, walk / frozen: 3.6 M tets 269 / 187
     // against 272 / 193 us, 0.97 M 86.1 / 57.6 and 84.7 / 57.9, 0.45 M 45.2 /
     // 29.6 against 43.2 / 28.6)
-    if (!JA) return AIR && m->E >= SWEEP_LARGE ? launch_sweep_mb<FR, JA, BA, AIR, 128, 7>(m, s, args...)
-                                               : launch_sweep_mb<FR, JA, BA, false, 256, 3>(m, s, args...);
-    switch (m->tune.elem_threads_per_sm) {
-        case 640: launch_sweep_mb<FR, JA, BA, AIR, 128, 5>(m, s, args...); break;
-        case 768: launch_sweep_mb<FR, JA, BA, AIR, 128, 6>(m, s, args...); break;
-        default: launch_sweep_mb<FR, JA, BA, AIR, 256, 2>(m, s, args...); break;
+    if constexpr (!JA) {
+        if constexpr (AIR)
+            if (m->E >= SWEEP_LARGE) return launch_sweep_mb<FR, JA, BA, AIR, 128, 7>(m, s, args...);
+        launch_sweep_mb<FR, JA, BA, false, 256, 3>(m, s, args...);
+    } else {
+        switch (m->tune.elem_threads_per_sm) {
+            case 640: launch_sweep_mb<FR, JA, BA, AIR, 128, 5>(m, s, args...); break;
+            case 768: launch_sweep_mb<FR, JA, BA, AIR, 128, 6>(m, s, args...); break;
+            default: launch_sweep_mb<FR, JA, BA, AIR, 256, 2>(m, s, args...); break;
+        }
     }
 }
 
