@@ -456,9 +456,9 @@ int up3d_residual_jacobian_batched(up3d_mesh* mesh, const double* phi, int n_cas
  *                    block-sized tiles
  *   elem_threads_per_sm  register budget of the Newton-Jacobian sweep as
  *                    the resident threads per SM it allows: 512 (256-thread
- *                    blocks, up to 128 registers), 640 (128-thread blocks,
- *                    up to 96, no spills for air) or 768 (128-thread blocks,
- *                    up to 80, spilling to L1)
+ *                    blocks, up to 128 registers, no spills), 640 (128-thread
+ *                    blocks, up to 96, few or no spills) or 768 (128-thread
+ *                    blocks, up to 80, spilling to L1)
  *   row_lanes        lanes per row of the row gather: 4, 8, 16 or 32
  *   row_plan8        1: the row gather reads each upper slot's
  *                    contributors from a fixed-width record (built at mesh

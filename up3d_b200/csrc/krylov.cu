@@ -28,7 +28,8 @@ namespace {
 
 // The kernels of an iteration are launched overlapped (each starts while the
 // one before drains: 2 us less between two of them): vectors and scalars that
-// an earlier one writes are read after pdl_wait, and not through __restrict__.
+// an earlier one writes are read after pdl_wait, and not through __restrict__
+// (the basis among them: its newest vector comes from an overlapped launch).
 // Results for the host go to `host`, page-locked memory, from the kernel that
 // forms them: a copy behind it costs 5 us of an iteration.
 
@@ -720,9 +721,7 @@ int gmres_solve(const Operator& op, const T* b, T* x, double rtol, double atol, 
             // pass 1 takes V_0..V_col and the new vector itself in one
             // sweep (h and |w|^2), passes 2 and 3 are one sweep each
             // (update + the next pass's dots, update + |w|^2), and the
-            // normalisation writes the vector into V[col + 1].  The
-            // preconditioner's output stays the one buffer w, so its
-            // captured V-cycle graph is replayed, not captured per column.
+            // normalisation writes the vector into V[col + 1].
             double* hsum = hdev.get();                  // h_0..h_col, |w|^2 before, |w|^2 after
             double* hpass = hdev.get() + (restart + 3);
             double* hn = hsum + col + 1;

@@ -54,8 +54,9 @@ __global__ void __launch_bounds__(TPR == 0 ? CSR_WARP_BLOCK : CSR_ROWS_BLOCK)
 }
 
 // r = b - (A x + X x), masked as k_spmv, each row's sum carried as an
-// unevaluated pair (error-free products by fma, Knuth's two-sum): rounded
-// once, whatever the cancellation.  A restart's true residual is formed
+// unevaluated pair (error-free products by fma, Knuth's two-sum; the low
+// parts in plain FP64): within about eps^2 |A| |x| of the exact sum before its
+// one rounding.  A restart's true residual is formed
 // here: near a singular matrix |x| is so large that a plain sum's rounding
 // (eps |A| |x|) is above the tolerance asked for, and whether a cycle met it
 // hung on the order of the sums.  Four lanes per row; once per restart.

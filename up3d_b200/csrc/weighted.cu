@@ -180,14 +180,17 @@ __global__ void k_slice_lists(int64_t E, const int64_t* __restrict__ nb_off, con
 }
 
 // rho_tilde_kernel_sweep (kernels/upwind.py:345-454).  One thread per element,
-// the warp's neighbour lists interleaved (slices).
+// the warp's neighbour lists interleaved (slices), 33 neighbours at depth 3:
+// 132 bytes an element beside its 8 of offsets.
 //
 // The weights only matter where the switch can act: with the element and
 // every neighbour subcritical the sampled M^2, an average of theirs, is too,
 // and the density is the element's own.  So the neighbours' speeds are
 // looked at first (8 bytes each, no centroid, no exponential), against M_c^2
 // less a margin far above the average's rounding; a speed past the vacuum
-// limit or a NaN takes the full sum.  The sum runs at 64 registers for the
+// limit or a NaN takes the full sum.  (Where every weight is below 1e-311 the
+// sum's average is a quotient of subnormals and may leave the neighbours'
+// range; the skip gives the exact 0.)  The sum runs at 64 registers for the
 // warps in flight: it is bound by the latency of its gathers and FP64 work.
 // 3.6 M tets, a supersonic pocket over the bump: 870 -> 253 us; with most
 // elements supersonic the full sum is what counts (1.8 M tets: 275 us, issue
