@@ -51,8 +51,10 @@ int guarded(F&& body) {
         body();
         return UP3D_OK;
     } catch (const Error& e) {
+        cudaGetLastError();   // reported here: the next call's launch check must not see it
         return fail(e.status, e.msg);
     } catch (const std::exception& e) {
+        cudaGetLastError();
         return fail(UP3D_ERR_RUNTIME, e.what());
     }
 }
