@@ -1455,6 +1455,7 @@ static void capture_body(Amg& a, std::vector<Level<T>*>& L, Amg::Body& body) {
             L[i]->r.p = saved[i].second;
         }
     };
+    std::unique_lock<std::mutex> capturing(capture_mutex());   // no buffer is made or freed meanwhile
     const long long l0 = g_launches.load();
     cudaGraph_t graph = nullptr;
     UP3D_CUDA(cudaStreamBeginCapture(a.capture_stream, cudaStreamCaptureModeThreadLocal));
@@ -1469,6 +1470,7 @@ static void capture_body(Amg& a, std::vector<Level<T>*>& L, Amg::Body& body) {
     body.x = L[0]->x.p;
     restore();
     UP3D_CUDA(cudaStreamEndCapture(a.capture_stream, &graph));
+    capturing.unlock();
     body.launches = g_launches.load() - l0;
     g_launches.fetch_sub(body.launches);  // counted at each replay instead
     cudaGraphExec_t exec = nullptr;

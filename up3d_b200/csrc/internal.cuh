@@ -6,6 +6,7 @@
 #include <stdint.h>
 
 #include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -100,6 +101,10 @@ void launch_kernel(bool overlap, void (*kern)(P...), unsigned grid, int block, c
 // reused by later requests of nearly the same size.
 void* dev_alloc(size_t bytes);
 void dev_free(void* p);
+// Held by a thread while it captures a stream and while one waits for the
+// device: such a wait ends every capture under way on it, whoever made it.
+std::mutex& capture_mutex();
+cudaError_t device_sync();   // cudaDeviceSynchronize under it
 
 template <class T>
 struct DBuf {

@@ -591,7 +591,7 @@ int up3d_mesh_destroy(up3d_mesh* m) {
     return guarded([&] {
         if (!m) return;
         DeviceGuard g(m->device);
-        cudaDeviceSynchronize();
+        device_sync();
         drop_extra(m);
         delete m;
     });

@@ -131,6 +131,15 @@ void* dev_alloc(size_t bytes) {
     return p;
 }
 
+std::mutex& capture_mutex() {
+    static std::mutex* m = new std::mutex();   // never destroyed, as the pool
+    return *m;
+}
+cudaError_t device_sync() {
+    std::lock_guard<std::mutex> g(capture_mutex());
+    return cudaDeviceSynchronize();
+}
+
 void dev_free(void* p) {
     if (!p) return;
     Pool& P = pool();
@@ -150,7 +159,7 @@ void dev_free(void* p) {
     cudaGetDevice(&prev);
     if (prev != b.device) cudaSetDevice(b.device);
     // work in flight may still use the block: wait for it, as cudaFree does
-    const cudaError_t e = cudaDeviceSynchronize();
+    const cudaError_t e = device_sync();
     if (e != cudaSuccess || b.size > P.cap) {
         cudaFree(p);
         cudaGetLastError();
